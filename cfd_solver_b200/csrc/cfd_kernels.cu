@@ -18,30 +18,13 @@
 //                    boundary pressure, wall integrals   PSolver.cpp:1901-1983
 //   k_diag           dilatation, vorticity, dmax         PSolver.cpp:1807-1853
 //   k_si             stream function (output only)       PSolver.cpp:1789-1801
-#include <type_traits>
-
 #include "cfd_common.cuh"
 #include "cfd_reduce.cuh"
 #include "cfd_kernels.cuh"
 #include "cfd_bulk.cuh"
+#include "cfd_step.cuh"
 
 namespace cfd {
-
-#define AT(ptr, ii, jj) (ptr)[(long long)(jj) * ld + (ii)]
-
-constexpr int JTW = TX + 4;   // 32 x 16 tile columns incl. a 2-cell halo
-constexpr int JTH = TYJ + 4;  // 32 x 16 tile rows incl. a 2-cell halo
-
-// plane that holds the final multigrid V-cycle result of level l of case c (x on the
-// case's coarsest level; otherwise fixed by the numbers of pre- and post-sweeps)
-__device__ __forceinline__ int mg_result_plane(const BatchDev& b, const CaseDev& c, int l) {
-    return l == c.nlev - 1 ? M_X : b.mg_res;
-}
-
-__device__ __forceinline__ bool near_wall(const CaseDev& c, int i, int j) {
-    if (j == 1 || j == c.n1 - 2) return true;
-    return c.profile == CAVITY && (i == 1 || i == c.n0 - 2);
-}
 
 // ---------------------------------------------------------------------------
 // The 9-point pressure stencil at one cell (PSolver.cpp:944-1040) from the four metric
@@ -105,75 +88,6 @@ __global__ void __launch_bounds__(NT) k_assemble_p(BatchDev b, int toff) {
 }
 
 // ---------------------------------------------------------------------------
-// u/v/T operator coefficients, PSolver.cpp:765-849, computed in registers
-struct Coef25 {
-    double p, e, w, n, s, ne, nw, se, sw;
-    double ee, ww, nn, ss, nnee, nnww, ssee, ssww, nne, nnw, sse, ssw, nee, nww, see, sww;
-};
-
-__device__ __forceinline__ void build_coefs(const CaseDev& c, double al, double be, double ga,
-                                            bool nearw, int j, Coef25& A, Coef25& T) {
-    const double d0 = c.d0, d1 = c.d1, dt = c.dt, Re = c.Re, Pr = c.Pr;
-    if (nearw) {
-        A.e = A.w = -dt * (al / (d0 * d0)) / Re;
-        A.n = A.s = -dt * (ga / (d1 * d1)) / Re;
-        A.ne = A.sw = dt * be / (2.0 * d0 * d1 * Re);
-        A.nw = A.se = -dt * be / (2.0 * d0 * d1 * Re);
-        A.p = 1 + dt * 2.0 * (al / (d0 * d0) + ga / (d1 * d1)) / Re;
-        T.e = T.w = -dt * (al / (d0 * d0)) / (Re * Pr);
-        T.n = T.s = -dt * (ga / (d1 * d1)) / (Re * Pr);
-        T.ne = T.sw = dt * (be / (2.0 * d0 * d1)) / (Re * Pr);
-        T.nw = T.se = -dt * (be / (2.0 * d0 * d1)) / (Re * Pr);
-        T.p = 1 + dt * 2.0 * (al / (d0 * d0) + ga / (d1 * d1)) / (Re * Pr);
-        if (c.profile == OGRID) {
-            // wall-row couplings are folded into the right-hand side (PSolver.cpp:851-882)
-            if (j == 1) { A.s = A.se = A.sw = 0.0; T.s = T.se = T.sw = 0.0; }
-            if (j == c.n1 - 2) { A.n = A.ne = A.nw = 0.0; T.n = T.ne = T.nw = 0.0; }
-        }
-        A.ee = A.ww = A.nn = A.ss = A.nnee = A.nnww = A.ssee = A.ssww = 0.0;
-        A.nne = A.nnw = A.sse = A.ssw = A.nee = A.nww = A.see = A.sww = 0.0;
-        T.ee = T.ww = T.nn = T.ss = T.nnee = T.nnww = T.ssee = T.ssww = 0.0;
-        T.nne = T.nnw = T.sse = T.ssw = T.nee = T.nww = T.see = T.sww = 0.0;
-    } else {
-        A.e = A.w = (-dt) * ((4.0 * al) / (3.0 * d0 * d0)) / Re;
-        A.n = A.s = (-dt) * ((4.0 * ga) / (3.0 * d1 * d1)) / Re;
-        A.ne = A.sw = (-dt) * (-8.0 * be / (9.0 * d0 * d1)) / Re;
-        A.nw = A.se = (-dt) * (8.0 * be / (9.0 * d0 * d1)) / Re;
-        A.nn = A.ss = (-dt) * (-ga / (12.0 * d1 * d1)) / Re;
-        A.ee = A.ww = (-dt) * (-al / (12.0 * d0 * d0)) / Re;
-        A.nnee = A.ssww = (-dt) * (-be / (72.0 * d0 * d1)) / Re;
-        A.nnww = A.ssee = (-dt) * (be / (72.0 * d0 * d1)) / Re;
-        A.nne = A.ssw = A.nee = A.sww = (-dt) * (be / (9.0 * d0 * d1)) / Re;
-        A.nnw = A.sse = A.nww = A.see = (-dt) * (-be / (9.0 * d0 * d1)) / Re;
-        A.p = 1 + dt * (5.0 * al / (2.0 * d0 * d0) + 5.0 * ga / (2.0 * d1 * d1)) / Re;
-        T.e = A.e / Pr; T.w = A.w / Pr; T.n = A.n / Pr; T.s = A.s / Pr;
-        T.ne = A.ne / Pr; T.nw = A.nw / Pr; T.se = A.se / Pr; T.sw = A.sw / Pr;
-        T.nn = A.nn / Pr; T.ss = A.ss / Pr; T.ee = A.ee / Pr; T.ww = A.ww / Pr;
-        T.nnee = A.nnee / Pr; T.nnww = A.nnww / Pr; T.ssee = A.ssee / Pr; T.ssww = A.ssww / Pr;
-        T.nne = A.nne / Pr; T.nnw = A.nnw / Pr; T.sse = A.sse / Pr; T.ssw = A.ssw / Pr;
-        T.nee = A.nee / Pr; T.nww = A.nww / Pr; T.see = A.see / Pr; T.sww = A.sww / Pr;
-        T.p = 1 + dt * (5.0 * al / (2.0 * d0 * d0) + 5.0 * ga / (2.0 * d1 * d1)) / (Re * Pr);
-        // the reference's T solve passes atnw in the annw slot (PSolver.cpp:1290)
-        if (!c.fix_T_annw) T.nnw = T.nw;
-    }
-}
-
-// sum of the off-centre couplings, in the order of gauss() (PSolver.cpp:2408-2425)
-__device__ __forceinline__ double offsum(const double* F, long long k, int ld, const Coef25& a, bool nearw) {
-    double s = a.e * F[k + 1] + a.n * F[k + ld] + a.s * F[k - ld] + a.w * F[k - 1] +
-               a.nw * F[k + ld - 1] + a.ne * F[k + ld + 1] + a.sw * F[k - ld - 1] + a.se * F[k - ld + 1];
-    if (!nearw) {
-        const long long l2 = 2LL * ld;
-        s += a.ee * F[k + 2] + a.ww * F[k - 2] + a.nnee * F[k + l2 + 2] + a.nee * F[k + ld + 2] +
-             a.see * F[k - ld + 2] + a.ssee * F[k - l2 + 2] + a.nne * F[k + l2 + 1] +
-             a.sse * F[k - l2 + 1] + a.nnw * F[k + l2 - 1] + a.ssw * F[k - l2 - 1] +
-             a.nnww * F[k + l2 - 2] + a.nww * F[k + ld - 2] + a.sww * F[k - ld - 2] +
-             a.ssww * F[k - l2 - 2] + a.nn * F[k + l2] + a.ss * F[k - l2];
-    }
-    return s;
-}
-
-// ---------------------------------------------------------------------------
 // contravariant velocities + convection + the five right-hand sides
 // (PSolver.cpp:1063-1237); also seeds the five solves' iterates. A CTA owns a 32 x 16 tile
 // (two cells per thread); u, v, T, p, up, vp with a 2-cell halo and the seven metric
@@ -181,43 +95,6 @@ __device__ __forceinline__ double offsum(const double* F, long long k, int ld, c
 constexpr int RHS_HALO = 6, RHS_INT = 7;
 constexpr size_t RHS_SMEM = (size_t)(RHS_HALO * JTW * JTH + RHS_INT * TX * TYJ) * sizeof(double) + 128;
 const size_t kRhsSmem = RHS_SMEM;
-
-// One convective term ux df/dxi + ue df/deta of field F at tile offset o
-// (PSolver.cpp:1110-1180): 4th-order central differences when the cell Peclet number is in
-// (-2, 2] (and always in the rows / columns next to a wall, where the reference uses
-// 2nd-order central), otherwise 3rd-order upwind. The reference forms du = (ux D1 +
-// |ux| D4) / ux and multiplies by ux again; here the product is formed directly, and every
-// division by a grid spacing is a multiplication by its reciprocal.
-__device__ __forceinline__ double conv_one(const double* F, int o, bool near_i, bool near_j, double ux,
-                                           double ue, bool cen_i, bool cen_j, double rd0, double rd1) {
-    constexpr int R = JTW;
-    const double fc = F[o], fe = F[o + 1], fw = F[o - 1];
-    const double fn = F[o + R], fs = F[o - R];
-    double cx, cy;
-    if (near_i) {
-        cx = ux * (0.5 * (fe - fw) * rd0);
-    } else {
-        const double fee = F[o + 2], fww = F[o - 2];
-        if (near_j || cen_i) {
-            cx = ux * ((1.0 / 12.0) * (8.0 * (fe - fw) - (fee - fww)) * rd0);
-        } else {
-            cx = (ux * ((1.0 / 12.0) * (-fee + 8.0 * fe - 8.0 * fw + fww)) +
-                  fabs(ux) * (0.25 * (fee - 4.0 * fe + 6.0 * fc - 4.0 * fw + fww))) * rd0;
-        }
-    }
-    if (near_j) {
-        cy = ue * (0.5 * (fn - fs) * rd1);
-    } else {
-        const double fnn = F[o + 2 * R], fss = F[o - 2 * R];
-        if (near_i || cen_j) {
-            cy = ue * ((1.0 / 12.0) * (8.0 * (fn - fs) - (fnn - fss)) * rd1);
-        } else {
-            cy = (ue * ((1.0 / 12.0) * (-fnn + 8.0 * fn - 8.0 * fs + fss)) +
-                  fabs(ue) * (0.25 * (fnn - 4.0 * fn + 6.0 * fc - 4.0 * fs + fss))) * rd1;
-        }
-    }
-    return cx + cy;
-}
 
 // Three CTAs per SM (80 registers, 36 bytes of spills; the 63 KB staged per CTA fits three
 // times): while one CTA computes, two others' copies are in flight. Two CTAs per SM at 122
@@ -230,7 +107,7 @@ __global__ void __launch_bounds__(NT, 3) k_rhs(BatchDev b) {
     const Tile t = b.jtiles[blockIdx.x];
     const CaseDev& c = b.cases[t.c];
     const int tid = threadIdx.x;
-    const int cur = b.cur, nxt = cur ^ 1;
+    const int cur = b.cur;
     // halo tiles: u, v, T, p, up, vp; interior tiles: xix, xiy, etx, ety, alpha, gamma, beta
     double* SI = sm + RHS_HALO * JTW * JTH;
     const bool active = b.iscal[(long long)t.c * NISCAL + I_ACTIVE] != 0;
@@ -269,8 +146,9 @@ __global__ void __launch_bounds__(NT, 3) k_rhs(BatchDev b) {
     // the case's constants and planes, loaded while the copies are in flight
     const int ld = c.ld, W = c.W, per = c.periodic, n1 = c.n1, n0 = c.n0, ilo = c.ilo, ihi = c.ihi;
     const bool cav = c.profile == CAVITY;
-    const double d0 = c.d0, d1 = c.d1, dt = c.dt, Re = c.Re, Pr = c.Pr, Ri = c.Ri;
-    const double rd0 = 1.0 / d0, rd1 = 1.0 / d1;
+    RhsCase rc;
+    rc.d0 = c.d0; rc.d1 = c.d1; rc.rd0 = 1.0 / c.d0; rc.rd1 = 1.0 / c.d1;
+    rc.dt = c.dt; rc.Re = c.Re; rc.Pr = c.Pr; rc.Ri = c.Ri; rc.n0 = n0; rc.n1 = n1; rc.cav = cav;
     double* const fb = b.f64 + c.base + H;  // plane 0 of the case; plane k at fb + k * ps
     const long long ps = c.ps;
     const bool warm = c.warm_up != 0;
@@ -288,14 +166,6 @@ __global__ void __launch_bounds__(NT, 3) k_rhs(BatchDev b) {
     }
     const double *Us = sm, *Vs = sm + JTW * JTH, *Ts = sm + 2 * JTW * JTH, *Ps = sm + 3 * JTW * JTH,
                  *UPs = sm + 4 * JTW * JTH, *VPs = sm + 5 * JTW * JTH;
-    const double* U = fb + P_U * ps;
-    const double* V = fb + P_V * ps;
-    const double* T = fb + (P_T0 + cur) * ps;
-    const double* UP = fb + (P_UP0 + cur) * ps;
-    const double* VP = fb + (P_VP0 + cur) * ps;
-    // iterate buffers of field f: A (the solution) and B (the Jacobi scratch)
-    auto Ap = [&](int f) { return fb + (f < 2 ? P_US + f : P_T0 + 2 * (f - 2) + nxt) * ps; };
-    auto Bp = [&](int f) { return fb + (P_BU + f) * ps; };
     const int li = tid % TX, lj = tid / TX;
     const int i = t.i0 + li;
 #pragma unroll 1
@@ -305,100 +175,16 @@ __global__ void __launch_bounds__(NT, 3) k_rhs(BatchDev b) {
         const int o = (lj + h * TY + 2) * JTW + (li + 2);
         const int oi = (lj + h * TY) * TX + li;
         const long long k = (long long)j * ld + i;
-        const double xix = SI[oi], xiy = SI[TX * TYJ + oi], etx = SI[2 * TX * TYJ + oi], ety = SI[3 * TX * TYJ + oi];
-        const double al = SI[4 * TX * TYJ + oi], ga = SI[5 * TX * TYJ + oi];
-        const double uc = Us[o], vc = Vs[o], tc = Ts[o];
-        const double ux = xix * uc + xiy * vc;
-        const double ue = etx * uc + ety * vc;
-        const bool near_j = (j == 1 || j == n1 - 2);
-        const bool near_i = cav && (i == 1 || i == n0 - 2);
-        // cell Peclet numbers ux Re dxi / alpha, ue Re deta / gamma (x Pr for T)
-        const double pu1 = ux * (Re * d0) / al, pu2 = ue * (Re * d1) / ga;
-        const double pt1 = pu1 * Pr, pt2 = pu2 * Pr;
-        const bool cu1 = pu1 <= 2 && pu1 > -2, cu2 = pu2 <= 2 && pu2 > -2;
-        const bool ct1 = pt1 <= 2 && pt1 > -2, ct2 = pt2 <= 2 && pt2 > -2;
-        const double cv0 = conv_one(Us, o, near_i, near_j, ux, ue, cu1, cu2, rd0, rd1);
-        const double cv1 = conv_one(Vs, o, near_i, near_j, ux, ue, cu1, cu2, rd0, rd1);
-        const double cv2 = conv_one(Ts, o, near_i, near_j, ux, ue, ct1, ct2, rd0, rd1);
-        const double dp_dxi = (Ps[o + 1] - Ps[o - 1]) * (0.5 * rd0);
-        const double dp_de = (Ps[o + JTW] - Ps[o - JTW]) * (0.5 * rd1);
-        const double dp_dx = xix * dp_dxi + etx * dp_de;
-        const double dp_dy = xiy * dp_dxi + ety * dp_de;
-        double qu = dt * (-cv0 - dp_dx) + uc;
-        double qv = dt * (-cv1 - dp_dy + Ri * tc) + vc;
-        double qt = -dt * cv2 + tc;
-        double qup = qu + dt * dp_dx;
-        double qvp = qv + dt * dp_dy;
-        if (!cav && near_j) {
-            // folded wall-row couplings (PSolver.cpp:1195-1227)
-            const double be = SI[6 * TX * TYJ + oi];
-            const double bs = -dt * (ga / (d1 * d1)) / Re;
-            const double bpos = dt * be / (2.0 * d0 * d1 * Re);
-            const double bneg = -dt * be / (2.0 * d0 * d1 * Re);
-            const double ts = -dt * (ga / (d1 * d1)) / (Re * Pr);
-            const double tpos = dt * (be / (2.0 * d0 * d1)) / (Re * Pr);
-            const double tneg = -dt * (be / (2.0 * d0 * d1)) / (Re * Pr);
-            int s0, s1, s2;
-            double c1, c2, t1, t2;
-            if (j == 1) {  // bus, buse (= ause), busw (= ausw)
-                s0 = o - JTW; s1 = o - JTW + 1; s2 = o - JTW - 1;
-                c1 = bneg; c2 = bpos; t1 = tneg; t2 = tpos;
-            } else {       // bun, bune (= aune), bunw (= aunw)
-                s0 = o + JTW; s1 = o + JTW + 1; s2 = o + JTW - 1;
-                c1 = bpos; c2 = bneg; t1 = tpos; t2 = tneg;
-            }
-            double sumu = bs * Us[s0] + c1 * Us[s1] + c2 * Us[s2];
-            qu = qu - sumu;
-            double sumv = bs * Vs[s0] + c1 * Vs[s1] + c2 * Vs[s2];
-            qv = qv - sumv;
-            double sumt = ts * Ts[s0] + t1 * Ts[s1] + t2 * Ts[s2];
-            qt = qt - sumt;
-            sumu = bs * UPs[s0] + c1 * UPs[s1] + c2 * UPs[s2];
-            qup = qup - sumu;
-            sumv = bs * VPs[s0] + c1 * VPs[s1] + c2 * VPs[s2];
-            qvp = qvp - sumv;
-        }
-        fb[P_RU * ps + k] = qu;
-        fb[P_RV * ps + k] = qv;
-        fb[P_RT * ps + k] = qt;
-        fb[P_RUP * ps + k] = qup;
-        fb[P_RVP * ps + k] = qvp;
-        // seed the iterates (PSolver.cpp:1241-1337): u*, v*, T from the current fields;
-        // up/vp from the previous solution (warm start) or zero. A solve predicted to stop
-        // after an odd number of sweeps starts in the scratch plane, so that its result
-        // ends in the iterate plane (the prediction is the previous step's parity; FP64 form)
-        auto X0 = [&](int f) { return ((nextm >> f) & 1) ? Bp(f) : Ap(f); };
-        store_mirrored(X0(F_U), ld, i, j, W, per, uc);
-        store_mirrored(X0(F_V), ld, i, j, W, per, vc);
-        store_mirrored(X0(F_T), ld, i, j, W, per, tc);
-        store_mirrored(X0(F_UP), ld, i, j, W, per, warm ? UPs[o] : 0.0);
-        store_mirrored(X0(F_VP), ld, i, j, W, per, warm ? VPs[o] : 0.0);
-        // boundary values the stencils read (both iterate buffers)
-        auto put_bnd = [&](int bi, int bj) {
-            const long long kb = (long long)bj * ld + bi;
-            const bool zero_far = !cav && bj == n1 - 1;  // up/vp solves see zero on the far row
-#pragma unroll 1
-            for (int f = 0; f < NFIELD; f++) {
-                const double* src = f == F_U ? U : f == F_V ? V : f == F_T ? T : f == F_UP ? UP : VP;
-                const double val = (zero_far && f >= F_UP) ? 0.0 : src[kb];
-                store_mirrored(Ap(f), ld, bi, bj, W, per, val);
-                store_mirrored(Bp(f), ld, bi, bj, W, per, val);
-            }
-        };
-        if (j == 1) put_bnd(i, 0);
-        if (j == n1 - 2) put_bnd(i, n1 - 1);
-        if (cav) {
-            if (i == 1) {
-                put_bnd(0, j);
-                if (j == 1) put_bnd(0, 0);
-                if (j == n1 - 2) put_bnd(0, n1 - 1);
-            }
-            if (i == n0 - 2) {
-                put_bnd(n0 - 1, j);
-                if (j == 1) put_bnd(n0 - 1, 0);
-                if (j == n1 - 2) put_bnd(n0 - 1, n1 - 1);
-            }
-        }
+        const RhsOut r = rhs_cell(rc, i, j, Us, Vs, Ts, Ps, UPs, VPs, o, JTW, SI[oi], SI[TX * TYJ + oi],
+                                  SI[2 * TX * TYJ + oi], SI[3 * TX * TYJ + oi], SI[4 * TX * TYJ + oi],
+                                  SI[5 * TX * TYJ + oi], SI + 6 * TX * TYJ + oi);
+        fb[P_RU * ps + k] = r.qu;
+        fb[P_RV * ps + k] = r.qv;
+        fb[P_RT * ps + k] = r.qt;
+        fb[P_RUP * ps + k] = r.qup;
+        fb[P_RVP * ps + k] = r.qvp;
+        const double seed[NFIELD] = {Us[o], Vs[o], Ts[o], warm ? UPs[o] : 0.0, warm ? VPs[o] : 0.0};
+        rhs_seed(fb, ps, nextm, cur, ld, W, per, cav, n0, n1, i, j, seed);
     }
 }
 
@@ -421,8 +207,8 @@ __global__ void __launch_bounds__(BC_THREADS) k_upbc(BatchDev b) {
             a = U[k];
             bb = V[k];
         } else {
-            a = (5.0 * UP[k - ld] - 4.0 * UP[k - 2LL * ld] + UP[k - 3LL * ld]) / 2.0;
-            bb = (5.0 * VP[k - ld] - 4.0 * VP[k - 2LL * ld] + VP[k - 3LL * ld]) / 2.0;
+            a = upbc_out(UP, k, ld);
+            bb = upbc_out(VP, k, ld);
         }
         store_mirrored(UP, ld, i, j, c.W, 1, a);
         store_mirrored(VP, ld, i, j, c.W, 1, bb);
@@ -459,10 +245,7 @@ __global__ void __launch_bounds__(NT, 4) k_face_q(BatchDev b) {
     double* QP = plane(b, c, P_Q);
     double* KRP = plane(b, c, P_KR);
     float* B0 = mplane(b, c.lev[0], M_B);
-    // reciprocals once per thread: the per-cell quotients become products (each within an
-    // ulp of the quotient; 1 / (4 d) is 0.25 / d exactly)
-    const double dt = c.dt, rd0 = 1.0 / c.d0, rd1 = 1.0 / c.d1, q0 = 0.25 * rd0, q1 = 0.25 * rd1;
-    const double hdt = 0.5 * dt, rdt = 1.0 / dt;
+    const FaceCase fc(c);
     __syncthreads();
     const bool ok = __syncthreads_and(mbar_wait_bounded(&bar, 0, b.wait_polls));
     if (!ok) {
@@ -481,29 +264,7 @@ __global__ void __launch_bounds__(NT, 4) k_face_q(BatchDev b) {
         const int j = t.j0 + lj + h * TY;
         if (!ok || i < ilo || i > ihi || j > n1 - 2) continue;
         const int k = (lj + h * TY + 2) * JTW + (li + 2);
-        const int kE = k + 1, kW = k - 1, kN = k + JTW, kS = k - JTW;
-        double dpdxi_ip = (P[kE] - P[k]) * rd0;
-        double dpde_ip = (P[kN + 1] + P[kN] - P[kS] - P[kS + 1]) * q1;
-        double dpdxi_in = (P[k] - P[kW]) * rd0;
-        double dpde_in = (P[kN] + P[kN - 1] - P[kS] - P[kS - 1]) * q1;
-        double dpdxi_jp = (P[kN + 1] - P[kN - 1] + P[kE] - P[kW]) * q0;
-        double dpde_jp = (P[kN] - P[k]) * rd1;
-        double dpdxi_jn = (P[kE] - P[kW] + P[kS + 1] - P[kS - 1]) * q0;
-        double dpde_jn = (P[k] - P[kS]) * rd1;
-        double us_ip = 0.5 * (U[k] + U[kE]) - hdt * ((X[k] + X[kE]) * dpdxi_ip + (E[k] + E[kE]) * dpde_ip);
-        double us_in = 0.5 * (U[k] + U[kW]) - hdt * ((X[k] + X[kW]) * dpdxi_in + (E[k] + E[kW]) * dpde_in);
-        double us_jp = 0.5 * (U[k] + U[kN]) - hdt * ((X[k] + X[kN]) * dpdxi_jp + (E[k] + E[kN]) * dpde_jp);
-        double us_jn = 0.5 * (U[k] + U[kS]) - hdt * ((X[k] + X[kS]) * dpdxi_jn + (E[k] + E[kS]) * dpde_jn);
-        double vs_ip = 0.5 * (V[k] + V[kE]) - hdt * ((Y[k] + Y[kE]) * dpdxi_ip + (G[k] + G[kE]) * dpde_ip);
-        double vs_in = 0.5 * (V[k] + V[kW]) - hdt * ((Y[k] + Y[kW]) * dpdxi_in + (G[k] + G[kW]) * dpde_in);
-        double vs_jp = 0.5 * (V[k] + V[kN]) - hdt * ((Y[k] + Y[kN]) * dpdxi_jp + (G[k] + G[kN]) * dpde_jp);
-        double vs_jn = 0.5 * (V[k] + V[kS]) - hdt * ((Y[k] + Y[kS]) * dpdxi_jn + (G[k] + G[kS]) * dpde_jn);
-        double dusdxi = (us_ip - us_in) * rd0;
-        double dusde = (us_jp - us_jn) * rd1;
-        double dvsdxi = (vs_ip - vs_in) * rd0;
-        double dvsde = (vs_jp - vs_jn) * rd1;
-        double qq = (X[k] * dusdxi) + (E[k] * dusde) + (Y[k] * dvsdxi) + (G[k] * dvsde);
-        const double q = qq * rdt;
+        const double q = face_cell(fc, P, U, V, X, Y, E, G, k, JTW, U[k + JTW], V[k + JTW]);
         // q doubles as BiCGStab's shadow residual r_hat; p, v and the iterate pcor are
         // initialised by the first iteration's kernels (beta = 0, x = 0)
         const long long kg = (long long)j * ld + i;
@@ -584,7 +345,6 @@ __global__ void __launch_bounds__(NT, 3) k_bicg_p(BatchDev b) {
         const double p = r[h] + beta * (po[h] - omega * v[h]);
         Pv[k[h]] = p;
         mplane(b, L, M_B)[(long long)j * L.ld + i] = (float)p;
-        store_mirrored(mplane(b, L, M_X), L.ld, i, j, L.W, c.periodic, 0.0f);
     }
 }
 
@@ -611,11 +371,7 @@ __global__ void __launch_bounds__(NT, 5) k_spmv(BatchDev b, int mode) {
         const long long kk = (long long)jj * ld + ii, q = (long long)jj * l0 + ii;
         k[h] = kk;
         xc[h] = (double)X[q];
-        y[h] = plane(b, c, P_AP)[kk] * xc[h] + plane(b, c, P_AE)[kk] * (double)X[q + 1] +
-               plane(b, c, P_AW)[kk] * (double)X[q - 1] + plane(b, c, P_AN)[kk] * (double)X[q + l0] +
-               plane(b, c, P_AS)[kk] * (double)X[q - l0] + plane(b, c, P_ANE)[kk] * (double)X[q + l0 + 1] +
-               plane(b, c, P_ANW)[kk] * (double)X[q + l0 - 1] + plane(b, c, P_ASE)[kk] * (double)X[q - l0 + 1] +
-               plane(b, c, P_ASW)[kk] * (double)X[q - l0 - 1];
+        y[h] = spmv_cell(plane(b, c, P_AP), c.ps, kk, X, q, l0, xc[h]);
         dv[h] = DOT[kk];
     }
     double red[2] = {0.0, 0.0};
@@ -686,7 +442,6 @@ __global__ void __launch_bounds__(NT, 5) k_bicg_s(BatchDev b) {
         plane(b, c, P_KS)[k[h]] = s;
         store_mirrored(X, c.ld, i, j, c.W, c.periodic, x);
         mplane(b, L, M_B)[(long long)j * L.ld + i] = (float)s;
-        store_mirrored(mplane(b, L, M_X), L.ld, i, j, L.W, c.periodic, 0.0f);
         red[0] += fabs(s);
     }
     if (case_reduce<1, 0u>(b, t.c, blockIdx.x, c.jt_begin, c.jt_count, red) && threadIdx.x == 0) {
@@ -773,24 +528,9 @@ __global__ void __launch_bounds__(NT, 5) k_bicg_x(BatchDev b, int maxit) {
 // CTA schedule), as the Krylov method needs. The level's final result lives in r (x for a
 // case whose coarsest level it is).
 
-// stored column of level column gi, gi in [-W, inf): the periodic wrap without a division
-// in the common case (gi within one width of the level)
-__device__ __forceinline__ int mg_wrap(int gi, int W) {
-    int col = gi < 0 ? gi + W : gi;
-    if (col >= W) col = col >= 2 * W ? col % W : col - W;
-    return col;
-}
-
-__device__ __forceinline__ int mg_colour(int i, int j, int W, int periodic) {
-    // 4 colours by parity; an odd periodic width gets 2 extra colours for its last column
-    if (periodic && (W & 1) && i == W - 1) return 4 + (j & 1);
-    return (i & 1) | ((j & 1) << 1);
-}
-
-
 // Residual r = b - A x of level l on the fine points a coarse tile of level l + 1 needs,
 // in shared memory, then full-weighting restriction into b_{l+1} (tiles of level l + 1;
-// x_{l+1} is zeroed for the coarse solve). Fine points that are not unknowns contribute 0.
+// levels start from x = 0 on their own). Fine points that are not unknowns contribute 0.
 __global__ void __launch_bounds__(NT) k_mg_rr(BatchDev b, int l, int src) {
     constexpr int RW = 2 * TX + 1, RH = 2 * TY + 1;  // fine residual region
     constexpr int XW = RW + 2, XH = RH + 2;          // fine x region (one-cell halo)
@@ -839,328 +579,30 @@ __global__ void __launch_bounds__(NT) k_mg_rr(BatchDev b, int l, int src) {
                     0.125f * (rs[f - RW] + rs[f + RW] + rs[f - 1] + rs[f + 1]) + 0.25f * rs[f];
     const long long kc = (long long)J * C.ld + I;
     mplane(b, C, M_B)[kc] = v;
-    store_mirrored(mplane(b, C, M_X), C.ld, I, J, C.W, per, 0.0f);
 }
 
-// Pre-smoothing folded into the residual + restriction pass (schedule form `fused` = 2).
-// One CTA per 32 x 8 tile of level l + 1. Its fine region E (the 65 x 17 fine points the
-// restriction reads plus a one-cell ring: 67 x 19) is smoothed from zero in shared memory,
-// zero outside E, by `inner` multicolour Gauss-Seidel sweeps; the residual is formed from
-// that x and restricted into b_{l+1}; x is stored for the fine points the tile owns
-// (columns 2 i0 .. 2 i0 + 63, rows 2 j0 - 1 .. 2 j0 + 14, and in the last tile row also the
-// rows up to n1 - 2), where the post-smoother starts. Neighbouring regions overlap by up to
-// three cells, and on a region's ring the residual uses the region's own smoothed x, not
-// the owner's stored one. The V-cycle stays a fixed linear map (each CTA reads only level
-// planes no CTA of the launch writes); it is a different map from form 1's, with the
-// level's pre-smoothing pass and its read of the stencil saved.
-constexpr int MPR_EW = 2 * TX + 3, MPR_EH = 2 * TY + 3;  // smoothed region E
-constexpr int MPR_RW = 2 * TX + 1, MPR_RH = 2 * TY + 1;  // fine residual region
-constexpr int MPR_BX = (MPR_EW + 1) / 2, MPR_BY = (MPR_EH + 1) / 2;  // 2 x 2 blocks of E: 34 x 10
-// x of E with a zero ring (69 x 21 points), split by column parity; a parity half has rows
-// of 40 words, and the second half starts 16 banks after the first
-constexpr int MPR_XW = MPR_EW + 2, MPR_XH = MPR_EH + 2;
-constexpr int MPR_XS = 40, MPR_XP = MPR_XH * MPR_XS + 8;
-static_assert(MPR_XS >= (MPR_XW + 1) / 2 && MPR_XP % 32 == 16, "split layout of the region's x");
-static_assert(MG_PRR_THREADS >= MPR_BX * MPR_BY && MG_PRR_THREADS >= TX * TY && MG_PRR_THREADS % 32 == 0,
-              "one thread per 2 x 2 block of E, one per coarse point");
-
-__device__ __forceinline__ int mpr_at(int xx, int ry) {  // point (xx, ry) of the ringed region
-    return (xx & 1) * MPR_XP + ry * MPR_XS + (xx >> 1);
-}
-// the fine residual region (65 x 17 points), split by column parity like x: the blocks write
-// it and the restriction reads it at column stride 2, which a plain row-major tile serves
-// with two-way bank conflicts; split, consecutive threads touch consecutive words
-constexpr int MPR_RS = 33, MPR_RP = MPR_RH * MPR_RS + 16;
-__device__ __forceinline__ int mpr_rat(int x, int y) { return (x & 1) * MPR_RP + y * MPR_RS + (x >> 1); }
-
-// Each thread owns one 2 x 2 block of E, which holds one point of each colour (E starts at
-// an even column and row, and a level with a coarser one has an even width when periodic,
-// so the colours are the four parity classes); its four stencils stay in registers.
+// pre-smoothing folded into the residual + restriction pass (mg_prr_tile): one CTA per
+// 32 x 8 tile of level l + 1
 __global__ void __launch_bounds__(MG_PRR_THREADS, 3) k_mg_prr(BatchDev b, int l, int dst, int inner) {
     __shared__ float xs[2 * MPR_XP];
     __shared__ float rs[2 * MPR_RP];
     const Tile t = b.atiles[l + 1][blockIdx.x];
     if (b.iscal[(long long)t.c * NISCAL + I_PDONE]) return;
     const CaseDev& c = b.cases[t.c];
-    const LevelDev& F = c.lev[l];
-    const LevelDev& C = c.lev[l + 1];
-    const int tid = threadIdx.x;
-    const int fl = F.ld, W = F.W, per = c.periodic, n1 = F.n1;
-    if (per && (W & 1)) {
-        if (tid == 0) atomicExch(b.error, 1);
-        return;
-    }
-    const int ei0 = 2 * t.i0 - 2, ej0 = 2 * t.j0 - 2;  // level-l (column, row) of E's first point
-    const bool own = tid < MPR_BX * MPR_BY;
-    const int bx = own ? tid % MPR_BX : 0, by = own ? tid / MPR_BX : 0;
-    const int gi0 = ei0 + 2 * bx;
-    int c0, c1;  // stored columns of the block's two columns (c1 = c0 + 1 when both exist)
-    if (per) {
-        c0 = mg_wrap(gi0, W);
-        c1 = c0 + 1;
-    } else {
-        c0 = (gi0 >= 0 && gi0 < W) ? gi0 : -1;
-        c1 = (gi0 + 1 >= 0 && gi0 + 1 < W) ? gi0 + 1 : -1;
-    }
-    float a[2][2][10];  // [dy][dx][ap, ae, aw, an, as, ane, anw, ase, asw, b]
-    bool ok[2][2];
-#pragma unroll
-    for (int dy = 0; dy < 2; dy++) {
-        const int gj = ej0 + 2 * by + dy;
-        const bool rowok = own && gj >= 1 && gj <= n1 - 2 && 2 * by + dy < MPR_EH;
-        ok[dy][0] = rowok && c0 >= F.ilo && c0 <= F.ihi;
-        ok[dy][1] = rowok && c1 >= F.ilo && c1 <= F.ihi && 2 * bx + 1 < MPR_EW;
-        // the even column and its right neighbour, 8-byte aligned (safe row / column outside)
-        const long long k = (long long)((gj >= 0 && gj < n1) ? gj : 1) * fl + (c0 >= 0 ? c0 : 0);
-#pragma unroll
-        for (int q = 0; q < 10; q++) {
-            const float2 v = *reinterpret_cast<const float2*>(mplane(b, F, q < 9 ? M_AP + q : M_B) + k);
-            a[dy][0][q] = v.x;
-            a[dy][1][q] = v.y;
-        }
-    }
-    for (int e = tid; e < 2 * MPR_XP; e += MG_PRR_THREADS) xs[e] = 0.0f;
-    __syncthreads();
-    // point of colour cc in the block: (dx, dy) = (cc & 1, cc >> 1); its ringed position is
-    // (2 bx + dx + 1, 2 by + dy + 1)
-    float xr[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};
-    // the first sweep from zero: a colour's neighbours of the colours not yet relaxed are
-    // still zero, so colour 0 reads none, colour 1 its E/W neighbours (colour 0), colour 2
-    // its N/S (colour 0) and diagonal (colour 1) neighbours, colour 3 all eight
-    auto relax0 = [&](auto cc_) {
-        constexpr int cc = decltype(cc_)::value;
-        constexpr int dx = cc & 1, dy = cc >> 1;
-        if (ok[dy][dx]) {
-            const float(&f)[10] = a[dy][dx];
-            const int xx = 2 * bx + dx + 1, ry = 2 * by + dy + 1;
-            float sm = 0.0f;
-            if (cc == 1) sm = f[1] * xs[mpr_at(xx + 1, ry)] + f[2] * xs[mpr_at(xx - 1, ry)];
-            if (cc == 2)
-                sm = f[3] * xs[mpr_at(xx, ry + 1)] + f[4] * xs[mpr_at(xx, ry - 1)] +
-                     f[5] * xs[mpr_at(xx + 1, ry + 1)] + f[6] * xs[mpr_at(xx - 1, ry + 1)] +
-                     f[7] * xs[mpr_at(xx + 1, ry - 1)] + f[8] * xs[mpr_at(xx - 1, ry - 1)];
-            if (cc == 3)
-                sm = f[1] * xs[mpr_at(xx + 1, ry)] + f[2] * xs[mpr_at(xx - 1, ry)] +
-                     f[3] * xs[mpr_at(xx, ry + 1)] + f[4] * xs[mpr_at(xx, ry - 1)] +
-                     f[5] * xs[mpr_at(xx + 1, ry + 1)] + f[6] * xs[mpr_at(xx - 1, ry + 1)] +
-                     f[7] * xs[mpr_at(xx + 1, ry - 1)] + f[8] * xs[mpr_at(xx - 1, ry - 1)];
-            const float v = (f[9] - sm) / f[0];
-            xs[mpr_at(xx, ry)] = v;
-            xr[dy][dx] = v;
-        }
-        __syncthreads();
-    };
-    auto relax = [&](auto cc_) {
-        constexpr int cc = decltype(cc_)::value;
-        constexpr int dx = cc & 1, dy = cc >> 1;
-        if (ok[dy][dx]) {
-            const float(&f)[10] = a[dy][dx];
-            const int xx = 2 * bx + dx + 1, ry = 2 * by + dy + 1;
-            const float sm = f[1] * xs[mpr_at(xx + 1, ry)] + f[2] * xs[mpr_at(xx - 1, ry)] +
-                             f[3] * xs[mpr_at(xx, ry + 1)] + f[4] * xs[mpr_at(xx, ry - 1)] +
-                             f[5] * xs[mpr_at(xx + 1, ry + 1)] + f[6] * xs[mpr_at(xx - 1, ry + 1)] +
-                             f[7] * xs[mpr_at(xx + 1, ry - 1)] + f[8] * xs[mpr_at(xx - 1, ry - 1)];
-            const float v = (f[9] - sm) / f[0];
-            xs[mpr_at(xx, ry)] = v;
-            xr[dy][dx] = v;
-        }
-        __syncthreads();
-    };
-    using C0 = std::integral_constant<int, 0>;
-    using C1 = std::integral_constant<int, 1>;
-    using C2 = std::integral_constant<int, 2>;
-    using C3 = std::integral_constant<int, 3>;
-    if (inner > 0) {
-        relax0(C0{}); relax0(C1{}); relax0(C2{}); relax0(C3{});
-    }
-    for (int n = 1; n < inner; n++) {
-        relax(C0{}); relax(C1{}); relax(C2{}); relax(C3{});
-    }
-    // residual on the restriction's fine points (E without its ring), x of the owned points
-    float* OUT = mplane(b, F, dst);
-    const int jhi = (t.j0 + TY > C.n1 - 2) ? n1 - 2 : min(2 * t.j0 + 14, n1 - 2);
-#pragma unroll
-    for (int dy = 0; dy < 2; dy++)
-#pragma unroll
-        for (int dx = 0; dx < 2; dx++) {
-            const int x = 2 * bx + dx, y = 2 * by + dy;
-            if (!own || x < 1 || x > MPR_RW || y < 1 || y > MPR_RH) continue;
-            float r = 0.0f;
-            if (ok[dy][dx]) {
-                const float(&f)[10] = a[dy][dx];
-                const int xx = x + 1, ry = y + 1;
-                const float ax = f[0] * xr[dy][dx] + f[1] * xs[mpr_at(xx + 1, ry)] + f[2] * xs[mpr_at(xx - 1, ry)] +
-                                 f[3] * xs[mpr_at(xx, ry + 1)] + f[4] * xs[mpr_at(xx, ry - 1)] +
-                                 f[5] * xs[mpr_at(xx + 1, ry + 1)] + f[6] * xs[mpr_at(xx - 1, ry + 1)] +
-                                 f[7] * xs[mpr_at(xx + 1, ry - 1)] + f[8] * xs[mpr_at(xx - 1, ry - 1)];
-                r = f[9] - ax;
-            }
-            rs[mpr_rat(x - 1, y - 1)] = r;
-            // owned: columns 2 i0 .. 2 i0 + 63 (E columns 2 .. 65), rows 2 j0 - 1 .. jhi
-            const int gi = ei0 + x, gj = ej0 + y;
-            if (x >= 2 && gi >= F.ilo && gi <= F.ihi && gj <= jhi)
-                store_mirrored(OUT, fl, gi, gj, W, per, ok[dy][dx] ? xr[dy][dx] : 0.0f);
-        }
-    __syncthreads();
-    if (tid >= TX * TY) return;
-    const int li = tid % TX, lj = tid / TX;
-    const int I = t.i0 + li, J = t.j0 + lj;
-    if (I < C.ilo || I > C.ihi || J > C.n1 - 2) return;
-    const int fx = 2 * li + 1, fy = 2 * lj + 1;  // fine (2I, 2J) in the residual region
-    const float r4 = 0.0625f * (rs[mpr_rat(fx - 1, fy - 1)] + rs[mpr_rat(fx + 1, fy - 1)] + rs[mpr_rat(fx - 1, fy + 1)] +
-                                rs[mpr_rat(fx + 1, fy + 1)]) +
-                     0.125f * (rs[mpr_rat(fx, fy - 1)] + rs[mpr_rat(fx, fy + 1)] + rs[mpr_rat(fx - 1, fy)] +
-                               rs[mpr_rat(fx + 1, fy)]) +
-                     0.25f * rs[mpr_rat(fx, fy)];
-    mplane(b, C, M_B)[(long long)J * C.ld + I] = r4;
-    store_mirrored(mplane(b, C, M_X), C.ld, I, J, C.W, per, 0.0f);
+    mg_prr_tile(b, c, l, t.i0, t.j0, dst, inner, xs, rs, BlockGroup<MG_PRR_THREADS>());
 }
 
-// bilinear prolongation of the coarse result at fine point (i, j), i in [0, W)
-__device__ __forceinline__ float mg_prolong_at(const float* XC, int cl, int i, int j) {
-    const int I = i >> 1, J = j >> 1;
-    const long long q = (long long)J * cl + I;
-    if (!(i & 1) && !(j & 1)) return XC[q];
-    if (!(j & 1)) return 0.5f * (XC[q] + XC[q + 1]);
-    if (!(i & 1)) return 0.5f * (XC[q] + XC[q + cl]);
-    return 0.25f * (XC[q] + XC[q + 1] + XC[q + cl] + XC[q + cl + 1]);
-}
-
-// Multicolour Gauss-Seidel sweeps of level l on a 32 x 16 tile (block Gauss-Seidel at tile
-// edges: the halo ring holds the neighbouring tiles' values from before the first sweep).
-// The sweeps read plane `src` and write plane `dst` != src, so nothing is read that another
-// CTA writes.
-//   mode 0: from x = 0, colours in order (first pre-sweep; src unused)
-//   mode 1: from src, colours in order (further pre-sweeps)
-//   mode 2: from src plus the prolonged result of level l + 1, colours reversed (first
-//           post-sweep)
-//   mode 3: from src, colours reversed (further post-sweeps)
-// `inner` sweeps run back to back in shared memory (one launch and one read of the stencil
-// for several sweeps, at the price of weaker coupling between tiles).
-//
-// A level with a coarser one has an even width when periodic, so its colours are the four
-// parity classes. Tiles start at an even column and an odd row, so every 2 x 2 block of the
-// tile holds one point of each colour: a thread owns one block (16 x 8 blocks, 128
-// threads), keeps its four stencils in registers (loaded as column pairs) and relaxes one
-// point per colour. x with its halo is held in shared memory split by column parity, rows
-// padded so that a warp's two block rows fall in different banks: every read of a
-// colour pass is free of bank conflicts.
-constexpr int MG_GS_XW = TX + 2, MG_GS_XH = TYJ + 2;  // x halo region
-constexpr int MG_GS_XS = 24;                           // row stride of a parity half
-constexpr int MG_GS_XP = MG_GS_XH * MG_GS_XS;          // 432 = 16 mod 32 words
-static_assert(MG_GS_XS >= (MG_GS_XW + 1) / 2 && (2 * MG_GS_XS) % 32 == 16 && MG_GS_XP % 32 == 16,
-              "parity halves must keep a colour pass free of bank conflicts");
-static_assert(MG_GS_THREADS == (TX / 2) * (TYJ / 2), "one thread per 2 x 2 block");
-
-__device__ __forceinline__ int mg_gs_at(int xx, int ry) {  // halo point (xx, ry) in the split layout
-    return (xx & 1) * MG_GS_XP + ry * MG_GS_XS + (xx >> 1);
-}
-
+// multicolour Gauss-Seidel sweeps of level l on a 32 x 16 tile (mg_gs_tile)
 __global__ void __launch_bounds__(MG_GS_THREADS, 8) k_mg_gs(BatchDev b, int l, int mode, int src, int dst, int inner) {
     __shared__ float xs[2 * MG_GS_XP];
     const Tile t = b.mtiles[l][blockIdx.x];
     if (b.iscal[(long long)t.c * NISCAL + I_PDONE]) return;
     const CaseDev& c = b.cases[t.c];
-    const LevelDev& L = c.lev[l];
-    const int tid = threadIdx.x;
-    const int ld = L.ld, W = L.W, per = c.periodic, n1 = L.n1;
-    if (per && (W & 1)) {
-        if (tid == 0) atomicExch(b.error, 1);
-        return;
-    }
-    const bool zero = mode == 0, prolong = mode == 2, reverse = mode >= 2;
-    const float* X = mplane(b, L, src);
-    const float* XC = prolong ? mplane(b, c.lev[l + 1], mg_result_plane(b, c, l + 1)) : nullptr;
-    const int cl = prolong ? c.lev[l + 1].ld : 0;
-    // stored column of level column gi (periodic wrap), or -1 outside the level
-    auto column = [&](int gi) -> int {
-        if (per) return mg_wrap(gi, W);
-        return (gi >= 0 && gi < W) ? gi : -1;
-    };
-    // this thread's 2 x 2 block: tile columns 2 bx, 2 bx + 1, rows 2 by, 2 by + 1
-    const int bx = tid % (TX / 2), by = tid / (TX / 2);
-    const int gi0 = t.i0 + 2 * bx;
-    const int c0 = column(gi0), c1 = column(gi0 + 1);  // c1 = c0 + 1 whenever both are in the level
-    float a[2][2][10];  // [dy][dx][ap^-1, ae, aw, an, as, ane, anw, ase, asw, b]
-    bool ok[2][2];
-#pragma unroll
-    for (int dy = 0; dy < 2; dy++) {
-        const int gj = t.j0 + 2 * by + dy;
-        ok[dy][0] = gj >= 1 && gj <= n1 - 2 && c0 >= L.ilo && c0 <= L.ihi;
-        ok[dy][1] = gj >= 1 && gj <= n1 - 2 && c1 >= L.ilo && c1 <= L.ihi;
-        // an even column and its right neighbour, 8-byte aligned (safe row / column when outside)
-        const long long k = (long long)((gj >= 0 && gj < n1) ? gj : 1) * ld + (c0 >= 0 ? c0 : 0);
-#pragma unroll
-        for (int q = 0; q < 10; q++) {
-            const float2 v = *reinterpret_cast<const float2*>(mplane(b, L, q < 9 ? M_AP + q : M_B) + k);
-            a[dy][0][q] = v.x;
-            a[dy][1][q] = v.y;
-        }
-    }
-    // x and its halo (with the prolonged coarse correction in mode 2)
-    constexpr int NXL = (MG_GS_XW * MG_GS_XH + MG_GS_THREADS - 1) / MG_GS_THREADS;
-    float xv[NXL];
-#pragma unroll
-    for (int m = 0; m < NXL; m++) {
-        const int e = tid + m * MG_GS_THREADS;
-        const int gj = t.j0 - 1 + e / MG_GS_XW, col = column(t.i0 - 1 + e % MG_GS_XW);
-        float v = 0.0f;
-        if (!zero && e < MG_GS_XW * MG_GS_XH && gj >= 0 && gj < n1 && col >= 0) {
-            v = X[(long long)gj * ld + col];
-            if (prolong && gj >= 1 && gj <= n1 - 2 && col >= L.ilo && col <= L.ihi)
-                v += mg_prolong_at(XC, cl, col, gj);
-        }
-        xv[m] = v;
-    }
-#pragma unroll
-    for (int m = 0; m < NXL; m++) {
-        const int e = tid + m * MG_GS_THREADS;
-        if (e < MG_GS_XW * MG_GS_XH) xs[mg_gs_at(e % MG_GS_XW, e / MG_GS_XW)] = xv[m];
-    }
-#pragma unroll
-    for (int dy = 0; dy < 2; dy++)
-#pragma unroll
-        for (int dx = 0; dx < 2; dx++) a[dy][dx][0] = ok[dy][dx] ? 1.0f / a[dy][dx][0] : 0.0f;
-    __syncthreads();
-    // point of colour cc in this thread's block: (dx, dy) = (cc & 1, 1 - (cc >> 1)) (the tile's
-    // first row is odd); its halo position is (2 bx + dx + 1, 2 by + dy + 1)
-    auto relax = [&](auto cc_) {
-        constexpr int cc = decltype(cc_)::value;
-        constexpr int dx = cc & 1, dy = 1 - (cc >> 1);
-        if (ok[dy][dx]) {
-            const float(&f)[10] = a[dy][dx];
-            const int xx = 2 * bx + dx + 1, ry = 2 * by + dy + 1;
-            const float sm = f[1] * xs[mg_gs_at(xx + 1, ry)] + f[2] * xs[mg_gs_at(xx - 1, ry)] +
-                             f[3] * xs[mg_gs_at(xx, ry + 1)] + f[4] * xs[mg_gs_at(xx, ry - 1)] +
-                             f[5] * xs[mg_gs_at(xx + 1, ry + 1)] + f[6] * xs[mg_gs_at(xx - 1, ry + 1)] +
-                             f[7] * xs[mg_gs_at(xx + 1, ry - 1)] + f[8] * xs[mg_gs_at(xx - 1, ry - 1)];
-            xs[mg_gs_at(xx, ry)] = (f[9] - sm) * f[0];
-        }
-        __syncthreads();
-    };
-    using C0 = std::integral_constant<int, 0>;
-    using C1 = std::integral_constant<int, 1>;
-    using C2 = std::integral_constant<int, 2>;
-    using C3 = std::integral_constant<int, 3>;
-    for (int n = 0; n < inner; n++) {
-        if (reverse) { relax(C3{}); relax(C2{}); relax(C1{}); relax(C0{}); }
-        else { relax(C0{}); relax(C1{}); relax(C2{}); relax(C3{}); }
-    }
-    float* OUT = mplane(b, L, dst);
-#pragma unroll
-    for (int dy = 0; dy < 2; dy++)
-#pragma unroll
-        for (int dx = 0; dx < 2; dx++) {
-            const int i = gi0 + dx, j = t.j0 + 2 * by + dy;
-            if (i < L.ilo || i > L.ihi || j > n1 - 2) continue;
-            store_mirrored(OUT, ld, i, j, W, per, xs[mg_gs_at(2 * bx + dx + 1, 2 * by + dy + 1)]);
-        }
+    mg_gs_tile(b, c, l, t.i0, t.j0, mode, src, dst, inner, xs, BlockGroup<MG_GS_THREADS>());
 }
 
-// coarsest level: `sweeps` multicolour GS sweeps by one CTA per case, x in shared memory
-// and each thread's stencil in registers when the level fits (one unknown per thread);
-// larger levels (a case whose grid does not coarsen) sweep through global memory
-constexpr int MGC_THREADS = 1024, MGC_SMEM = 4096;
+// coarsest level: `sweeps` multicolour GS sweeps by one CTA per case (mg_coarse_solve)
+constexpr int MGC_THREADS = 1024, MGC_SMEM = 6144;
 __global__ void __launch_bounds__(MGC_THREADS) k_mg_coarse(BatchDev b, int l, int sweeps) {
     __shared__ float xs[MGC_SMEM];
     // l < 0: one launch for every case, each on its own coarsest level (the case lists of
@@ -1168,67 +610,7 @@ __global__ void __launch_bounds__(MGC_THREADS) k_mg_coarse(BatchDev b, int l, in
     const int cid = l >= 0 ? b.ccases[l][blockIdx.x] : b.ccases[0][blockIdx.x];
     if (b.iscal[(long long)cid * NISCAL + I_PDONE]) return;
     const CaseDev& c = b.cases[cid];
-    const LevelDev& L = c.lev[l >= 0 ? l : c.nlev - 1];
-    const int ld = L.ld, per = c.periodic;
-    const int nx = L.ihi - L.ilo + 1, ny = L.n1 - 2;
-    float* X = mplane(b, L, M_X);
-    const float* Bv = mplane(b, L, M_B);
-    const int ncol = (per && (L.W & 1)) ? 6 : 4;
-    const int sw = L.W + 2 * H;  // shared copy: all rows, columns -H .. W+H-1
-    if (nx * ny <= MGC_THREADS && L.n1 * sw <= MGC_SMEM) {
-        for (int e = threadIdx.x; e < L.n1 * sw; e += MGC_THREADS) xs[e] = 0.0f;  // x = 0 (and boundaries)
-        const int e = threadIdx.x;
-        const bool in = e < nx * ny;
-        const int i = L.ilo + (in ? e % nx : 0), j = 1 + (in ? e / nx : 0);
-        const long long k = (long long)j * ld + i;
-        float ap = 1.f, ae = 0.f, aw = 0.f, an = 0.f, as = 0.f, ane = 0.f, anw = 0.f, ase = 0.f, asw = 0.f, bv = 0.f;
-        int col = -1;
-        if (in) {
-            ap = mplane(b, L, M_AP)[k]; ae = mplane(b, L, M_AE)[k]; aw = mplane(b, L, M_AW)[k];
-            an = mplane(b, L, M_AN)[k]; as = mplane(b, L, M_AS)[k]; ane = mplane(b, L, M_ANE)[k];
-            anw = mplane(b, L, M_ANW)[k]; ase = mplane(b, L, M_ASE)[k]; asw = mplane(b, L, M_ASW)[k];
-            bv = Bv[k];
-            col = mg_colour(i, j, L.W, per);
-        }
-        const int o = j * sw + i + H;
-        const int m = mirror_col(i, L.W, per);
-        __syncthreads();
-        for (int s = 0; s < sweeps; s++) {
-            for (int cc = 0; cc < ncol; cc++) {
-                if (col == cc) {
-                    const float sm = ae * xs[o + 1] + aw * xs[o - 1] + an * xs[o + sw] + as * xs[o - sw] +
-                                     ane * xs[o + sw + 1] + anw * xs[o + sw - 1] + ase * xs[o - sw + 1] +
-                                     asw * xs[o - sw - 1];
-                    const float v = (bv - sm) / ap;
-                    xs[o] = v;
-                    if (m > -1000000) xs[j * sw + m + H] = v;
-                }
-                __syncthreads();
-            }
-        }
-        if (in) store_mirrored(X, ld, i, j, L.W, per, xs[o]);
-        return;
-    }
-    for (int e = threadIdx.x; e < nx * ny; e += blockDim.x) {  // x = 0
-        const int i = L.ilo + e % nx, j = 1 + e / nx;
-        store_mirrored(X, ld, i, j, L.W, per, 0.0f);
-    }
-    __syncthreads();
-    for (int s = 0; s < sweeps; s++) {
-        for (int col = 0; col < ncol; col++) {
-            for (int e = threadIdx.x; e < nx * ny; e += blockDim.x) {
-                const int i = L.ilo + e % nx, j = 1 + e / nx;
-                if (mg_colour(i, j, L.W, per) != col) continue;
-                const long long k = (long long)j * ld + i;
-                const float sm = mplane(b, L, M_AE)[k] * X[k + 1] + mplane(b, L, M_AW)[k] * X[k - 1] +
-                                 mplane(b, L, M_AN)[k] * X[k + ld] + mplane(b, L, M_AS)[k] * X[k - ld] +
-                                 mplane(b, L, M_ANE)[k] * X[k + ld + 1] + mplane(b, L, M_ANW)[k] * X[k + ld - 1] +
-                                 mplane(b, L, M_ASE)[k] * X[k - ld + 1] + mplane(b, L, M_ASW)[k] * X[k - ld - 1];
-                store_mirrored(X, ld, i, j, L.W, per, (Bv[k] - sm) / mplane(b, L, M_AP)[k]);
-            }
-            __syncthreads();
-        }
-    }
+    mg_coarse_solve(b, c, c.lev[l >= 0 ? l : c.nlev - 1], sweeps, xs, MGC_SMEM, BlockGroup<MGC_THREADS>());
 }
 
 // Galerkin coarse operator A_{l+1} = R A_l P (R full weighting, P bilinear, R = P^T / 4)
@@ -1319,7 +701,6 @@ __global__ void __launch_bounds__(NT, 4) k_correct(BatchDev b) {
     const double* VEC = plane(b, c, P_VEC);
     const int i = t.i0 + (int)(threadIdx.x % TX);
     bool in[2];
-    long long kk[2];
     double pc0[2], pn0[2], ps0[2], pe0[2], pw0[2], us[2], vs[2], xix[2], etx[2], xiy[2], ety[2], u0[2], v0[2],
         p0[2];
 #pragma unroll
@@ -1327,7 +708,6 @@ __global__ void __launch_bounds__(NT, 4) k_correct(BatchDev b) {
         const int j = t.j0 + (int)(threadIdx.x / TX) + h * TY;
         in[h] = i >= c.ilo && i <= c.ihi && j <= n1 - 2;
         const long long k = in[h] ? (long long)j * ld + i : (long long)ld + c.ilo;  // a safe cell when out
-        kk[h] = k;
         pc0[h] = PC[k]; pn0[h] = PC[k + ld]; ps0[h] = PC[k - ld]; pe0[h] = PC[k + 1]; pw0[h] = PC[k - 1];
         us[h] = US[k]; vs[h] = VS[k];
         xix[h] = XIX[k]; etx[h] = ETX[k]; xiy[h] = XIY[k]; ety[h] = ETY[k];
@@ -1340,7 +720,6 @@ __global__ void __launch_bounds__(NT, 4) k_correct(BatchDev b) {
     for (int h = 0; h < 2; h++) {
         if (!in[h]) continue;
         const int j = t.j0 + (int)(threadIdx.x / TX) + h * TY;
-        const long long k = kk[h];
         const double pc = none ? 0.0 : pc0[h];
         // pcor on the boundary after its conditions: wall copy, far field 0 / copy at inflow
         const double far = (!cav && vnn >= 0) ? pc : 0.0;
@@ -1348,27 +727,15 @@ __global__ void __launch_bounds__(NT, 4) k_correct(BatchDev b) {
         const double pS = none ? 0.0 : (j == 1) ? pc : ps0[h];
         const double pE = none ? 0.0 : (cav && i == n0 - 2) ? pc : pe0[h];
         const double pW = none ? 0.0 : (cav && i == 1) ? pc : pw0[h];
-        const double dpcor_dxi = (pE - pW) * h0;
-        const double dpcor_de = (pN - pS) * h1;
-        const double un = us[h] - dt * (xix[h] * dpcor_dxi + etx[h] * dpcor_de);
-        const double vn = vs[h] - dt * (xiy[h] * dpcor_dxi + ety[h] * dpcor_de);
-        red[0] += fabs(un - u0[h]) + fabs(vn - v0[h]);
-        store_mirrored(U, ld, i, j, W, per, un);
-        store_mirrored(V, ld, i, j, W, per, vn);
-        const double pn = (c.omega_p == 1.0) ? p0[h] + pc : p0[h] + c.omega_p * pc;
-        store_mirrored(P, ld, i, j, W, per, pn);
+        const CorrOut r = correct_cell(pc, pN, pS, pE, pW, us[h], vs[h], xix[h], xiy[h], etx[h], ety[h], p0[h], h0, h1,
+                                       dt, c.omega_p);
+        red[0] += fabs(r.un - u0[h]) + fabs(r.vn - v0[h]);
+        store_mirrored(U, ld, i, j, W, per, r.un);
+        store_mirrored(V, ld, i, j, W, per, r.vn);
+        store_mirrored(P, ld, i, j, W, per, r.pn);
         if (none) store_mirrored(PC, ld, i, j, W, per, 0.0);
         // record the boundary pcor (output only)
-        if (j == 1) store_mirrored(PC, ld, i, 0, W, per, pc);
-        if (j == n1 - 2) store_mirrored(PC, ld, i, n1 - 1, W, per, cav ? pc : far);
-        if (cav) {
-            if (i == 1) PC[k - 1] = pc;
-            if (i == n0 - 2) PC[k + 1] = pc;
-            if (i == 1 && j == 1) PC[0] = pc;
-            if (i == n0 - 2 && j == 1) PC[n0 - 1] = pc;
-            if (i == 1 && j == n1 - 2) PC[(long long)(n1 - 1) * ld] = pc;
-            if (i == n0 - 2 && j == n1 - 2) PC[(long long)(n1 - 1) * ld + n0 - 1] = pc;
-        }
+        correct_bnd(PC, ld, W, per, cav, n0, n1, i, j, pc, far);
     }
     if (case_reduce<1, 0u>(b, t.c, blockIdx.x, c.jt_begin, c.jt_count, red) && threadIdx.x == 0)
         b.scal[(long long)t.c * NSCAL + S_DUL1] = red[0];
@@ -1381,232 +748,54 @@ __global__ void __launch_bounds__(BC_THREADS, 2) k_bc(BatchDev b) {
     const int cid = blockIdx.x;
     const CaseDev& c = b.cases[cid];
     if (!b.iscal[(long long)cid * NISCAL + I_ACTIVE]) return;
-    const int ld = c.ld, W = c.W, per = c.periodic, n1 = c.n1, n0 = c.n0;
-    const int cur = b.cur, nxt = cur ^ 1;
+    const BcCase a(b, c, b.cur);
+    const int W = c.W, n1 = c.n1, n0 = c.n0;
     const bool cav = c.profile == CAVITY;
-    const double d0 = c.d0, d1 = c.d1, dt = c.dt, Re = c.Re, Ri = c.Ri, Pi = c.Pi;
-    double* U = plane(b, c, P_U);
-    double* V = plane(b, c, P_V);
-    double* Tn = plane(b, c, P_T0 + nxt);
-    const double* To = plane(b, c, P_T0 + cur);
-    double* UPn = plane(b, c, P_UP0 + nxt);
-    double* VPn = plane(b, c, P_VP0 + nxt);
-    double* P = plane(b, c, P_P);
-    double* VORT = plane(b, c, P_VORT);
-    const double* X = plane(b, c, P_X);
-    const double* Yc = plane(b, c, P_Y);
-    const double* XIX = plane(b, c, P_XIX);
-    const double* XIY = plane(b, c, P_XIY);
-    const double* ETX = plane(b, c, P_ETX);
-    const double* ETY = plane(b, c, P_ETY);
-    const double* ALPH = plane(b, c, P_ALPH);
-    const double* BETA = plane(b, c, P_BETA);
-    const double* GAM = plane(b, c, P_GAM);
-    const double* JAC = plane(b, c, P_JAC);
-    const double* VEC = plane(b, c, P_VEC);
     __shared__ double red[16 * 32];
     __shared__ double s_circ;
     int* is = b.iscal + (long long)cid * NISCAL;
     double* sc = b.scal + (long long)cid * NSCAL;
-    const int time_new = (int)((double)is[I_TIME] + dt);
+    const int time_new = (int)((double)is[I_TIME] + c.dt);
     // the time the wall motion sees: the reference's int (PSolver.cpp:186), or t = n dt
-    const double t_new = c.time_accurate ? sc[S_TIME] + dt : (double)time_new;
-    const int jf = n1 - 1;
-    // far-field u/v before this update (uold of PSolver.cpp:1456); W <= 4096
-    extern __shared__ double s_old[];  // 2 * (W + 1)
+    const double t_new = c.time_accurate ? sc[S_TIME] + c.dt : (double)time_new;
+    extern __shared__ double s_old[];  // 2 * (W + 1); W <= 4096
 
     if (!cav) {
-        // circulation at j = n1-2 (PSolver.cpp:1568-1576)
         {
-            const int j = n1 - 2;
-            const double de = c.fix_circ_de ? 1.0 / (n0 - 1) : 1.0 / (n0 - 2);
             double acc[1] = {0.0};
-            for (int i = threadIdx.x; i < W; i += blockDim.x) {
-                const long long k = (long long)j * ld + i, kp = k + 1;
-                double f1 = (U[k] * ETY[k] - V[k] * ETX[k]) * fabs(JAC[k]);
-                double f2 = (U[kp] * ETY[kp] - V[kp] * ETX[kp]) * fabs(JAC[kp]);
-                acc[0] += de * 0.5 * (f1 + f2);
-                const long long kf = (long long)jf * ld + i;
-                s_old[i] = U[kf];
-                s_old[W + 1 + i] = V[kf];
-            }
+            for (int i = threadIdx.x; i < W; i += blockDim.x) acc[0] += bc_circ(a, i, s_old);
             block_sum<1>(acc, red);
             if (threadIdx.x == 0) s_circ = acc[0];
             __syncthreads();
         }
         const double circ = s_circ;
-        const double cwall = cos(2.0 * Pi * c.F * t_new);
+        const double cwall = cos(2.0 * c.Pi * c.F * t_new);
         for (int i = threadIdx.x; i < W; i += blockDim.x) {
-            // vr/vth just inside (PSolver.cpp:1549-1562) and their far-field prediction (:1582-1609)
-            const long long kb = (long long)(jf - 1) * ld + i, k = (long long)jf * ld + i;
-            const double costb = X[kb] / sqrt(X[kb] * X[kb] + Yc[kb] * Yc[kb]);
-            const double sintb = Yc[kb] / sqrt(X[kb] * X[kb] + Yc[kb] * Yc[kb]);
-            const double vr0 = U[kb] * costb + V[kb] * sintb;
-            const double vth0 = -U[kb] * sintb + V[kb] * costb;
-            const double cr = sqrt(X[kb] * X[kb] + Yc[kb] * Yc[kb]) / sqrt(X[k] * X[k] + Yc[k] * Yc[k]);
-            const double costh = X[k] / sqrt(X[k] * X[k] + Yc[k] * Yc[k]);
-            const double sinth = Yc[k] / sqrt(X[k] * X[k] + Yc[k] * Yc[k]);
-            const double vrinf = c.uinf * costh + c.vinf * sinth;
-            const double vtinf = -c.uinf * sinth + c.vinf * costh;
-            const double cr2 = cr * cr;
-            const double crk = fabs(circ) > 1e-2 ? cr : cr2;
-            const double vr1 = vr0 * cr2 + vrinf * (1 - cr2);
-            const double vth1 = vth0 * crk + vtinf * (1 - crk);
-            // far-field u/v/T (PSolver.cpp:1632-1656)
-            const double vnn = c.uinf * VEC[2LL * ld + i] + c.vinf * VEC[3LL * ld + i];
-            double un, vn, tn;
-            if (vnn >= 0) {
-                un = c.uinf; vn = c.vinf; tn = 0.0;
-            } else {
-                un = costh * vr1 - sinth * vth1;
-                vn = sinth * vr1 + costh * vth1;
-                const double uet_old = ETX[k] * s_old[i] + ETY[k] * s_old[W + 1 + i];
-                tn = To[k] - (uet_old * dt / d1) * (To[k] - To[k - ld]);
-            }
-            store_mirrored(U, ld, i, jf, W, per, un);
-            store_mirrored(V, ld, i, jf, W, per, vn);
-            store_mirrored(Tn, ld, i, jf, W, per, tn);
-            // wall velocity (PSolver.cpp:1617-1630)
-            const double uw = -c.speed_amp * cwall * Yc[i];
-            const double vw = c.speed_amp * cwall * X[i];
-            store_mirrored(U, ld, i, 0, W, per, uw);
-            store_mirrored(V, ld, i, 0, W, per, vw);
-            store_mirrored(UPn, ld, i, 0, W, per, uw);
-            store_mirrored(VPn, ld, i, 0, W, per, vw);
+            bc_far(a, i, circ, s_old);
+            bc_wall(a, i, cwall);
         }
         __syncthreads();
-        // boundary pressure (PSolver.cpp:1668-1783)
-        const double swall = sin(2.0 * Pi * c.F * t_new);
-        const double* Fl[2] = {U, V};
+        const double swall = sin(2.0 * c.Pi * c.F * t_new);
         for (int i = threadIdx.x; i < W; i += blockDim.x) {
-            {   // wall, j = 0
-                const long long k = i;
-                double dpd[2];
-                const double uxi = XIX[k] * U[k] + XIY[k] * V[k];
-                const double uet = ETX[k] * U[k] + ETY[k] * V[k];
-                for (int m = 0; m < 2; m++) {
-                    const double* f = Fl[m];
-                    const double aa = ALPH[k] * (f[k + 1] + f[k - 1] - 2 * f[k]) / (d0 * d0);
-                    const double gg = GAM[k] * (f[k + 2LL * ld] + f[k] - 2 * f[k + ld]) / (d1 * d1);
-                    const double bb = BETA[k] * (f[k + ld + 1] + f[k - 1] - f[k + ld - 1] - f[k + 1]) / (2 * d0 * d1);
-                    const double d2u = aa + gg - 2 * bb;
-                    double cv = uxi * 0.5 * (f[k + 1] - f[k - 1]) / d0;
-                    cv = cv + uet * (f[k + ld] - f[k]) / d1;
-                    const double alc = (m == 0) ? c.accn_amp * swall * Yc[k] : -c.accn_amp * swall * X[k];
-                    dpd[m] = 1.0 * d2u / Re - cv - alc + (m == 1 ? Ri * Tn[k] : 0.0);
-                }
-                const double pw = P[k + ld] - (dpd[0] * (-XIY[k] * JAC[k]) + dpd[1] * (XIX[k] * JAC[k])) * d1;
-                store_mirrored(P, ld, i, 0, W, per, pw);
-            }
-            {   // far field, j = n1-1
-                const long long k = (long long)jf * ld + i;
-                const double vnn = c.uinf * VEC[2LL * ld + i] + c.vinf * VEC[3LL * ld + i];
-                double pf;
-                if (vnn >= 0) {
-                    const double uxi = XIX[k] * U[k] + XIY[k] * V[k];
-                    const double uet = ETX[k] * U[k] + ETY[k] * V[k];
-                    double dpd[2];
-                    for (int m = 0; m < 2; m++) {
-                        const double* f = Fl[m];
-                        const double fo = s_old[m * (W + 1) + i];
-                        const double aa = ALPH[k] * (f[k + 1] + f[k - 1] - 2 * f[k]) / (d0 * d0);
-                        const double gg = GAM[k] * (f[k] + f[k - 2LL * ld] - 2 * f[k - ld]) / (d1 * d1);
-                        const double bb = BETA[k] * (f[k + 1] + f[k - ld - 1] - f[k - ld + 1] - f[k - 1]) / (2 * d0 * d1);
-                        const double d2u = aa + gg - 2 * bb;
-                        double cv = uxi * 0.5 * (f[k + 1] - f[k - 1]) / d0;
-                        cv = cv + uet * (3.0 * f[k] - 4 * f[k - ld] + f[k - 2LL * ld]) / (2 * d1);
-                        const double alc = (f[k] - fo) / dt;
-                        dpd[m] = 1.0 * d2u / Re - cv - alc + (m == 1 ? Ri * Tn[k] : 0.0);
-                    }
-                    pf = P[k - ld] + (dpd[0] * (-XIY[k] * JAC[k]) + dpd[1] * (XIX[k] * JAC[k])) * d1;
-                } else {
-                    const double e0 = ETX[k] * U[k] + ETY[k] * V[k];
-                    const long long k1 = k - ld, k2 = k - 2LL * ld;
-                    const double e1 = ETX[k1] * U[k1] + ETY[k1] * V[k1];
-                    const double e2 = ETX[k2] * U[k2] + ETY[k2] * V[k2];
-                    pf = 0.5 * (1.0 / Re) * ((3 * e0 - 4 * e1 + e2) / d1);
-                }
-                store_mirrored(P, ld, i, jf, W, per, pf);
-            }
+            bc_wall_p(a, i, swall);
+            bc_far_p(a, i, s_old);
         }
     } else {
-        // cavity: adiabatic side walls, zero normal pressure gradient, static walls
-        for (int j = 1 + threadIdx.x; j <= n1 - 2; j += blockDim.x) {
-            const long long r = (long long)j * ld;
-            Tn[r] = (4.0 * Tn[r + 1] - Tn[r + 2]) / 3.0;
-            Tn[r + n0 - 1] = (4.0 * Tn[r + n0 - 2] - Tn[r + n0 - 3]) / 3.0;
-            P[r] = P[r + 1];
-            P[r + n0 - 1] = P[r + n0 - 2];
-        }
-        for (int i = 1 + threadIdx.x; i <= n0 - 2; i += blockDim.x) {
-            P[i] = P[i + ld];
-            P[(long long)jf * ld + i] = P[(long long)(jf - 1) * ld + i];
-        }
+        // static walls
+        for (int j = 1 + threadIdx.x; j <= n1 - 2; j += blockDim.x) bc_cav_row(a, j);
+        for (int i = 1 + threadIdx.x; i <= n0 - 2; i += blockDim.x) bc_cav_col(a, i);
         __syncthreads();
-        if (threadIdx.x == 0) {
-            P[0] = 0.5 * (P[1] + P[ld]);
-            P[n0 - 1] = 0.5 * (P[n0 - 2] + P[ld + n0 - 1]);
-            const long long r = (long long)jf * ld;
-            P[r] = 0.5 * (P[r + 1] + P[r - ld]);
-            P[r + n0 - 1] = 0.5 * (P[r + n0 - 2] + P[r - ld + n0 - 1]);
-        }
+        if (threadIdx.x == 0) bc_cav_corners(a);
     }
     __syncthreads();
-    // vorticity on the j-boundaries (PSolver.cpp:1855-1888)
-    for (int e = threadIdx.x; e < 2 * (c.ihi - c.ilo + 1); e += blockDim.x) {
-        const int nb = c.ihi - c.ilo + 1;
-        const int i = c.ilo + e % nb;
-        const int j = (e < nb) ? 0 : jf;
-        const long long k = (long long)j * ld + i;
-        const double dv_dxi = 0.5 / d0 * (V[k + 1] - V[k - 1]);
-        const double dv_det = (j == 0) ? 1.0 / d1 * (V[k + ld] - V[k]) : 1.0 / d1 * (V[k] - V[k - ld]);
-        const double dv_dx = XIX[k] * dv_dxi + ETX[k] * dv_det;
-        const double du_dxi = 0.5 / d0 * (U[k + 1] - U[k - 1]);
-        const double du_det = (j == 0) ? 1.0 / d1 * (U[k + ld] - U[k]) : 1.0 / d1 * (U[k] - U[k - ld]);
-        const double du_dy = XIY[k] * du_dxi + ETY[k] * du_det;
-        store_mirrored(VORT, ld, i, j, W, per, dv_dx - du_dy);
-    }
+    const int nb = c.ihi - c.ilo + 1;
+    for (int e = threadIdx.x; e < 2 * nb; e += blockDim.x) bc_vort(a, c.ilo + e % nb, (e < nb) ? 0 : n1 - 1);
     __syncthreads();
-    // forces, moment, Nusselt number on j = 0 (PSolver.cpp:1901-1983)
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
-    for (int i = threadIdx.x; i <= n0 - 2; i += blockDim.x) {
-        const long long k = i, kp = i + 1;
-        const double PJ1 = P[k] * JAC[k], pj2 = P[kp] * JAC[kp];
-        const double VJ1 = VORT[k] * JAC[k], VJ2 = VORT[kp] * JAC[kp];
-        acc[0] += 0.5 * d0 * (PJ1 * ETX[k] + pj2 * ETX[kp]);
-        acc[1] += 0.5 * d0 * (PJ1 * ETY[k] + pj2 * ETY[kp]);
-        acc[2] += 0.5 * d0 * (VJ1 * ETY[k] + VJ2 * ETY[kp]);
-        acc[3] += 0.5 * d0 * (VJ1 * ETX[k] + VJ2 * ETX[kp]);
-        const double TJ1 = JAC[k] * (ETX[k] * ETX[k] + ETY[k] * ETY[k]);
-        const double TJ2 = JAC[kp] * (ETX[kp] * ETX[kp] + ETY[kp] * ETY[kp]);
-        const double fp1 = PJ1 * (X[k] * ETY[k] - Yc[k] * ETX[k]);
-        const double fp2 = pj2 * (X[kp] * ETY[kp] - Yc[kp] * ETX[kp]);
-        const double fv1 = VJ1 * (X[k] * ETX[k] + Yc[k] * ETY[k]);
-        const double fv2 = VJ2 * (X[kp] * ETX[kp] + Yc[kp] * ETY[kp]);
-        const double fh1 = TJ1 * (4 * Tn[k + ld] - 3 * Tn[k] - Tn[k + 2LL * ld]) / (2 * d1);
-        const double fh2 = TJ2 * (4 * Tn[kp + ld] - 3 * Tn[kp] - Tn[kp + 2LL * ld]) / (2 * d1);
-        acc[4] += 0.5 * d0 * (fp1 + fp2);
-        acc[5] += 0.5 * d0 * (fv1 + fv2);
-        acc[6] += 0.5 * (fh1 + fh2) * d0;
-    }
+    for (int i = threadIdx.x; i <= n0 - 2; i += blockDim.x) bc_integral(a, i, acc);
     block_sum<7>(acc, red);
     if (threadIdx.x == 0) {
-        const double pr_x = acc[0], pr_y = acc[1], vor_x = acc[2], vor_y = acc[3];
-        const double cx = 2 * pr_x + (2.0 / Re) * vor_x;
-        const double cy = 2 * pr_y - (2.0 / Re) * vor_y;
-        const double sa = c.sa, ca = c.ca;
-        sc[S_CLP] = 2 * pr_y * sa - 2 * pr_x * ca;
-        sc[S_CDP] = 2 * pr_y * ca + 2 * pr_x * sa;
-        sc[S_CLV] = -(2.0 / Re) * vor_y * sa - (2.0 / Re) * vor_x * ca;
-        sc[S_CDV] = -(2.0 / Re) * vor_y * ca + (2.0 / Re) * vor_x * sa;
-        sc[S_CL] = cy * sa - cx * ca;
-        sc[S_CD] = cy * ca + cx * sa;
-        sc[S_CM] = 2 * acc[4] - (2.0 / Re) * acc[5];
-        const double ar = c.ar;
-        if (!cav)
-            sc[S_NU] = (2 * acc[6]) / (Pi * (3 * (1 + (1.0 / ar)) - sqrt((3 + (1.0 / ar)) * ((3.0 / ar) + 1))));
-        else
-            sc[S_NU] = -acc[6];
+        bc_scalars(c, acc, sc);
         sc[S_CIRC] = cav ? 0.0 : s_circ;
         is[I_TIME] = time_new;
         sc[S_TIME] = t_new;
@@ -1649,17 +838,12 @@ __global__ void __launch_bounds__(NT, 3) k_diag(BatchDev b) {
     for (int h = 0; h < 2; h++) {
         if (!in[h]) continue;
         const int j = t.j0 + (int)(threadIdx.x / TX) + h * TY;
-        const double dil = xix[h] * (ue[h] - uw[h]) * h0 + etx[h] * (un[h] - us[h]) * h1 +
-                           ety[h] * (vn[h] - vs[h]) * h1 + xiy[h] * (ve[h] - vw[h]) * h0;
-        const double dv_dxi = h0 * (ve[h] - vw[h]);
-        const double dv_det = h1 * (vn[h] - vs[h]);
-        const double du_dxi = h0 * (ue[h] - uw[h]);
-        const double du_det = h1 * (un[h] - us[h]);
-        const double vort = (xix[h] * dv_dxi + etx[h] * dv_det) - (xiy[h] * du_dxi + ety[h] * du_det);
-        store_mirrored(plane(b, c, P_VORT), ld, i, j, W, per, vort);
-        store_mirrored(plane(b, c, P_DIL), ld, i, j, W, per, dil);
+        const DiagOut d = diag_cell(ue[h], uw[h], un[h], us[h], ve[h], vw[h], vn[h], vs[h], xix[h], xiy[h], etx[h],
+                                    ety[h], h0, h1);
+        store_mirrored(plane(b, c, P_VORT), ld, i, j, W, per, d.vort);
+        store_mirrored(plane(b, c, P_DIL), ld, i, j, W, per, d.dil);
         const double dT = fabs(tn[h] - to[h]);
-        red[0] = fmax(red[0], dil);
+        red[0] = fmax(red[0], d.dil);
         red[1] += dT;
         red[2] = fmax(red[2], dT);
     }
@@ -1721,7 +905,6 @@ __global__ void k_if_cond(cudaGraphConditionalHandle h, const int* flag, int* to
     }
 }
 
-#undef AT
 // ---------------------------------------------------------------------------
 // Resident state <-> one contiguous staging buffer (so a state snapshot crosses PCIe as one
 // copy per direction). Per case: the six state planes u, v, p, T, up, vp, each n1 rows of the

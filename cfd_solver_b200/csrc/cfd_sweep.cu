@@ -48,6 +48,7 @@
 #include "cfd_bulk.cuh"
 #include "cfd_common.cuh"
 #include "cfd_reduce.cuh"
+#include "cfd_step.cuh"
 #include "cfd_sweep.cuh"
 
 namespace cfd {
@@ -108,9 +109,6 @@ struct SwLayout {
     static constexpr int TOTAL = RAP + 2 * SW_CELLS * (int)sizeof(float);
 };
 
-// FP64 plane of field f's iterate for state parity nxt (u*, v*, T, up, vp)
-__device__ __forceinline__ int sw_iter_plane(int f, int nxt) { return f < 2 ? P_US + f : P_T0 + 2 * (f - 2) + nxt; }
-
 // issue the tensor copies of field f of tile t into buffer `sm` (with alpha, beta, gamma)
 template <int MODE>
 __device__ __forceinline__ void sw_issue(const Tile& t, int f, int sweep, int nxt, const char* maps,
@@ -149,30 +147,6 @@ __device__ __forceinline__ void sw_issue(const Tile& t, int f, int sweep, int nx
     // alpha, beta, gamma: three consecutive planes in one box
     if (met) tma_load_3d(met, maps + TMAP_F64_TILE3, t.i0 + 2, t.j0, P_ALPH, bar);
 }
-
-// off-centre sums of the u-type operator for the cell whose window centre row is `r0 + 2`:
-// the 25-point (4th-order) rows and the 9-point near-wall rows
-#define WX(dy, dx) w[r0 + 2 + (dy)][2 + (dx)]
-template <typename ST>
-__device__ __forceinline__ ST sw_sum25(const ST (&w)[8][5], int r0, ST E, ST G, ST B) {
-    const ST ex = ST(-4.0 / 3.0) * (WX(0, 1) + WX(0, -1)) + ST(1.0 / 12.0) * (WX(0, 2) + WX(0, -2));
-    const ST gy = ST(-4.0 / 3.0) * (WX(1, 0) + WX(-1, 0)) + ST(1.0 / 12.0) * (WX(2, 0) + WX(-2, 0));
-    const ST bx = ST(8.0 / 9.0) * (WX(1, 1) + WX(-1, -1) - WX(1, -1) - WX(-1, 1)) +
-                  ST(1.0 / 72.0) * (WX(2, 2) + WX(-2, -2) - WX(2, -2) - WX(-2, 2)) +
-                  ST(1.0 / 9.0) * (WX(2, -1) + WX(-2, 1) + WX(1, -2) + WX(-1, 2) - WX(2, 1) - WX(-2, -1) -
-                                   WX(1, 2) - WX(-1, -2));
-    return E * ex + G * gy + B * bx;
-}
-template <typename ST>
-__device__ __forceinline__ ST sw_sum9(const ST (&w)[8][5], int r0, ST E, ST G, ST B, bool drop_s, bool drop_n) {
-    ST s = -E * (WX(0, 1) + WX(0, -1));
-    const ST n = -G * WX(1, 0) + ST(0.5) * B * (WX(1, 1) - WX(1, -1));
-    const ST so = -G * WX(-1, 0) + ST(0.5) * B * (WX(-1, -1) - WX(-1, 1));
-    if (!drop_n) s += n;
-    if (!drop_s) s += so;
-    return s;
-}
-#undef WX
 
 template <int MODE>
 __device__ __forceinline__ void sweep_tile(const BatchDev& b, unsigned char* sm, uint64_t* bar) {
@@ -323,15 +297,9 @@ __device__ __forceinline__ void sweep_tile(const BatchDev& b, unsigned char* sm,
         for (int q = 0; q < SW_ROWS; q++) {
             const int o = (wrp * SW_ROWS + q) * TX + lane;
             const ST E = OPS[o], G = OPS[SW_CELLS + o], B = OPS[2 * SW_CELLS + o];
-            // off-centre sum: the 25-point form, or the 9-point form on the near-wall cells
-            ST sm_ = nearw[q] ? sw_sum9<ST>(w, q, E, G, B, drop_s[q], drop_n[q]) : sw_sum25<ST>(w, q, E, G, B);
-            if (tbug && !nearw[q]) sm_ -= B * w[q + 4][1];
-            sm_ *= scale;
-            const ST D = (nearw[q] ? ST(2) : ST(2.5)) * (E + G);
-            const ST ap = ST(1) + D * scale;
+            const ST res = sw_residual<ST>(w, q, E, G, B, nearw[q], drop_s[q], drop_n[q], tbug, scale, rhs[q]);
             const ST rap = (ST)RAP[rapoff + o];
             const ST xk = w[q + 2][2];
-            const ST res = rhs[q] - ap * xk - sm_;
             racc += inq[q] ? fabs((double)res) : 0.0;
             const long long kk = (long long)(t.j0 + wrp * SW_ROWS + q) * dld;
             if (MODE == SW_MX0) {
@@ -345,8 +313,7 @@ __device__ __forceinline__ void sweep_tile(const BatchDev& b, unsigned char* sm,
                     }
                 }
             } else {
-                ST xn = xk + g * res * rap;
-                if (weighted) xn = wgt * (xn - xm[q]) + xm[q];
+                const ST xn = sw_next<ST>(xk, g, res, rap, weighted, wgt, xm[q]);
                 if (inq[q]) {
                     if (MODE == SW_F64) {
                         dst64[kk + i] = (double)xn;
@@ -475,9 +442,7 @@ __device__ __forceinline__ int fin_case(const BatchDev& b, int cid, int* is, int
     is[I_MWORD] = nword;
 #pragma unroll
     for (int ty = 0; ty < 2; ty++) {  // Chebyshev weight of the next sweep
-        const double ca = in.ca[ty], cb = in.cb[ty];
-        const double s2 = ((cb + ca) / (cb - ca)) * ((cb + ca) / (cb - ca));
-        scw[S_CW0 + ty] = (sweep == 0) ? 1.0 / (1.0 - 1.0 / (2.0 * s2)) : 1.0 / (1.0 - in.cw[ty] / (4.0 * s2));
+        scw[S_CW0 + ty] = cheb_next(sweep, in.cw[ty], in.ca[ty], in.cb[ty]);
     }
     // algorithmic-traffic counters (cells and field-cells swept)
     const unsigned long long nf = (unsigned long long)__popc(mask) * in.ncell;
