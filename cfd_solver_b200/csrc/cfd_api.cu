@@ -583,6 +583,12 @@ void case_scalars_to_dev(CaseDev& d, double dxi0, double dxi1, double ar, const 
     d.swk[1] = d.dt / (d.Re * d.d1 * d.d1);
     d.swk[2] = d.dt / (d.Re * d.d0 * d.d1);
     d.rPr = 1.0 / d.Pr;
+    d.rd0 = 1.0 / d.d0; d.rd1 = 1.0 / d.d1; d.hd0 = 0.5 / d.d0; d.hd1 = 0.5 / d.d1; d.rdt = 1.0 / d.dt;
+    d.circ_de = p.fix_circ_de ? 1.0 / (d.n0 - 1) : 1.0 / (d.n0 - 2);
+    auto by = [](double x) { return DivBy{x, 1.0 / x}; };
+    d.v0 = by(d.d0); d.v1 = by(d.d1); d.v00 = by(d.d0 * d.d0); d.v11 = by(d.d1 * d.d1);
+    d.v01 = by(2.0 * d.d0 * d.d1); d.v1x2 = by(2.0 * d.d1); d.vdt = by(d.dt); d.vRe = by(d.Re);
+    d.vRePr = by(d.Re * d.Pr); d.v01Re = by(2.0 * d.d0 * d.d1 * d.Re);
     d.pc1 = 1.0 / (2.0 * g.dxi0 * g.dxi0);
     d.pc2 = 1.0 / (8.0 * g.dxi0 * g.dxi1);
     d.pc3 = 1.0 / (2.0 * g.dxi1 * g.dxi1);

@@ -101,6 +101,23 @@ struct LevelDev {
     int tile_begin, tile_count;  // tiles of this case in the level's tile table
 };
 
+// A divisor that is fixed for a case, with its correctly rounded reciprocal (formed on the
+// host): div_by(n, D) rounds like n / D.d. One quotient and two residual corrections (P. Markstein,
+// Computation of elementary functions on the IBM RISC System/6000 processor, IBM J. Res. Dev.
+// 34, 1990: a quotient within an ulp and a correctly rounded reciprocal give the rounded
+// quotient) are five dependent operations and no branch, where a full FP64 division is some 300
+// cycles that nothing overlaps. Quotients near the ends of the exponent range are not exact.
+struct DivBy {
+    double d, y;
+};
+#ifdef __CUDACC__
+__device__ __forceinline__ double div_by(double n, const DivBy& D) {
+    double q = n * D.y;
+    q = fma(fma(-D.d, q, n), D.y, q);
+    return fma(fma(-D.d, q, n), D.y, q);
+}
+#endif
+
 struct CaseDev {
     int W, n0, n1, ld;
     int periodic, ilo, ihi, profile;
@@ -112,12 +129,17 @@ struct CaseDev {
     long long xbase, xps;
     int fix_T_annw, fix_circ_de, warm_up;
     int time_accurate;              // 1: time is a double (t = n dt), 0: the reference's int
-    double d0, d1, dt, Re, Pr, Ri, F;
-    double uinf, vinf, speed_amp, accn_amp, Pi, ar, omega_p, lid_u, sa, ca;
+    double d0, d1, dt, Re, Pr, Ri;
+    double rd0, rd1, hd0, hd1, rdt;  // 1 / dxi, 0.5 / dxi, 1 / dt
+    double uinf, vinf, omega_p;
+    double F, speed_amp, accn_amp, Pi, ar, lid_u, sa, ca;
     double tol_mom, atol_mom, tol_p, atol_p;
     double cheb_a[2], cheb_b[2];  // eigenvalue bounds of D^-1 A (u-type, T) for the Chebyshev sweeps
     double swk[3];                // dt / (Re dxi0^2), dt / (Re dxi1^2), dt / (Re dxi0 dxi1): E, G, B per metric
     double rPr;                   // 1 / Pr
+    double circ_de;               // spacing of the circulation integral
+    // fixed divisors: dxi0, dxi1, dxi0^2, dxi1^2, 2 dxi0 dxi1, 2 dxi1, dt, Re, Re Pr, 2 dxi0 dxi1 Re
+    DivBy v0, v1, v00, v11, v01, v1x2, vdt, vRe, vRePr, v01Re;
     double pc1, pc2, pc3;         // 1 / (2 dxi0^2), 1 / (8 dxi0 dxi1), 1 / (2 dxi1^2): pressure stencil
     LevelDev lev[MAXLEV];
 };

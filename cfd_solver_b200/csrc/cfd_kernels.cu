@@ -146,9 +146,7 @@ __global__ void __launch_bounds__(NT, 3) k_rhs(BatchDev b) {
     // the case's constants and planes, loaded while the copies are in flight
     const int ld = c.ld, W = c.W, per = c.periodic, n1 = c.n1, n0 = c.n0, ilo = c.ilo, ihi = c.ihi;
     const bool cav = c.profile == CAVITY;
-    RhsCase rc;
-    rc.d0 = c.d0; rc.d1 = c.d1; rc.rd0 = 1.0 / c.d0; rc.rd1 = 1.0 / c.d1;
-    rc.dt = c.dt; rc.Re = c.Re; rc.Pr = c.Pr; rc.Ri = c.Ri; rc.n0 = n0; rc.n1 = n1; rc.cav = cav;
+    const RhsCase rc(c);
     double* const fb = b.f64 + c.base + H;  // plane 0 of the case; plane k at fb + k * ps
     const long long ps = c.ps;
     const bool warm = c.warm_up != 0;
@@ -175,7 +173,7 @@ __global__ void __launch_bounds__(NT, 3) k_rhs(BatchDev b) {
         const int o = (lj + h * TY + 2) * JTW + (li + 2);
         const int oi = (lj + h * TY) * TX + li;
         const long long k = (long long)j * ld + i;
-        const RhsOut r = rhs_cell(rc, i, j, Us, Vs, Ts, Ps, UPs, VPs, o, JTW, SI[oi], SI[TX * TYJ + oi],
+        const RhsOut r = rhs_cell<CrossAt>(rc, i, j, Us, Vs, Ts, Ps, UPs, VPs, o, JTW, SI[oi], SI[TX * TYJ + oi],
                                   SI[2 * TX * TYJ + oi], SI[3 * TX * TYJ + oi], SI[4 * TX * TYJ + oi],
                                   SI[5 * TX * TYJ + oi], SI + 6 * TX * TYJ + oi);
         fb[P_RU * ps + k] = r.qu;
@@ -184,7 +182,7 @@ __global__ void __launch_bounds__(NT, 3) k_rhs(BatchDev b) {
         fb[P_RUP * ps + k] = r.qup;
         fb[P_RVP * ps + k] = r.qvp;
         const double seed[NFIELD] = {Us[o], Vs[o], Ts[o], warm ? UPs[o] : 0.0, warm ? VPs[o] : 0.0};
-        rhs_seed(fb, ps, nextm, cur, ld, W, per, cav, n0, n1, i, j, seed);
+        rhs_seed<false>(fb, ps, nextm, cur, ld, W, per, cav, n0, n1, i, j, seed);
     }
 }
 
@@ -371,7 +369,7 @@ __global__ void __launch_bounds__(NT, 5) k_spmv(BatchDev b, int mode) {
         const long long kk = (long long)jj * ld + ii, q = (long long)jj * l0 + ii;
         k[h] = kk;
         xc[h] = (double)X[q];
-        y[h] = spmv_cell(plane(b, c, P_AP), c.ps, kk, X, q, l0, xc[h]);
+        y[h] = spmv_cell([&](int m) { return plane(b, c, P_AP + m)[kk]; }, X, q, l0, xc[h]);
         dv[h] = DOT[kk];
     }
     double red[2] = {0.0, 0.0};
@@ -589,7 +587,7 @@ __global__ void __launch_bounds__(MG_PRR_THREADS, 3) k_mg_prr(BatchDev b, int l,
     const Tile t = b.atiles[l + 1][blockIdx.x];
     if (b.iscal[(long long)t.c * NISCAL + I_PDONE]) return;
     const CaseDev& c = b.cases[t.c];
-    mg_prr_tile(b, c, l, t.i0, t.j0, dst, inner, xs, rs, BlockGroup<MG_PRR_THREADS>());
+    mg_prr_tile<false>(b, c, l, t.i0, t.j0, dst, inner, xs, rs, BlockGroup<MG_PRR_THREADS>());
 }
 
 // multicolour Gauss-Seidel sweeps of level l on a 32 x 16 tile (mg_gs_tile)
@@ -714,7 +712,7 @@ __global__ void __launch_bounds__(NT, 4) k_correct(BatchDev b) {
         u0[h] = U[k]; v0[h] = V[k]; p0[h] = P[k];
     }
     const double vnn = c.uinf * VEC[2LL * ld + i] + c.vinf * VEC[3LL * ld + i];
-    const double h0 = 0.5 / c.d0, h1 = 0.5 / c.d1, dt = c.dt;  // the gradients' quotients as products
+    const double h0 = c.hd0, h1 = c.hd1, dt = c.dt;  // the gradients' quotients as products
     double red[1] = {0.0};
 #pragma unroll
     for (int h = 0; h < 2; h++) {
@@ -769,16 +767,17 @@ __global__ void __launch_bounds__(BC_THREADS, 2) k_bc(BatchDev b) {
             __syncthreads();
         }
         const double circ = s_circ;
-        const double cwall = cos(2.0 * c.Pi * c.F * t_new);
+        double cwall, swall;
+        bc_phase(c, t_new, cwall, swall);
         for (int i = threadIdx.x; i < W; i += blockDim.x) {
             bc_far(a, i, circ, s_old);
-            bc_wall(a, i, cwall);
+            bc_wall(a, i, bc_wall_u(a, i, cwall), bc_wall_v(a, i, cwall));
         }
         __syncthreads();
-        const double swall = sin(2.0 * c.Pi * c.F * t_new);
         for (int i = threadIdx.x; i < W; i += blockDim.x) {
-            bc_wall_p(a, i, swall);
-            bc_far_p(a, i, s_old);
+            bc_wall_p(a, i, edge_at(a, i), swall);
+            const long long kf = (long long)a.jf * a.ld + i;
+            bc_far_p(a, i, edge_at(a, kf), a.Tn[kf], s_old);
         }
     } else {
         // static walls
@@ -789,10 +788,13 @@ __global__ void __launch_bounds__(BC_THREADS, 2) k_bc(BatchDev b) {
     }
     __syncthreads();
     const int nb = c.ihi - c.ilo + 1;
-    for (int e = threadIdx.x; e < 2 * nb; e += blockDim.x) bc_vort(a, c.ilo + e % nb, (e < nb) ? 0 : n1 - 1);
+    for (int e = threadIdx.x; e < 2 * nb; e += blockDim.x) {
+        const int i = c.ilo + e % nb, j = (e < nb) ? 0 : n1 - 1;
+        bc_vort(a, i, j, edge_at(a, (long long)j * a.ld + i));
+    }
     __syncthreads();
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
-    for (int i = threadIdx.x; i <= n0 - 2; i += blockDim.x) bc_integral(a, i, acc);
+    for (int i = threadIdx.x; i <= n0 - 2; i += blockDim.x) bc_integral(a, i, a.P, a.VORT, acc);
     block_sum<7>(acc, red);
     if (threadIdx.x == 0) {
         bc_scalars(c, acc, sc);
@@ -832,7 +834,7 @@ __global__ void __launch_bounds__(NT, 3) k_diag(BatchDev b) {
         tn[h] = TN[k]; to[h] = TO[k];
     }
     // 0.5 / d is 1 / (2 d) exactly: the dilatation's quotients become products
-    const double h0 = 0.5 / c.d0, h1 = 0.5 / c.d1;
+    const double h0 = c.hd0, h1 = c.hd1;
     double red[3] = {-1.0e300, 0.0, 0.0};
 #pragma unroll
     for (int h = 0; h < 2; h++) {

@@ -42,21 +42,58 @@ __device__ __forceinline__ int mg_result_plane(const BatchDev& b, const CaseDev&
 // ---------------------------------------------------------------------------
 // convection and the five right-hand sides
 
-// One convective term ux df/dxi + ue df/deta of field F at offset o, rows R apart
-// (PSolver.cpp:1110-1180): 4th-order central differences when the cell Peclet number is in
-// (-2, 2] (and always in the rows / columns next to a wall, where the reference uses
-// 2nd-order central), otherwise 3rd-order upwind. The reference forms du = (ux D1 +
-// |ux| D4) / ux and multiplies by ux again; here the product is formed directly, and every
-// division by a grid spacing is a multiplication by its reciprocal.
-__device__ __forceinline__ double conv_one(const double* F, int o, bool near_i, bool near_j, double ux,
-                                           double ue, bool cen_i, bool cen_j, double rd0, double rd1, int R) {
-    const double fc = F[o], fe = F[o + 1], fw = F[o - 1];
-    const double fn = F[o + R], fs = F[o - R];
+// A field at a cell and two cells to each side, rows R apart. From shared memory (CrossAt)
+// each value is read where it is used; from global memory (Cross) all loads come first and
+// without a branch, and next to a wall the second cell along that axis is not read (it may
+// lie outside).
+struct CrossAt {
+    const double* f;
+    int R;
+    __device__ __forceinline__ CrossAt(const double* F, int o, int R_, bool, bool) : f(F + o), R(R_) {}
+    __device__ __forceinline__ double c() const { return f[0]; }
+    __device__ __forceinline__ double e() const { return f[1]; }
+    __device__ __forceinline__ double w() const { return f[-1]; }
+    __device__ __forceinline__ double n() const { return f[R]; }
+    __device__ __forceinline__ double s() const { return f[-R]; }
+    __device__ __forceinline__ double ee() const { return f[2]; }
+    __device__ __forceinline__ double ww() const { return f[-2]; }
+    __device__ __forceinline__ double nn() const { return f[2 * R]; }
+    __device__ __forceinline__ double ss() const { return f[-2 * R]; }
+};
+struct Cross {
+    double v[9];
+    __device__ __forceinline__ Cross(const double* F, int o, int R, bool near_i, bool near_j) {
+        const int a = near_i ? 1 : 2, b = near_j ? R : 2 * R;
+        v[0] = F[o]; v[1] = F[o + 1]; v[2] = F[o - 1]; v[3] = F[o + R]; v[4] = F[o - R];
+        v[5] = F[o + a]; v[6] = F[o - a]; v[7] = F[o + b]; v[8] = F[o - b];
+    }
+    __device__ __forceinline__ double c() const { return v[0]; }
+    __device__ __forceinline__ double e() const { return v[1]; }
+    __device__ __forceinline__ double w() const { return v[2]; }
+    __device__ __forceinline__ double n() const { return v[3]; }
+    __device__ __forceinline__ double s() const { return v[4]; }
+    __device__ __forceinline__ double ee() const { return v[5]; }
+    __device__ __forceinline__ double ww() const { return v[6]; }
+    __device__ __forceinline__ double nn() const { return v[7]; }
+    __device__ __forceinline__ double ss() const { return v[8]; }
+};
+
+// One convective term ux df/dxi + ue df/deta of a field (PSolver.cpp:1110-1180): 4th-order
+// central differences when the cell Peclet number is in (-2, 2] (and always in the rows /
+// columns next to a wall, where the reference uses 2nd-order central), otherwise 3rd-order
+// upwind. The reference forms du = (ux D1 + |ux| D4) / ux and multiplies by ux again; here
+// the product is formed directly, and every division by a grid spacing is a multiplication
+// by its reciprocal.
+template <class S>
+__device__ __forceinline__ double conv_one(const S& f, bool near_i, bool near_j, double ux, double ue, bool cen_i,
+                                           bool cen_j, double rd0, double rd1) {
+    const double fc = f.c(), fe = f.e(), fw = f.w();
+    const double fn = f.n(), fs = f.s();
     double cx, cy;
     if (near_i) {
         cx = ux * (0.5 * (fe - fw) * rd0);
     } else {
-        const double fee = F[o + 2], fww = F[o - 2];
+        const double fee = f.ee(), fww = f.ww();
         if (near_j || cen_i) {
             cx = ux * ((1.0 / 12.0) * (8.0 * (fe - fw) - (fee - fww)) * rd0);
         } else {
@@ -67,7 +104,7 @@ __device__ __forceinline__ double conv_one(const double* F, int o, bool near_i, 
     if (near_j) {
         cy = ue * (0.5 * (fn - fs) * rd1);
     } else {
-        const double fnn = F[o + 2 * R], fss = F[o - 2 * R];
+        const double fnn = f.nn(), fss = f.ss();
         if (near_i || cen_j) {
             cy = ue * ((1.0 / 12.0) * (8.0 * (fn - fs) - (fnn - fss)) * rd1);
         } else {
@@ -78,11 +115,21 @@ __device__ __forceinline__ double conv_one(const double* F, int o, bool near_i, 
     return cx + cy;
 }
 
+// Is the cell Peclet number n / a in (-2, 2]? Decided without the quotient: for a > 0, RN(n / a)
+// is in (-2, 2] exactly when n is in (-2 a, 2 a] (2 a is exact, and the doubles next to it are
+// more than half a unit in the last place of 2 away).
+__device__ __forceinline__ bool peclet_central(double n, double a) { return n <= 2.0 * a && n > -2.0 * a; }
 
+// what every cell's right-hand sides read of the case
 struct RhsCase {
-    double d0, d1, rd0, rd1, dt, Re, Pr, Ri;
+    const CaseDev& c;
+    double rd0, rd1, dt, Red0, Red1, Pr, Ri;
     int n0, n1;
     bool cav;
+    __device__ __forceinline__ explicit RhsCase(const CaseDev& c_) : c(c_) {
+        rd0 = c.rd0; rd1 = c.rd1; dt = c.dt; Red0 = c.Re * c.d0; Red1 = c.Re * c.d1; Pr = c.Pr; Ri = c.Ri;
+        n0 = c.n0; n1 = c.n1; cav = c.profile == CAVITY;
+    }
 };
 struct RhsOut {
     double qu, qv, qt, qup, qvp;
@@ -90,26 +137,29 @@ struct RhsOut {
 
 // The five right-hand sides of cell (i, j) (PSolver.cpp:1063-1237). The fields are read at
 // offset o with rows R apart; `be` points at the cell's beta (read next to an O-grid's walls).
+template <class S>
 __device__ __forceinline__ RhsOut rhs_cell(const RhsCase& a, int i, int j, const double* Us, const double* Vs,
                                            const double* Ts, const double* Ps, const double* UPs, const double* VPs,
                                            int o, int R, double xix, double xiy, double etx, double ety, double al,
                                            double ga, const double* bep) {
-    const double dt = a.dt, Re = a.Re, Pr = a.Pr, d0 = a.d0, d1 = a.d1, rd0 = a.rd0, rd1 = a.rd1;
-    const double uc = Us[o], vc = Vs[o], tc = Ts[o];
+    const double dt = a.dt, rd0 = a.rd0, rd1 = a.rd1;
+    const bool cav = a.cav;
+    const bool near_j = (j == 1 || j == a.n1 - 2);
+    const bool near_i = cav && (i == 1 || i == a.n0 - 2);
+    const S fu(Us, o, R, near_i, near_j), fv(Vs, o, R, near_i, near_j), ft(Ts, o, R, near_i, near_j);
+    const S fp(Ps, o, R, true, true);
+    const double uc = fu.c(), vc = fv.c(), tc = ft.c();
     const double ux = xix * uc + xiy * vc;
     const double ue = etx * uc + ety * vc;
-    const bool near_j = (j == 1 || j == a.n1 - 2);
-    const bool near_i = a.cav && (i == 1 || i == a.n0 - 2);
     // cell Peclet numbers ux Re dxi / alpha, ue Re deta / gamma (x Pr for T)
-    const double pu1 = ux * (Re * d0) / al, pu2 = ue * (Re * d1) / ga;
-    const double pt1 = pu1 * Pr, pt2 = pu2 * Pr;
-    const bool cu1 = pu1 <= 2 && pu1 > -2, cu2 = pu2 <= 2 && pu2 > -2;
-    const bool ct1 = pt1 <= 2 && pt1 > -2, ct2 = pt2 <= 2 && pt2 > -2;
-    const double cv0 = conv_one(Us, o, near_i, near_j, ux, ue, cu1, cu2, rd0, rd1, R);
-    const double cv1 = conv_one(Vs, o, near_i, near_j, ux, ue, cu1, cu2, rd0, rd1, R);
-    const double cv2 = conv_one(Ts, o, near_i, near_j, ux, ue, ct1, ct2, rd0, rd1, R);
-    const double dp_dxi = (Ps[o + 1] - Ps[o - 1]) * (0.5 * rd0);
-    const double dp_de = (Ps[o + R] - Ps[o - R]) * (0.5 * rd1);
+    const double pn1 = ux * a.Red0, pn2 = ue * a.Red1;
+    const bool cu1 = peclet_central(pn1, al), cu2 = peclet_central(pn2, ga);
+    const bool ct1 = peclet_central(pn1 * a.Pr, al), ct2 = peclet_central(pn2 * a.Pr, ga);
+    const double cv0 = conv_one(fu, near_i, near_j, ux, ue, cu1, cu2, rd0, rd1);
+    const double cv1 = conv_one(fv, near_i, near_j, ux, ue, cu1, cu2, rd0, rd1);
+    const double cv2 = conv_one(ft, near_i, near_j, ux, ue, ct1, ct2, rd0, rd1);
+    const double dp_dxi = (fp.e() - fp.w()) * (0.5 * rd0);
+    const double dp_de = (fp.n() - fp.s()) * (0.5 * rd1);
     const double dp_dx = xix * dp_dxi + etx * dp_de;
     const double dp_dy = xiy * dp_dxi + ety * dp_de;
     RhsOut q;
@@ -118,15 +168,15 @@ __device__ __forceinline__ RhsOut rhs_cell(const RhsCase& a, int i, int j, const
     q.qt = -dt * cv2 + tc;
     q.qup = q.qu + dt * dp_dx;
     q.qvp = q.qv + dt * dp_dy;
-    if (!a.cav && near_j) {
+    if (!cav && near_j) {
         // folded wall-row couplings (PSolver.cpp:1195-1227)
+        const CaseDev& c = a.c;
         const double be = *bep;
-        const double bs = -dt * (ga / (d1 * d1)) / Re;
-        const double bpos = dt * be / (2.0 * d0 * d1 * Re);
-        const double bneg = -dt * be / (2.0 * d0 * d1 * Re);
-        const double ts = -dt * (ga / (d1 * d1)) / (Re * Pr);
-        const double tpos = dt * (be / (2.0 * d0 * d1)) / (Re * Pr);
-        const double tneg = -dt * (be / (2.0 * d0 * d1)) / (Re * Pr);
+        const double g11 = div_by(ga, c.v11);
+        const double bs = div_by(-dt * g11, c.vRe);
+        const double bpos = div_by(dt * be, c.v01Re), bneg = -bpos;
+        const double ts = div_by(-dt * g11, c.vRePr);
+        const double tpos = div_by(dt * div_by(be, c.v01), c.vRePr), tneg = -tpos;
         int s0, s1, s2;
         double c1, c2, t1, t2;
         if (j == 1) {  // bus, buse (= ause), busw (= ausw)
@@ -155,6 +205,9 @@ __device__ __forceinline__ RhsOut rhs_cell(const RhsCase& a, int i, int j, const
 // solve predicted to stop after an odd number of sweeps (bit of `nextm`) starts in the scratch
 // plane, so that its result ends in the iterate plane. Cells next to a boundary also write the
 // boundary values the stencils read, into both iterate buffers. `fb` is plane 0 of the case.
+// AHEAD: a boundary point's five loads are issued together (one latency instead of five, for
+// more registers than k_rhs has to spare).
+template <bool AHEAD>
 __device__ __forceinline__ void rhs_seed(double* fb, long long ps, int nextm, int cur, int ld, int W, int per,
                                          bool cav, int n0, int n1, int i, int j, const double (&seed)[NFIELD]) {
     const int nxt = cur ^ 1;
@@ -172,12 +225,21 @@ __device__ __forceinline__ void rhs_seed(double* fb, long long ps, int nextm, in
     auto put_bnd = [&](int bi, int bj) {
         const long long kb = (long long)bj * ld + bi;
         const bool zero_far = !cav && bj == n1 - 1;  // up/vp solves see zero on the far row
+        if constexpr (AHEAD) {
+            const double val[NFIELD] = {U[kb], V[kb], T[kb], zero_far ? 0.0 : UP[kb], zero_far ? 0.0 : VP[kb]};
+#pragma unroll
+            for (int f = 0; f < NFIELD; f++) {
+                store_mirrored(Ap(f), ld, bi, bj, W, per, val[f]);
+                store_mirrored(Bp(f), ld, bi, bj, W, per, val[f]);
+            }
+        } else {
 #pragma unroll 1
-        for (int f = 0; f < NFIELD; f++) {
-            const double* src = f == F_U ? U : f == F_V ? V : f == F_T ? T : f == F_UP ? UP : VP;
-            const double val = (zero_far && f >= F_UP) ? 0.0 : src[kb];
-            store_mirrored(Ap(f), ld, bi, bj, W, per, val);
-            store_mirrored(Bp(f), ld, bi, bj, W, per, val);
+            for (int f = 0; f < NFIELD; f++) {
+                const double* src = f == F_U ? U : f == F_V ? V : f == F_T ? T : f == F_UP ? UP : VP;
+                const double val = (zero_far && f >= F_UP) ? 0.0 : src[kb];
+                store_mirrored(Ap(f), ld, bi, bj, W, per, val);
+                store_mirrored(Bp(f), ld, bi, bj, W, per, val);
+            }
         }
     };
     if (j == 1) put_bnd(i, 0);
@@ -247,9 +309,9 @@ __device__ __forceinline__ ST sw_next(ST xk, ST g, ST res, ST rap, bool weighted
     return xn;
 }
 
-// Chebyshev weight of the sweep after `sweep` (bounds a, b; cw the weight of `sweep`)
-__device__ __forceinline__ double cheb_next(int sweep, double cw, double ca, double cb) {
-    const double s2 = ((cb + ca) / (cb - ca)) * ((cb + ca) / (cb - ca));
+// Chebyshev weight of the sweep after `sweep` (s2 of the bounds a, b; cw the weight of `sweep`)
+__device__ __forceinline__ double cheb_s2(double ca, double cb) { return ((cb + ca) / (cb - ca)) * ((cb + ca) / (cb - ca)); }
+__device__ __forceinline__ double cheb_next(int sweep, double cw, double s2) {
     return (sweep == 0) ? 1.0 / (1.0 - 1.0 / (2.0 * s2)) : 1.0 / (1.0 - cw / (4.0 * s2));
 }
 
@@ -264,11 +326,10 @@ __device__ __forceinline__ double upbc_out(const double* UP, long long k, int ld
 struct FaceCase {
     double rd0, rd1, q0, q1, hdt, rdt;
     __device__ __forceinline__ explicit FaceCase(const CaseDev& c) {
-        // reciprocals once per thread: the per-cell quotients become products (each within an
-        // ulp of the quotient; 1 / (4 d) is 0.25 / d exactly)
-        const double dt = c.dt;
-        rd0 = 1.0 / c.d0; rd1 = 1.0 / c.d1; q0 = 0.25 * rd0; q1 = 0.25 * rd1;
-        hdt = 0.5 * dt; rdt = 1.0 / dt;
+        // the per-cell quotients as products (each within an ulp of the quotient; 1 / (4 d) is
+        // 0.25 / d exactly)
+        rd0 = c.rd0; rd1 = c.rd1; q0 = 0.25 * rd0; q1 = 0.25 * rd1;
+        hdt = 0.5 * c.dt; rdt = c.rdt;
     }
 };
 
@@ -307,14 +368,13 @@ __device__ __forceinline__ double face_cell(const FaceCase& a, const double* P, 
 // ---------------------------------------------------------------------------
 // pressure correction
 
-// the stored FP64 9-point stencil (planes P_AP .. P_ASW from A, ps apart) at k, applied to
-// the FP32 field X at q, rows l0 apart
-__device__ __forceinline__ double spmv_cell(const double* A, long long ps, long long kk, const float* X, long long q,
-                                            int l0, double xc) {
-    return A[kk] * xc + A[ps + kk] * (double)X[q + 1] + A[2 * ps + kk] * (double)X[q - 1] +
-           A[3 * ps + kk] * (double)X[q + l0] + A[4 * ps + kk] * (double)X[q - l0] +
-           A[5 * ps + kk] * (double)X[q + l0 + 1] + A[6 * ps + kk] * (double)X[q + l0 - 1] +
-           A[7 * ps + kk] * (double)X[q - l0 + 1] + A[8 * ps + kk] * (double)X[q - l0 - 1];
+// a 9-point stencil (a(0) .. a(8) in the order of the planes P_AP .. P_ASW) applied to the FP32
+// field X at q, rows l0 apart; xc = X[q]
+template <class A>
+__device__ __forceinline__ double spmv_cell(const A& a, const float* X, long long q, int l0, double xc) {
+    return a(0) * xc + a(1) * (double)X[q + 1] + a(2) * (double)X[q - 1] + a(3) * (double)X[q + l0] +
+           a(4) * (double)X[q - l0] + a(5) * (double)X[q + l0 + 1] + a(6) * (double)X[q + l0 - 1] +
+           a(7) * (double)X[q - l0 + 1] + a(8) * (double)X[q - l0 - 1];
 }
 
 // stored column of level column gi, gi in [-W, inf): the periodic wrap without a division
@@ -329,6 +389,18 @@ __device__ __forceinline__ int mg_colour(int i, int j, int W, int periodic) {
     // 4 colours by parity; an odd periodic width gets 2 extra colours for its last column
     if (periodic && (W & 1) && i == W - 1) return 4 + (j & 1);
     return (i & 1) | ((j & 1) << 1);
+}
+
+// n / d rounded as the division rounds it, from y = the correctly rounded 1 / d: two residual
+// corrections of n y (P. Markstein, Computation of elementary functions on the IBM RISC
+// System/6000 processor, IBM J. Res. Dev. 34, 1990: with y correctly rounded, a quotient within
+// an ulp is corrected to the rounded one). Five dependent operations instead of the twenty of a
+// full division, which end every colour pass of a smoother whose diagonal never changes. For
+// quotients outside 1e-30 .. 1e38 the last bit may differ.
+__device__ __forceinline__ float mg_div(float n, float d, float y) {
+    float q = n * y;
+    q = fmaf(fmaf(-d, q, n), y, q);
+    return fmaf(fmaf(-d, q, n), y, q);
 }
 
 // Pre-smoothing folded into the residual + restriction pass (schedule form `fused` = 2).
@@ -365,7 +437,7 @@ __device__ __forceinline__ int mpr_rat(int x, int y) { return (x & 1) * MPR_RP +
 // Each thread owns one 2 x 2 block of E, which holds one point of each colour (E starts at
 // an even column and row, and a level with a coarser one has an even width when periodic,
 // so the colours are the four parity classes); its four stencils stay in registers.
-template <class Grp>
+template <bool WIDE, class Grp>
 __device__ __forceinline__ void mg_prr_tile(const BatchDev& b, const CaseDev& c, int l, int i0, int j0, int dst,
                                             int inner, float* xs, float* rs, const Grp& g) {
     static_assert(Grp::N >= MPR_BX * MPR_BY && Grp::N >= TX * TY, "a thread per block of E, one per coarse point");
@@ -406,6 +478,11 @@ __device__ __forceinline__ void mg_prr_tile(const BatchDev& b, const CaseDev& c,
             a[dy][1][q] = v.y;
         }
     }
+    float rdiag[2][2];  // reciprocals of the diagonals
+#pragma unroll
+    for (int dy = 0; dy < 2; dy++)
+#pragma unroll
+        for (int dx = 0; dx < 2; dx++) rdiag[dy][dx] = ok[dy][dx] ? __frcp_rn(a[dy][dx][0]) : 0.0f;
     for (int e = tid; e < 2 * MPR_XP; e += Grp::N) xs[e] = 0.0f;
     g.sync();
     // point of colour cc in the block: (dx, dy) = (cc & 1, cc >> 1); its ringed position is
@@ -431,7 +508,7 @@ __device__ __forceinline__ void mg_prr_tile(const BatchDev& b, const CaseDev& c,
                      f[3] * xs[mpr_at(xx, ry + 1)] + f[4] * xs[mpr_at(xx, ry - 1)] +
                      f[5] * xs[mpr_at(xx + 1, ry + 1)] + f[6] * xs[mpr_at(xx - 1, ry + 1)] +
                      f[7] * xs[mpr_at(xx + 1, ry - 1)] + f[8] * xs[mpr_at(xx - 1, ry - 1)];
-            const float v = (f[9] - sm) / f[0];
+            const float v = mg_div(f[9] - sm, f[0], rdiag[dy][dx]);
             xs[mpr_at(xx, ry)] = v;
             xr[dy][dx] = v;
         }
@@ -447,7 +524,7 @@ __device__ __forceinline__ void mg_prr_tile(const BatchDev& b, const CaseDev& c,
                              f[3] * xs[mpr_at(xx, ry + 1)] + f[4] * xs[mpr_at(xx, ry - 1)] +
                              f[5] * xs[mpr_at(xx + 1, ry + 1)] + f[6] * xs[mpr_at(xx - 1, ry + 1)] +
                              f[7] * xs[mpr_at(xx + 1, ry - 1)] + f[8] * xs[mpr_at(xx - 1, ry - 1)];
-            const float v = (f[9] - sm) / f[0];
+            const float v = mg_div(f[9] - sm, f[0], rdiag[dy][dx]);
             xs[mpr_at(xx, ry)] = v;
             xr[dy][dx] = v;
         }
@@ -463,31 +540,55 @@ __device__ __forceinline__ void mg_prr_tile(const BatchDev& b, const CaseDev& c,
     for (int n = 1; n < inner; n++) {
         relax(C0{}); relax(C1{}); relax(C2{}); relax(C3{});
     }
-    // residual on the restriction's fine points (E without its ring), x of the owned points
+    // residual on the restriction's fine points (E without its ring), x of the owned points. The
+    // block's four stencils read a 4 x 4 neighbourhood; WIDE holds it in registers (where one
+    // CTA per SM leaves room: its latency is then one round of shared loads instead of four),
+    // else every point reads its own eight neighbours
     float* OUT = mplane(b, F, dst);
     const int jhi = (j0 + TY > C.n1 - 2) ? n1 - 2 : min(2 * j0 + 14, n1 - 2);
+    if (own) {
+        float w[4][4] = {};
+        if constexpr (WIDE) {
 #pragma unroll
-    for (int dy = 0; dy < 2; dy++)
+            for (int r = 0; r < 4; r++)
 #pragma unroll
-        for (int dx = 0; dx < 2; dx++) {
-            const int x = 2 * bx + dx, y = 2 * by + dy;
-            if (!own || x < 1 || x > MPR_RW || y < 1 || y > MPR_RH) continue;
-            float r = 0.0f;
-            if (ok[dy][dx]) {
-                const float(&f)[10] = a[dy][dx];
-                const int xx = x + 1, ry = y + 1;
-                const float ax = f[0] * xr[dy][dx] + f[1] * xs[mpr_at(xx + 1, ry)] + f[2] * xs[mpr_at(xx - 1, ry)] +
-                                 f[3] * xs[mpr_at(xx, ry + 1)] + f[4] * xs[mpr_at(xx, ry - 1)] +
-                                 f[5] * xs[mpr_at(xx + 1, ry + 1)] + f[6] * xs[mpr_at(xx - 1, ry + 1)] +
-                                 f[7] * xs[mpr_at(xx + 1, ry - 1)] + f[8] * xs[mpr_at(xx - 1, ry - 1)];
-                r = f[9] - ax;
-            }
-            rs[mpr_rat(x - 1, y - 1)] = r;
-            // owned: columns 2 i0 .. 2 i0 + 63 (E columns 2 .. 65), rows 2 j0 - 1 .. jhi
-            const int gi = ei0 + x, gj = ej0 + y;
-            if (x >= 2 && gi >= F.ilo && gi <= F.ihi && gj <= jhi)
-                store_mirrored(OUT, fl, gi, gj, W, per, ok[dy][dx] ? xr[dy][dx] : 0.0f);
+                for (int q = 0; q < 4; q++)
+                    if (r >= 1 && r <= 2 && q >= 1 && q <= 2) w[r][q] = xr[r - 1][q - 1];
+                    else w[r][q] = (2 * bx + q < MPR_XW && 2 * by + r < MPR_XH) ? xs[mpr_at(2 * bx + q, 2 * by + r)] : 0.0f;
         }
+        auto nb = [&](int r, int q) -> float { return WIDE ? w[r][q] : xs[mpr_at(2 * bx + q, 2 * by + r)]; };
+#pragma unroll
+        for (int dy = 0; dy < 2; dy++) {
+            const int y = 2 * by + dy, gj = ej0 + y;
+            if (y < 1 || y > MPR_RH) continue;
+            float v[2];
+#pragma unroll
+            for (int dx = 0; dx < 2; dx++) {
+                const float(&f)[10] = a[dy][dx];
+                float r = 0.0f;
+                if (ok[dy][dx]) {
+                    const float ax = f[0] * xr[dy][dx] + f[1] * nb(dy + 1, dx + 2) + f[2] * nb(dy + 1, dx) +
+                                     f[3] * nb(dy + 2, dx + 1) + f[4] * nb(dy, dx + 1) + f[5] * nb(dy + 2, dx + 2) +
+                                     f[6] * nb(dy + 2, dx) + f[7] * nb(dy, dx + 2) + f[8] * nb(dy, dx);
+                    r = f[9] - ax;
+                }
+                const int x = 2 * bx + dx;
+                if (x >= 1 && x <= MPR_RW) rs[mpr_rat(x - 1, y - 1)] = r;
+                v[dx] = ok[dy][dx] ? xr[dy][dx] : 0.0f;
+            }
+            // owned: columns 2 i0 .. 2 i0 + 63 (E columns 2 .. 65, both of a block or none), rows up to jhi
+            const int gi = ei0 + 2 * bx;
+            if (bx < 1 || bx > TX || gj > jhi) continue;
+            float* row = OUT + (long long)gj * fl;
+            if (gi >= F.ilo && gi + 1 <= F.ihi) *reinterpret_cast<float2*>(row + gi) = make_float2(v[0], v[1]);
+            else {
+                if (gi >= F.ilo && gi <= F.ihi) row[gi] = v[0];
+                if (gi + 1 >= F.ilo && gi + 1 <= F.ihi) row[gi + 1] = v[1];
+            }
+            if (per && gi == 0) { row[W] = v[0]; row[W + 1] = v[1]; }
+            if (per && gi == W - 2) { row[-2] = v[0]; row[-1] = v[1]; }
+        }
+    }
     g.sync();
     if (tid >= TX * TY) return;
     const int li = tid % TX, lj = tid / TX;
@@ -502,14 +603,19 @@ __device__ __forceinline__ void mg_prr_tile(const BatchDev& b, const CaseDev& c,
     mplane(b, C, M_B)[(long long)J * C.ld + I] = r4;
 }
 
-// bilinear prolongation of the coarse result at fine point (i, j), i in [0, W)
+// bilinear prolongation of the coarse result at fine point (i, j), i in [0, W): the four
+// coarse points around it are loaded without a branch (an even index repeats its own point),
+// since lanes of different parity would otherwise wait for one another's loads in turn: with
+// that and one set of coarse loads per 2 x 2 block, k_mg_gs went from 279 to 218 us per step
+// of the 256-case twin sweep
 __device__ __forceinline__ float mg_prolong_at(const float* XC, int cl, int i, int j) {
-    const int I = i >> 1, J = j >> 1;
-    const long long q = (long long)J * cl + I;
-    if (!(i & 1) && !(j & 1)) return XC[q];
-    if (!(j & 1)) return 0.5f * (XC[q] + XC[q + 1]);
-    if (!(i & 1)) return 0.5f * (XC[q] + XC[q + cl]);
-    return 0.25f * (XC[q] + XC[q + 1] + XC[q + cl] + XC[q + cl + 1]);
+    const int di = i & 1, dj = (j & 1) * cl;
+    const float* q = XC + (long long)(j >> 1) * cl + (i >> 1);
+    const float a = q[0], b = q[di], c = q[dj], d = q[dj + di];
+    if (di && dj) return 0.25f * (a + b + c + d);
+    if (di) return 0.5f * (a + b);
+    if (dj) return 0.5f * (a + c);
+    return a;
 }
 
 // Multicolour Gauss-Seidel sweeps of level l on a 32 x 16 tile (block Gauss-Seidel at tile
@@ -537,6 +643,7 @@ constexpr int MG_GS_XP = MG_GS_XH * MG_GS_XS;          // 432 = 16 mod 32 words
 static_assert(MG_GS_XS >= (MG_GS_XW + 1) / 2 && (2 * MG_GS_XS) % 32 == 16 && MG_GS_XP % 32 == 16,
               "parity halves must keep a colour pass free of bank conflicts");
 static_assert(MG_GS_THREADS == (TX / 2) * (TYJ / 2), "one thread per 2 x 2 block");
+static_assert(MG_GS_THREADS >= 2 * (MG_GS_XW + TYJ), "one thread per point of the ring");
 
 __device__ __forceinline__ int mg_gs_at(int xx, int ry) {  // halo point (xx, ry) in the split layout
     return (xx & 1) * MG_GS_XP + ry * MG_GS_XS + (xx >> 1);
@@ -582,26 +689,46 @@ __device__ __forceinline__ void mg_gs_tile(const BatchDev& b, const CaseDev& c, 
             a[dy][1][q] = v.y;
         }
     }
-    // x and its halo (with the prolonged coarse correction in mode 2)
-    constexpr int NXL = (MG_GS_XW * MG_GS_XH + MG_GS_THREADS - 1) / MG_GS_THREADS;
-    float xv[NXL];
-#pragma unroll
-    for (int m = 0; m < NXL; m++) {
-        const int e = tid + m * MG_GS_THREADS;
-        const int gj = j0 - 1 + e / MG_GS_XW, col = column(i0 - 1 + e % MG_GS_XW);
-        float v = 0.0f;
-        if (!zero && e < MG_GS_XW * MG_GS_XH && gj >= 0 && gj < n1 && col >= 0) {
-            v = X[(long long)gj * ld + col];
-            if (prolong && gj >= 1 && gj <= n1 - 2 && col >= L.ilo && col <= L.ihi)
-                v += mg_prolong_at(XC, cl, col, gj);
+    // x with the prolonged coarse correction (mode 2). The thread's own block starts at an even
+    // column and an odd row, so the same four coarse points serve all of its four points;
+    // the tile's ring of 100 points takes one thread each
+    float xv[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}}, xr = 0.0f;
+    const bool ring = tid < 2 * (MG_GS_XW + TYJ);
+    const int rx = tid < 2 * MG_GS_XW ? tid % MG_GS_XW : (tid & 1) * (MG_GS_XW - 1);
+    const int ry0 = tid < MG_GS_XW ? 0 : tid < 2 * MG_GS_XW ? MG_GS_XH - 1 : 1 + (tid - 2 * MG_GS_XW) / 2;
+    if (!zero) {
+        const int ga = j0 + 2 * by;  // the block's odd row
+        const int cc = c0 >= 0 ? c0 : 0, ra = ga < n1 ? ga : 1, rb = ga + 1 < n1 ? ga + 1 : 1;
+        const float2 va = *reinterpret_cast<const float2*>(X + (long long)ra * ld + cc);
+        const float2 vb = *reinterpret_cast<const float2*>(X + (long long)rb * ld + cc);
+        const int gj = j0 - 1 + ry0, col = column(i0 - 1 + rx);
+        const bool rin = ring && gj >= 0 && gj < n1 && col >= 0;
+        const float vr = rin ? X[(long long)gj * ld + col] : 0.0f;
+        float pa = 0.0f, pb = 0.0f, pc = 0.0f, pd = 0.0f, pr = 0.0f;
+        if (prolong) {
+            const float* q = XC + (long long)(ga <= n1 - 2 ? ga >> 1 : 0) * cl + (cc >> 1);
+            const float A = q[0], B = q[1], C = q[cl], D = q[cl + 1];
+            const bool run = rin && gj >= 1 && gj <= n1 - 2 && col >= L.ilo && col <= L.ihi;
+            pr = mg_prolong_at(XC, cl, run ? col : L.ilo, run ? gj : 1);
+            if (!run) pr = 0.0f;
+            pa = 0.5f * (A + C);
+            pb = 0.25f * (A + B + C + D);
+            pc = C;
+            pd = 0.5f * (C + D);
         }
-        xv[m] = v;
+        // a point outside the level is zero; a boundary point takes no correction
+        const bool in0 = c0 >= 0, in1 = c1 >= 0;
+        xv[0][0] = (in0 && ga < n1) ? (prolong && ok[0][0] ? va.x + pa : va.x) : 0.0f;
+        xv[0][1] = (in1 && ga < n1) ? (prolong && ok[0][1] ? va.y + pb : va.y) : 0.0f;
+        xv[1][0] = (in0 && ga + 1 < n1) ? (prolong && ok[1][0] ? vb.x + pc : vb.x) : 0.0f;
+        xv[1][1] = (in1 && ga + 1 < n1) ? (prolong && ok[1][1] ? vb.y + pd : vb.y) : 0.0f;
+        xr = vr + pr;
     }
 #pragma unroll
-    for (int m = 0; m < NXL; m++) {
-        const int e = tid + m * MG_GS_THREADS;
-        if (e < MG_GS_XW * MG_GS_XH) xs[mg_gs_at(e % MG_GS_XW, e / MG_GS_XW)] = xv[m];
-    }
+    for (int dy = 0; dy < 2; dy++)
+#pragma unroll
+        for (int dx = 0; dx < 2; dx++) xs[mg_gs_at(2 * bx + dx + 1, 2 * by + dy + 1)] = xv[dy][dx];
+    if (ring) xs[mg_gs_at(rx, ry0)] = xr;
 #pragma unroll
     for (int dy = 0; dy < 2; dy++)
 #pragma unroll
@@ -661,7 +788,7 @@ __device__ __forceinline__ void mg_coarse_regs(const BatchDev& b, const CaseDev&
     const float* A = mplane(b, L, M_AP);
     const float* Bv = mplane(b, L, M_B);
     for (int e = tid; e < L.n1 * sw; e += Grp::N) xs[e] = 0.0f;  // x = 0 (and boundaries)
-    float a[M][9], bv[M];
+    float a[M][9], bv[M], y[M];
     int col[M], o[M], mo[M];
 #pragma unroll
     for (int m = 0; m < M; m++) {
@@ -672,6 +799,7 @@ __device__ __forceinline__ void mg_coarse_regs(const BatchDev& b, const CaseDev&
 #pragma unroll
         for (int q = 0; q < 9; q++) a[m][q] = A[q * L.ps + k];
         bv[m] = Bv[k];
+        y[m] = __frcp_rn(a[m][0]);
         col[m] = in ? mg_colour(i, j, L.W, per) : -1;
         o[m] = j * sw + i + H;
         const int mi = mirror_col(i, L.W, per);
@@ -687,7 +815,7 @@ __device__ __forceinline__ void mg_coarse_regs(const BatchDev& b, const CaseDev&
                 const float sm = a[m][1] * x[1] + a[m][2] * x[-1] + a[m][3] * x[sw] + a[m][4] * x[-sw] +
                                  a[m][5] * x[sw + 1] + a[m][6] * x[sw - 1] + a[m][7] * x[-sw + 1] +
                                  a[m][8] * x[-sw - 1];
-                const float v = (bv[m] - sm) / a[m][0];
+                const float v = mg_div(bv[m] - sm, a[m][0], y[m]);
                 xs[o[m]] = v;
                 if (mo[m] >= 0) xs[mo[m]] = v;
             }
@@ -803,13 +931,13 @@ __device__ __forceinline__ DiagOut diag_cell(double ue, double uw, double un, do
 struct BcCase {
     const CaseDev& c;
     int ld, W, per, n1, n0, jf;
-    double d0, d1, dt, Re, Ri, Pi;
+    double d0, d1, dt, Ri;
     double *U, *V, *Tn, *UPn, *VPn, *P, *VORT;
     const double *To, *X, *Yc, *XIX, *XIY, *ETX, *ETY, *ALPH, *BETA, *GAM, *JAC, *VEC;
     __device__ __forceinline__ BcCase(const BatchDev& b, const CaseDev& c_, int cur) : c(c_) {
         const int nxt = cur ^ 1;
         ld = c.ld; W = c.W; per = c.periodic; n1 = c.n1; n0 = c.n0; jf = n1 - 1;
-        d0 = c.d0; d1 = c.d1; dt = c.dt; Re = c.Re; Ri = c.Ri; Pi = c.Pi;
+        d0 = c.d0; d1 = c.d1; dt = c.dt; Ri = c.Ri;
         U = plane(b, c, P_U); V = plane(b, c, P_V); P = plane(b, c, P_P); VORT = plane(b, c, P_VORT);
         Tn = plane(b, c, P_T0 + nxt); UPn = plane(b, c, P_UP0 + nxt); VPn = plane(b, c, P_VP0 + nxt);
         To = plane(b, c, P_T0 + cur);
@@ -823,7 +951,7 @@ struct BcCase {
 // O-grid: circulation contribution of column i at j = n1-2 (PSolver.cpp:1568-1576); saves the
 // far-field u, v before this update (uold of PSolver.cpp:1456) in s_old (2 (W + 1) doubles)
 __device__ __forceinline__ double bc_circ(const BcCase& a, int i, double* s_old) {
-    const double de = a.c.fix_circ_de ? 1.0 / (a.n0 - 1) : 1.0 / (a.n0 - 2);
+    const double de = a.c.circ_de;
     const long long k = (long long)(a.n1 - 2) * a.ld + i, kp = k + 1;
     double f1 = (a.U[k] * a.ETY[k] - a.V[k] * a.ETX[k]) * fabs(a.JAC[k]);
     double f2 = (a.U[kp] * a.ETY[kp] - a.V[kp] * a.ETX[kp]) * fabs(a.JAC[kp]);
@@ -834,7 +962,10 @@ __device__ __forceinline__ double bc_circ(const BcCase& a, int i, double* s_old)
 }
 
 // O-grid: far-field u, v, T of column i (PSolver.cpp:1549-1562, 1582-1609, 1632-1656)
-__device__ __forceinline__ void bc_far(const BcCase& a, int i, double circ, const double* s_old) {
+struct FarOut {
+    double u, v, T;
+};
+__device__ __forceinline__ FarOut bc_far(const BcCase& a, int i, double circ, const double* s_old) {
     const CaseDev& c = a.c;
     const double *U = a.U, *V = a.V, *X = a.X, *Yc = a.Yc;
     const long long kb = (long long)(a.jf - 1) * a.ld + i, k = (long long)a.jf * a.ld + i;
@@ -852,112 +983,139 @@ __device__ __forceinline__ void bc_far(const BcCase& a, int i, double circ, cons
     const double vr1 = vr0 * cr2 + vrinf * (1 - cr2);
     const double vth1 = vth0 * crk + vtinf * (1 - crk);
     const double vnn = c.uinf * a.VEC[2LL * a.ld + i] + c.vinf * a.VEC[3LL * a.ld + i];
-    double un, vn, tn;
+    FarOut o;
     if (vnn >= 0) {
-        un = c.uinf; vn = c.vinf; tn = 0.0;
+        o.u = c.uinf; o.v = c.vinf; o.T = 0.0;
     } else {
-        un = costh * vr1 - sinth * vth1;
-        vn = sinth * vr1 + costh * vth1;
+        o.u = costh * vr1 - sinth * vth1;
+        o.v = sinth * vr1 + costh * vth1;
         const double uet_old = a.ETX[k] * s_old[i] + a.ETY[k] * s_old[a.W + 1 + i];
-        tn = a.To[k] - (uet_old * a.dt / a.d1) * (a.To[k] - a.To[k - a.ld]);
+        o.T = a.To[k] - div_by(uet_old * a.dt, c.v1) * (a.To[k] - a.To[k - a.ld]);
     }
-    store_mirrored(a.U, a.ld, i, a.jf, a.W, a.per, un);
-    store_mirrored(a.V, a.ld, i, a.jf, a.W, a.per, vn);
-    store_mirrored(a.Tn, a.ld, i, a.jf, a.W, a.per, tn);
+    store_mirrored(a.U, a.ld, i, a.jf, a.W, a.per, o.u);
+    store_mirrored(a.V, a.ld, i, a.jf, a.W, a.per, o.v);
+    store_mirrored(a.Tn, a.ld, i, a.jf, a.W, a.per, o.T);
+    return o;
 }
 
 // O-grid: wall velocity of column i (PSolver.cpp:1617-1630)
-__device__ __forceinline__ void bc_wall(const BcCase& a, int i, double cwall) {
-    const double uw = -a.c.speed_amp * cwall * a.Yc[i];
-    const double vw = a.c.speed_amp * cwall * a.X[i];
+__device__ __forceinline__ double bc_wall_u(const BcCase& a, int i, double cwall) { return -a.c.speed_amp * cwall * a.Yc[i]; }
+__device__ __forceinline__ double bc_wall_v(const BcCase& a, int i, double cwall) { return a.c.speed_amp * cwall * a.X[i]; }
+__device__ __forceinline__ void bc_wall(const BcCase& a, int i, double uw, double vw) {
     store_mirrored(a.U, a.ld, i, 0, a.W, a.per, uw);
     store_mirrored(a.V, a.ld, i, 0, a.W, a.per, vw);
     store_mirrored(a.UPn, a.ld, i, 0, a.W, a.per, uw);
     store_mirrored(a.VPn, a.ld, i, 0, a.W, a.per, vw);
 }
 
-// O-grid: wall pressure of column i (PSolver.cpp:1668-1725); swall = sin(2 pi F t)
-__device__ __forceinline__ void bc_wall_p(const BcCase& a, int i, double swall) {
-    const int ld = a.ld;
-    const double *U = a.U, *V = a.V;
-    const double* Fl[2] = {U, V};
-    const double d0 = a.d0, d1 = a.d1;
-    const long long k = i;
-    double dpd[2];
-    const double uxi = a.XIX[k] * U[k] + a.XIY[k] * V[k];
-    const double uet = a.ETX[k] * U[k] + a.ETY[k] * V[k];
-    for (int m = 0; m < 2; m++) {
-        const double* f = Fl[m];
-        const double aa = a.ALPH[k] * (f[k + 1] + f[k - 1] - 2 * f[k]) / (d0 * d0);
-        const double gg = a.GAM[k] * (f[k + 2LL * ld] + f[k] - 2 * f[k + ld]) / (d1 * d1);
-        const double bb = a.BETA[k] * (f[k + ld + 1] + f[k - 1] - f[k + ld - 1] - f[k + 1]) / (2 * d0 * d1);
-        const double d2u = aa + gg - 2 * bb;
-        double cv = uxi * 0.5 * (f[k + 1] - f[k - 1]) / d0;
-        cv = cv + uet * (f[k + ld] - f[k]) / d1;
-        const double alc = (m == 0) ? a.c.accn_amp * swall * a.Yc[k] : -a.c.accn_amp * swall * a.X[k];
-        dpd[m] = 1.0 * d2u / a.Re - cv - alc + (m == 1 ? a.Ri * a.Tn[k] : 0.0);
+// cos and sin of the wall's phase 2 pi F t; exactly 1 and 0 for a wall at rest
+__device__ __forceinline__ void bc_phase(const CaseDev& c, double t, double& cw, double& sw) {
+    cw = 1.0;
+    sw = 0.0;
+    const double ang = 2.0 * c.Pi * c.F * t;
+    if (ang != 0.0) {
+        cw = cos(ang);
+        sw = sin(ang);
     }
-    const double pw = a.P[k + ld] - (dpd[0] * (-a.XIY[k] * a.JAC[k]) + dpd[1] * (a.XIX[k] * a.JAC[k])) * d1;
-    store_mirrored(a.P, ld, i, 0, a.W, a.per, pw);
 }
 
-// O-grid: far-field pressure of column i (PSolver.cpp:1726-1783)
-__device__ __forceinline__ void bc_far_p(const BcCase& a, int i, const double* s_old) {
+// u and v at a boundary point and its two neighbours along the boundary
+struct Edge {
+    double u, ue, uw, v, ve, vw;
+};
+__device__ __forceinline__ Edge edge_at(const BcCase& a, long long k) {
+    return Edge{a.U[k], a.U[k + 1], a.U[k - 1], a.V[k], a.V[k + 1], a.V[k - 1]};
+}
+
+// One component of the boundary momentum balance dp/dx_m = lap(f) / Re - conv(f) - accel +
+// (buoyancy) at a boundary point: f at the point (f0), its neighbours along the boundary (fe,
+// fw) and the two rows inside (f1, f2), the cross difference bd, the convection cy across
+// the boundary
+__device__ __forceinline__ double bc_force(const CaseDev& c, double f0, double fe, double fw, double f1, double f2,
+                                           double bd, double al, double ga, double be, double uxi, double cy,
+                                           double alc, double Ri, double T) {
+    const double aa = div_by(al * (fe + fw - 2 * f0), c.v00);
+    const double gg = div_by(ga * (f0 + f2 - 2 * f1), c.v11);
+    const double bb = div_by(be * bd, c.v01);
+    const double d2u = aa + gg - 2 * bb;
+    double cv = div_by(uxi * 0.5 * (fe - fw), c.v0);
+    cv = cv + cy;
+    return div_by(1.0 * d2u, c.vRe) - cv - alc + Ri * T;
+}
+
+// O-grid: wall pressure of column i (PSolver.cpp:1668-1725); swall = sin(2 pi F t)
+__device__ __forceinline__ double bc_wall_p(const BcCase& a, int i, const Edge& g, double swall) {
+    const int ld = a.ld;
+    const double *U = a.U, *V = a.V;
+    const double d1 = a.d1;
+    const long long k = i, k1 = k + ld, k2 = k + 2LL * ld;
+    const double al = a.ALPH[k], ga = a.GAM[k], be = a.BETA[k], x = a.XIX[k], y = a.XIY[k], J = a.JAC[k];
+    const double uxi = x * g.u + y * g.v;
+    const double uet = a.ETX[k] * g.u + a.ETY[k] * g.v;
+    const double u1 = U[k1], u2 = U[k2], ub = U[k1 + 1] + g.uw - U[k1 - 1] - g.ue;
+    const double v1 = V[k1], v2 = V[k2], vb = V[k1 + 1] + g.vw - V[k1 - 1] - g.ve;
+    const double alu = a.c.accn_amp * swall * a.Yc[k], alv = -a.c.accn_amp * swall * a.X[k];
+    const double T = a.Tn[k], p1 = a.P[k1];
+    const double fu = bc_force(a.c, g.u, g.ue, g.uw, u1, u2, ub, al, ga, be, uxi, div_by(uet * (u1 - g.u), a.c.v1), alu, 0.0, T);
+    const double fv = bc_force(a.c, g.v, g.ve, g.vw, v1, v2, vb, al, ga, be, uxi, div_by(uet * (v1 - g.v), a.c.v1), alv, a.Ri, T);
+    const double pw = p1 - (fu * (-y * J) + fv * (x * J)) * d1;
+    store_mirrored(a.P, ld, i, 0, a.W, a.per, pw);
+    return pw;
+}
+
+// O-grid: far-field pressure of column i (PSolver.cpp:1726-1783); T = its temperature
+__device__ __forceinline__ void bc_far_p(const BcCase& a, int i, const Edge& g, double T, const double* s_old) {
     const int ld = a.ld, W = a.W;
     const double *U = a.U, *V = a.V;
-    const double* Fl[2] = {U, V};
-    const double d0 = a.d0, d1 = a.d1;
-    const long long k = (long long)a.jf * ld + i;
+    const double d1 = a.d1;
+    const long long k = (long long)a.jf * ld + i, k1 = k - ld, k2 = k - 2LL * ld;
     const double vnn = a.c.uinf * a.VEC[2LL * ld + i] + a.c.vinf * a.VEC[3LL * ld + i];
+    const double ex = a.ETX[k], ey = a.ETY[k];
+    const double u1 = U[k1], u2 = U[k2], v1 = V[k1], v2 = V[k2];
     double pf;
     if (vnn >= 0) {
-        const double uxi = a.XIX[k] * U[k] + a.XIY[k] * V[k];
-        const double uet = a.ETX[k] * U[k] + a.ETY[k] * V[k];
-        double dpd[2];
-        for (int m = 0; m < 2; m++) {
-            const double* f = Fl[m];
-            const double fo = s_old[m * (W + 1) + i];
-            const double aa = a.ALPH[k] * (f[k + 1] + f[k - 1] - 2 * f[k]) / (d0 * d0);
-            const double gg = a.GAM[k] * (f[k] + f[k - 2LL * ld] - 2 * f[k - ld]) / (d1 * d1);
-            const double bb = a.BETA[k] * (f[k + 1] + f[k - ld - 1] - f[k - ld + 1] - f[k - 1]) / (2 * d0 * d1);
-            const double d2u = aa + gg - 2 * bb;
-            double cv = uxi * 0.5 * (f[k + 1] - f[k - 1]) / d0;
-            cv = cv + uet * (3.0 * f[k] - 4 * f[k - ld] + f[k - 2LL * ld]) / (2 * d1);
-            const double alc = (f[k] - fo) / a.dt;
-            dpd[m] = 1.0 * d2u / a.Re - cv - alc + (m == 1 ? a.Ri * a.Tn[k] : 0.0);
-        }
-        pf = a.P[k - ld] + (dpd[0] * (-a.XIY[k] * a.JAC[k]) + dpd[1] * (a.XIX[k] * a.JAC[k])) * d1;
+        const double al = a.ALPH[k], ga = a.GAM[k], be = a.BETA[k], x = a.XIX[k], y = a.XIY[k], J = a.JAC[k];
+        const double uxi = x * g.u + y * g.v;
+        const double uet = ex * g.u + ey * g.v;
+        const double ub = g.ue + U[k1 - 1] - U[k1 + 1] - g.uw, vb = g.ve + V[k1 - 1] - V[k1 + 1] - g.vw;
+        const double alu = div_by(g.u - s_old[i], a.c.vdt), alv = div_by(g.v - s_old[W + 1 + i], a.c.vdt);
+        const double nu = uet * (3.0 * g.u - 4 * u1 + u2), nv = uet * (3.0 * g.v - 4 * v1 + v2);
+        const double fu = bc_force(a.c, g.u, g.ue, g.uw, u1, u2, ub, al, ga, be, uxi, div_by(nu, a.c.v1x2), alu, 0.0, T);
+        const double fv = bc_force(a.c, g.v, g.ve, g.vw, v1, v2, vb, al, ga, be, uxi, div_by(nv, a.c.v1x2), alv, a.Ri, T);
+        pf = a.P[k1] + (fu * (-y * J) + fv * (x * J)) * d1;
     } else {
-        const double e0 = a.ETX[k] * U[k] + a.ETY[k] * V[k];
-        const long long k1 = k - ld, k2 = k - 2LL * ld;
-        const double e1 = a.ETX[k1] * U[k1] + a.ETY[k1] * V[k1];
-        const double e2 = a.ETX[k2] * U[k2] + a.ETY[k2] * V[k2];
-        pf = 0.5 * (1.0 / a.Re) * ((3 * e0 - 4 * e1 + e2) / d1);
+        const double e0 = ex * g.u + ey * g.v;
+        const double e1 = a.ETX[k1] * u1 + a.ETY[k1] * v1;
+        const double e2 = a.ETX[k2] * u2 + a.ETY[k2] * v2;
+        pf = 0.5 * a.c.vRe.y * div_by(3 * e0 - 4 * e1 + e2, a.c.v1);
     }
     store_mirrored(a.P, ld, i, a.jf, W, a.per, pf);
 }
 
 // vorticity of column i on boundary row j = 0 or n1-1 (PSolver.cpp:1855-1888)
-__device__ __forceinline__ void bc_vort(const BcCase& a, int i, int j) {
+__device__ __forceinline__ double bc_vort(const BcCase& a, int i, int j, const Edge& g) {
     const int ld = a.ld;
     const double *U = a.U, *V = a.V;
-    const double d0 = a.d0, d1 = a.d1;
+    const double hd0 = a.c.hd0, rd1 = a.c.rd1;
     const long long k = (long long)j * ld + i;
-    const double dv_dxi = 0.5 / d0 * (V[k + 1] - V[k - 1]);
-    const double dv_det = (j == 0) ? 1.0 / d1 * (V[k + ld] - V[k]) : 1.0 / d1 * (V[k] - V[k - ld]);
+    const double dv_dxi = hd0 * (g.ve - g.vw);
+    const double dv_det = (j == 0) ? rd1 * (V[k + ld] - g.v) : rd1 * (g.v - V[k - ld]);
     const double dv_dx = a.XIX[k] * dv_dxi + a.ETX[k] * dv_det;
-    const double du_dxi = 0.5 / d0 * (U[k + 1] - U[k - 1]);
-    const double du_det = (j == 0) ? 1.0 / d1 * (U[k + ld] - U[k]) : 1.0 / d1 * (U[k] - U[k - ld]);
+    const double du_dxi = hd0 * (g.ue - g.uw);
+    const double du_det = (j == 0) ? rd1 * (U[k + ld] - g.u) : rd1 * (g.u - U[k - ld]);
     const double du_dy = a.XIY[k] * du_dxi + a.ETY[k] * du_det;
-    store_mirrored(a.VORT, ld, i, j, a.W, a.per, dv_dx - du_dy);
+    const double w = dv_dx - du_dy;
+    store_mirrored(a.VORT, ld, i, j, a.W, a.per, w);
+    return w;
 }
 
 // contributions of column i to the forces, moment and Nusselt number on j = 0
-// (PSolver.cpp:1901-1983)
-__device__ __forceinline__ void bc_integral(const BcCase& a, int i, double (&acc)[7]) {
+// (PSolver.cpp:1901-1983); P, VORT: row 0 of p and the vorticity
+__device__ __forceinline__ void bc_integral(const BcCase& a, int i, const double* P, const double* VORT,
+                                            double (&acc)[7]) {
     const int ld = a.ld;
-    const double *P = a.P, *JAC = a.JAC, *VORT = a.VORT, *ETX = a.ETX, *ETY = a.ETY, *X = a.X, *Yc = a.Yc, *Tn = a.Tn;
-    const double d0 = a.d0, d1 = a.d1;
+    const double *JAC = a.JAC, *ETX = a.ETX, *ETY = a.ETY, *X = a.X, *Yc = a.Yc, *Tn = a.Tn;
+    const double d0 = a.d0;
     const long long k = i, kp = i + 1;
     const double PJ1 = P[k] * JAC[k], pj2 = P[kp] * JAC[kp];
     const double VJ1 = VORT[k] * JAC[k], VJ2 = VORT[kp] * JAC[kp];
@@ -971,8 +1129,8 @@ __device__ __forceinline__ void bc_integral(const BcCase& a, int i, double (&acc
     const double fp2 = pj2 * (X[kp] * ETY[kp] - Yc[kp] * ETX[kp]);
     const double fv1 = VJ1 * (X[k] * ETX[k] + Yc[k] * ETY[k]);
     const double fv2 = VJ2 * (X[kp] * ETX[kp] + Yc[kp] * ETY[kp]);
-    const double fh1 = TJ1 * (4 * Tn[k + ld] - 3 * Tn[k] - Tn[k + 2LL * ld]) / (2 * d1);
-    const double fh2 = TJ2 * (4 * Tn[kp + ld] - 3 * Tn[kp] - Tn[kp + 2LL * ld]) / (2 * d1);
+    const double fh1 = div_by(TJ1 * (4 * Tn[k + ld] - 3 * Tn[k] - Tn[k + 2LL * ld]), a.c.v1x2);
+    const double fh2 = div_by(TJ2 * (4 * Tn[kp + ld] - 3 * Tn[kp] - Tn[kp + 2LL * ld]), a.c.v1x2);
     acc[4] += 0.5 * d0 * (fp1 + fp2);
     acc[5] += 0.5 * d0 * (fv1 + fv2);
     acc[6] += 0.5 * (fh1 + fh2) * d0;
@@ -1004,8 +1162,9 @@ __device__ __forceinline__ void bc_cav_row(const BcCase& a, int j) {
     double *Tn = a.Tn, *P = a.P;
     const int n0 = a.n0;
     const long long r = (long long)j * a.ld;
-    Tn[r] = (4.0 * Tn[r + 1] - Tn[r + 2]) / 3.0;
-    Tn[r + n0 - 1] = (4.0 * Tn[r + n0 - 2] - Tn[r + n0 - 3]) / 3.0;
+    const DivBy three{3.0, 1.0 / 3.0};
+    Tn[r] = div_by(4.0 * Tn[r + 1] - Tn[r + 2], three);
+    Tn[r + n0 - 1] = div_by(4.0 * Tn[r + n0 - 2] - Tn[r + n0 - 3], three);
     P[r] = P[r + 1];
     P[r + n0 - 1] = P[r + n0 - 2];
 }

@@ -442,7 +442,7 @@ __device__ __forceinline__ int fin_case(const BatchDev& b, int cid, int* is, int
     is[I_MWORD] = nword;
 #pragma unroll
     for (int ty = 0; ty < 2; ty++) {  // Chebyshev weight of the next sweep
-        scw[S_CW0 + ty] = cheb_next(sweep, in.cw[ty], in.ca[ty], in.cb[ty]);
+        scw[S_CW0 + ty] = cheb_next(sweep, in.cw[ty], cheb_s2(in.ca[ty], in.cb[ty]));
     }
     // algorithmic-traffic counters (cells and field-cells swept)
     const unsigned long long nf = (unsigned long long)__popc(mask) * in.ncell;
