@@ -22,6 +22,7 @@
 #include "cfd_kernels.cuh"
 #include "cfd_reduce.cuh"
 #include "cfd_sweep.cuh"
+#include "cfd_team.cuh"
 
 using namespace cfd;
 
@@ -50,6 +51,7 @@ namespace {
 
 long long rup(long long x, long long a) { return (x + a - 1) / a * a; }
 
+constexpr int kTeamSteps = 32;  // steps of one team launch at most
 constexpr int NFLAGS = 10;  // device flag words of a batch
 
 enum KernelId {
@@ -209,6 +211,14 @@ struct cfd_batch {
     long long steps_done = 0;
     cudaStream_t st = nullptr;
     int dev = 0;
+    // the team kernel's launch (plan_team): CTAs per team (0: the step graph runs instead),
+    // cluster or cooperative grid, the cases with the largest first, its barrier counters
+    int team_nr = 0, team_cluster = 0;
+    int* team_ids = nullptr;
+    unsigned* team_bar = nullptr;
+    size_t cap_team_ids = 0, cap_team_bar = 0;
+    size_t team_smem_bytes = 0;
+    int team_clusters[5] = {};  // clusters of 1, 2, 4, 8, 16 CTAs resident at once (for team_smem_bytes)
     // profiling
     bool prof = false;
     std::vector<Launch> pending;
@@ -920,6 +930,47 @@ int one_step(cfd_batch* b) {
     return CFD_OK;
 }
 
+// `nsteps` steps of every case by the team kernel
+int team_steps(cfd_batch* b, int nsteps) {
+    TeamArgs a{};
+    a.b = b->bd;
+    a.b.cur = b->cur;
+    a.ids = b->team_ids;
+    a.bar = b->team_bar;
+    a.nr = b->team_nr;
+    a.cluster = b->team_cluster;
+    a.nsteps = nsteps;
+    a.sweep_cap = b->precision == CFD_PRECISION_MIXED ? 1 + mom_loop_cap(b) : 2 * mom_loop_cap(b);
+    a.maxit_p = b->maxit_p;
+    a.fin_threads = b->swf_threads;
+    a.nu_pre = b->mg_pre;
+    a.nu_post = b->mg_post;
+    a.coarse_sweeps = b->coarse_sweeps;
+    if (!a.cluster) CK(cudaMemsetAsync(b->team_bar, 0, sizeof(unsigned) * b->ntable_cases, b->st));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(a.nr * b->ntable_cases));
+    cfg.blockDim = dim3(TEAM_THREADS);
+    cfg.dynamicSmemBytes = b->team_smem_bytes;
+    cfg.stream = b->st;
+    cudaLaunchAttribute at = {};
+    if (a.cluster) {
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = (unsigned)a.nr;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    } else {
+        at.id = cudaLaunchAttributeCooperative;
+        at.val.cooperative = 1;
+    }
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    if (b->precision == CFD_PRECISION_MIXED) CK(cudaLaunchKernelEx(&cfg, k_team_mx, a));
+    else CK(cudaLaunchKernelEx(&cfg, k_team_f64, a));
+    b->launches++;
+    b->cur ^= nsteps & 1;
+    b->steps_done += nsteps;
+    return CFD_OK;
+}
+
 // adds the loop launches of graph steps (from the cumulative device counters) to the count
 void drop_graphs(cfd_batch* b) {
     for (int k = 0; k < 2; k++)
@@ -1109,6 +1160,80 @@ int grow(T*& ptr, size_t& cap, size_t need) {
     return CFD_OK;
 }
 
+// How the team kernel (cfd_team.cu) steps these cases, or whether the step graph does: sets
+// b->team_nr and b->team_cluster.
+//
+// The teams of all cases run at the same time (one CTA per SM), so a team gets 1 / n of the chip:
+// as a cluster, the largest power of two up to 16 that n clusters of leave room for, or as a
+// share of a cooperative grid. A step costs a team about 80 us (FP64 form) plus 14 us per
+// 32 x 16 tile and CTA of the largest case, the step graph 160 us plus 0.25 us per tile of the
+// batch, with less to gain the more of the chip the work fills. Measured, us per step, graph
+// against team:
+//   O-grids, 1 case:   65^2 169 / 90, 129^2 166 / 105, 257^2 197 / 121, 513^2 300 / 241 (3.5
+//                      tiles per CTA), 1025^2 672 / 698 (13.8)
+//   n cases:           16 x 33^2 169 / 82, 128 x 33^2 201 / 123, 64 x 65^2 252 / 188, 128 x 65^2
+//                      355 / 318 (8), 16 x 193^2 373 / 331 (8), 64 x 129^2 506 / 550 (16),
+//                      4 x 513^2 598 / 612 (13.8); a second wave of teams loses (256 x 65^2 558 / 630)
+//   cavities, mixed:   65^2 273 / 129, 257^2 319 / 203, 16 x 129^2 478 / 358, 64 x 129^2 901 / 1151 (16)
+// so teams run when they all fit at once and have at most 8 tiles per CTA. A cluster's barrier
+// is quicker than a counter's, but its size is a power of two: with more than two tiles per CTA
+// the larger share of a grid pays (16 x 129^2: clusters of 4 266, grid shares of 9 192).
+constexpr int kTeamTilesPerCta = 8;
+int plan_team(cfd_batch* b, const std::vector<int>& ids) {
+    b->team_nr = 0;
+    const int n = (int)ids.size();
+    if (n == 0) return CFD_OK;
+    std::vector<int> order(ids);
+    auto tiles = [&](int c) { return b->hc[c].jt_count; };
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return tiles(x) > tiles(y); });
+    const int most = tiles(order[0]);
+    int sms = 0;
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->dev));
+    if (n > sms || most > kTeamTilesPerCta * (sms / n)) return CFD_OK;
+    const size_t smem = team_smem(b->max_W);
+    const void* k = b->precision == CFD_PRECISION_MIXED ? (const void*)k_team_mx : (const void*)k_team_f64;
+    if (smem != b->team_smem_bytes) {
+        // clusters of 2^q CTAs that are resident at once; the kernel's limit is the device's, since
+        // batches of other widths share the attribute
+        int most_smem = 0;
+        CK(cudaDeviceGetAttribute(&most_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->dev));
+        if (smem > (size_t)most_smem) return CFD_OK;
+        CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most_smem));
+        CK(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        for (int q = 0; q <= 4; q++) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(1u << q);
+            cfg.blockDim = dim3(TEAM_THREADS);
+            cfg.dynamicSmemBytes = smem;
+            cudaLaunchAttribute at = {};
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = 1u << q;
+            at.val.clusterDim.y = at.val.clusterDim.z = 1;
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            if (cudaOccupancyMaxActiveClusters(&b->team_clusters[q], k, &cfg) != cudaSuccess) {
+                cudaGetLastError();
+                b->team_clusters[q] = 0;
+            }
+        }
+        b->team_smem_bytes = smem;
+    }
+    int nr_c = 0;
+    for (int q = 0; q <= 4; q++)
+        if (b->team_clusters[q] >= n) nr_c = 1 << q;
+    const int nr_g = sms / n;
+    const bool cluster = nr_c > 0 && (most <= 2 * nr_c || 2 * nr_g < 3 * nr_c);
+    const int nr = cluster ? nr_c : nr_g;
+    if (most > kTeamTilesPerCta * nr) return CFD_OK;
+    if (int rc = grow(b->team_ids, b->cap_team_ids, order.size())) return rc;
+    if (int rc = grow(b->team_bar, b->cap_team_bar, order.size())) return rc;
+    CK(cudaMemcpyAsync(b->team_ids, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice, b->st));
+    CK(cudaStreamSynchronize(b->st));
+    b->team_nr = nr;
+    b->team_cluster = cluster;
+    return CFD_OK;
+}
+
 // The tile tables of the cases `ids` (in that order; a case's tiles in row-major tile order,
 // so every per-case reduction sums in the same order whatever else is in the tables), each
 // case's offsets into them, the batch-wide maxima the launches use, and the device copies.
@@ -1182,6 +1307,7 @@ int build_tables(cfd_batch* b, const std::vector<int>& ids) {
         bd.mtiles[l] = b->dtiles + pos_mt[l]; bd.nmtiles[l] = (int)mt[l].size();
         bd.ccases[l] = b->dcc + pos_cc[l]; bd.nccases[l] = (int)cc[l].size();
     }
+    if (int rc = plan_team(b, ids)) return rc;
     b->ntable_cases = (int)ids.size();
     b->sw_grid = (int)jtiles.size();  // one CTA per 32 x 16 tile
     b->swf_threads = jt_max >= 1024 ? SWF_THREADS : 128;
@@ -1656,7 +1782,11 @@ size_t cfd_pool_case_bytes(int n0, int n1, int profile) {
 
 int cfd_batch_step(cfd_batch* b, int nsteps) {
     if (!b || nsteps < 0) return fail(CFD_E_ARG, "bad arguments");
-    for (int s = 0; s < nsteps; s++) {
+    // the team kernel has form 2 of the V-cycle only, and no copy waits for a limit to bound
+    const bool team = b->team_nr > 0 && b->use_graph && !b->prof && b->mg_fused == 2 && b->bd.wait_polls == kWaitPolls;
+    for (int s = 0; team && s < nsteps; s += kTeamSteps)
+        if (int rc = team_steps(b, std::min(kTeamSteps, nsteps - s))) return rc;
+    for (int s = 0; !team && s < nsteps; s++) {
         int rc = one_step(b);
         if (rc) return rc;
     }
@@ -1700,6 +1830,7 @@ int cfd_batch_destroy(cfd_batch* b) {
     cudaFree(b->f64); cudaFree(b->dc); cudaFree(b->scal); cudaFree(b->iscal);
     cudaFree(b->stage); cudaFree(b->stage_off);
     cudaFree(b->partial); cudaFree(b->counter); cudaFree(b->flags); cudaFree(b->work); cudaFree(b->tword); cudaFree(b->dtiles); cudaFree(b->dcc); cudaFree(b->dtmaps);
+    cudaFree(b->team_ids); cudaFree(b->team_bar);
     if (b->h_flags) cudaFreeHost(b->h_flags);
     if (b->st) cudaStreamDestroy(b->st);
     delete b;

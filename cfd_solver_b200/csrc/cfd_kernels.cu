@@ -608,7 +608,7 @@ __global__ void __launch_bounds__(MGC_THREADS) k_mg_coarse(BatchDev b, int l, in
     const int cid = l >= 0 ? b.ccases[l][blockIdx.x] : b.ccases[0][blockIdx.x];
     if (b.iscal[(long long)cid * NISCAL + I_PDONE]) return;
     const CaseDev& c = b.cases[cid];
-    mg_coarse_solve(b, c, c.lev[l >= 0 ? l : c.nlev - 1], sweeps, xs, MGC_SMEM, BlockGroup<MGC_THREADS>());
+    mg_coarse_solve<1>(b, c, c.lev[l >= 0 ? l : c.nlev - 1], sweeps, xs, MGC_SMEM, BlockGroup<MGC_THREADS>());
 }
 
 // Galerkin coarse operator A_{l+1} = R A_l P (R full weighting, P bilinear, R = P^T / 4)

@@ -770,63 +770,91 @@ __device__ __forceinline__ void mg_gs_tile(const BatchDev& b, const CaseDev& c, 
 }
 
 // Coarsest level: `sweeps` multicolour Gauss-Seidel sweeps by one group, x in shared memory
-// (all rows, columns -H .. W+H-1) and M unknowns' stencils in each thread's registers. The
-// points of a colour do not read one another, so the split over threads does not show in the
-// result. M = 1, 2, 4 cover every level of up to 4 N unknowns. A sweep is bound by the latency
-// of its colour passes (a barrier and eight shared loads each); through global memory, which
-// levels of more than one unknown per thread used before, each pass paid L2 round trips
-// instead: five steps of a 181 x 91 O-grid (45 x 44 unknowns on its coarsest level, six
-// colours, 12 sweeps) took 5.75 ms and now take 2.84 ms.
-template <int M, class Grp>
+// (all rows, columns -H .. W+H-1). A thread holds the stencils of up to K points of each of the
+// four parity colours in registers, so that every pass keeps all lanes busy; the last column
+// of an odd periodic width has two colours of its own, whose few stencils are read where
+// they are used. The points of a colour do not read one another, so the split over threads
+// does not show in the result. A sweep is bound by the latency of its passes (a barrier,
+// eight shared loads, eight multiply-adds, a quotient); through global memory, which levels
+// of more than one unknown per thread used before, each pass paid L2 round trips instead: five
+// steps of a 181 x 91 O-grid (90 x 44 unknowns on its coarsest level) took 5.75 ms, with the
+// stencils in registers 2.68.
+struct MgColour {
+    int fi, fj, nx, n;  // first column and row, points in a row, points
+    __device__ __forceinline__ MgColour(const LevelDev& L, int per, int cc) {
+        const int ie = per && (L.W & 1) ? L.W - 2 : L.ihi;
+        fi = L.ilo + ((L.ilo ^ cc) & 1);
+        fj = 1 + ((1 ^ (cc >> 1)) & 1);
+        nx = ie >= fi ? (ie - fi) / 2 + 1 : 0;
+        n = L.n1 - 2 >= fj ? nx * ((L.n1 - 2 - fj) / 2 + 1) : 0;
+    }
+};
+template <int K, class Grp>
 __device__ __forceinline__ void mg_coarse_regs(const BatchDev& b, const CaseDev& c, const LevelDev& L, int sweeps,
                                                float* xs, const Grp& g) {
-    const int ld = L.ld, per = c.periodic, tid = g.tid;
-    const int nx = L.ihi - L.ilo + 1, ny = L.n1 - 2;
-    const int ncol = (per && (L.W & 1)) ? 6 : 4;
-    const int sw = L.W + 2 * H;
+    const int ld = L.ld, per = c.periodic, tid = g.tid, W = L.W;
+    const int sw = W + 2 * H;
     float* X = mplane(b, L, M_X);
     const float* A = mplane(b, L, M_AP);
     const float* Bv = mplane(b, L, M_B);
     for (int e = tid; e < L.n1 * sw; e += Grp::N) xs[e] = 0.0f;  // x = 0 (and boundaries)
-    float a[M][9], bv[M], y[M];
-    int col[M], o[M], mo[M];
+    float a[4][K][9], bv[4][K], y[4][K];
+    int o[4][K];  // position in xs, and 1 / 2 in the top bits for a mirror W to the right / left; -1: none
 #pragma unroll
-    for (int m = 0; m < M; m++) {
-        const int e = tid + m * Grp::N;
-        const bool in = e < nx * ny;
-        const int i = L.ilo + (in ? e % nx : 0), j = 1 + (in ? e / nx : 0);
-        const long long k = (long long)j * ld + i;
+    for (int cc = 0; cc < 4; cc++) {
+        const MgColour q(L, per, cc);
 #pragma unroll
-        for (int q = 0; q < 9; q++) a[m][q] = A[q * L.ps + k];
-        bv[m] = Bv[k];
-        y[m] = __frcp_rn(a[m][0]);
-        col[m] = in ? mg_colour(i, j, L.W, per) : -1;
-        o[m] = j * sw + i + H;
-        const int mi = mirror_col(i, L.W, per);
-        mo[m] = mi > -1000000 ? j * sw + mi + H : -1;
+        for (int k = 0; k < K; k++) {
+            const int e = tid + k * Grp::N;
+            const bool in = e < q.n;
+            const int i = in ? q.fi + 2 * (e % q.nx) : L.ilo, j = in ? q.fj + 2 * (e / q.nx) : 1;
+            const long long p = (long long)j * ld + i;
+#pragma unroll
+            for (int m = 0; m < 9; m++) a[cc][k][m] = A[m * L.ps + p];
+            bv[cc][k] = Bv[p];
+            y[cc][k] = __frcp_rn(a[cc][k][0]);
+            o[cc][k] = in ? (j * sw + i + H) | ((per ? (i < 2 ? 1 : i >= W - 2 ? 2 : 0) : 0) << 28) : -1;
+        }
     }
+    auto relax = [&](int at, const float(&f)[9], float rhs, float rd) -> float {
+        const float* x = xs + at;
+        const float sm = f[1] * x[1] + f[2] * x[-1] + f[3] * x[sw] + f[4] * x[-sw] + f[5] * x[sw + 1] +
+                         f[6] * x[sw - 1] + f[7] * x[-sw + 1] + f[8] * x[-sw - 1];
+        return mg_div(rhs - sm, f[0], rd);
+    };
     g.sync();
     for (int s = 0; s < sweeps; s++) {
-        for (int cc = 0; cc < ncol; cc++) {
 #pragma unroll
-            for (int m = 0; m < M; m++) {
-                if (col[m] != cc) continue;
-                const float* x = xs + o[m];
-                const float sm = a[m][1] * x[1] + a[m][2] * x[-1] + a[m][3] * x[sw] + a[m][4] * x[-sw] +
-                                 a[m][5] * x[sw + 1] + a[m][6] * x[sw - 1] + a[m][7] * x[-sw + 1] +
-                                 a[m][8] * x[-sw - 1];
-                const float v = mg_div(bv[m] - sm, a[m][0], y[m]);
-                xs[o[m]] = v;
-                if (mo[m] >= 0) xs[mo[m]] = v;
+        for (int cc = 0; cc < 4; cc++) {
+#pragma unroll
+            for (int k = 0; k < K; k++) {
+                if (o[cc][k] < 0) continue;
+                const int at = o[cc][k] & 0xfffffff, m = o[cc][k] >> 28;
+                const float v = relax(at, a[cc][k], bv[cc][k], y[cc][k]);
+                xs[at] = v;
+                if (m) xs[m == 1 ? at + W : at - W] = v;
+            }
+            g.sync();
+        }
+        if (!(per && (W & 1))) continue;
+        for (int cc = 0; cc < 2; cc++) {  // the last column's even rows, then its odd rows
+            for (int j = 2 - cc + 2 * tid; j <= L.n1 - 2; j += 2 * Grp::N) {
+                const long long p = (long long)j * ld + W - 1;
+                float f[9];
+#pragma unroll
+                for (int m = 0; m < 9; m++) f[m] = A[m * L.ps + p];
+                const int at = j * sw + W - 1 + H;
+                const float v = relax(at, f, Bv[p], __frcp_rn(f[0]));
+                xs[at] = v;
+                xs[at - W] = v;
             }
             g.sync();
         }
     }
-#pragma unroll
-    for (int m = 0; m < M; m++) {
-        if (col[m] < 0) continue;
-        const int e = tid + m * Grp::N;
-        store_mirrored(X, ld, L.ilo + e % nx, 1 + e / nx, L.W, per, xs[o[m]]);
+    const int nx = L.ihi - L.ilo + 1;
+    for (int e = tid; e < nx * (L.n1 - 2); e += Grp::N) {
+        const int i = L.ilo + e % nx, j = 1 + e / nx;
+        store_mirrored(X, ld, i, j, W, per, xs[j * sw + i + H]);
     }
 }
 
@@ -861,14 +889,16 @@ __device__ __forceinline__ void mg_coarse_global(const BatchDev& b, const CaseDe
     }
 }
 
-template <class Grp>
+// KMAX: points of a colour per thread that the kernel's registers have room for
+template <int KMAX, class Grp>
 __device__ __forceinline__ void mg_coarse_solve(const BatchDev& b, const CaseDev& c, const LevelDev& L, int sweeps,
                                                 float* xs, int xs_cap, const Grp& g) {
-    const int n = (L.ihi - L.ilo + 1) * (L.n1 - 2);
-    if (n > 4 * Grp::N || L.n1 * (L.W + 2 * H) > xs_cap) mg_coarse_global(b, c, L, sweeps, g);
-    else if (n <= Grp::N) mg_coarse_regs<1>(b, c, L, sweeps, xs, g);
-    else if (n <= 2 * Grp::N) mg_coarse_regs<2>(b, c, L, sweeps, xs, g);
-    else mg_coarse_regs<4>(b, c, L, sweeps, xs, g);
+    // the odd rows' colours have at least as many points as the even rows', and one of the two
+    // column parities the most
+    const int most = max(MgColour(L, c.periodic, 2).n, MgColour(L, c.periodic, 3).n);
+    if (most > KMAX * Grp::N || L.n1 * (L.W + 2 * H) > xs_cap) mg_coarse_global(b, c, L, sweeps, g);
+    else if (KMAX == 1 || most <= Grp::N) mg_coarse_regs<1>(b, c, L, sweeps, xs, g);
+    else mg_coarse_regs<KMAX>(b, c, L, sweeps, xs, g);
 }
 
 // ---------------------------------------------------------------------------
@@ -998,9 +1028,14 @@ __device__ __forceinline__ FarOut bc_far(const BcCase& a, int i, double circ, co
     return o;
 }
 
-// O-grid: wall velocity of column i (PSolver.cpp:1617-1630)
-__device__ __forceinline__ double bc_wall_u(const BcCase& a, int i, double cwall) { return -a.c.speed_amp * cwall * a.Yc[i]; }
-__device__ __forceinline__ double bc_wall_v(const BcCase& a, int i, double cwall) { return a.c.speed_amp * cwall * a.X[i]; }
+// O-grid: wall velocity of column i (PSolver.cpp:1617-1630). Rounded products: the team kernel
+// forms a neighbour's value where k_bc reads it, so it must not melt into a later sum.
+__device__ __forceinline__ double bc_wall_u(const BcCase& a, int i, double cwall) {
+    return __dmul_rn(__dmul_rn(-a.c.speed_amp, cwall), a.Yc[i]);
+}
+__device__ __forceinline__ double bc_wall_v(const BcCase& a, int i, double cwall) {
+    return __dmul_rn(__dmul_rn(a.c.speed_amp, cwall), a.X[i]);
+}
 __device__ __forceinline__ void bc_wall(const BcCase& a, int i, double uw, double vw) {
     store_mirrored(a.U, a.ld, i, 0, a.W, a.per, uw);
     store_mirrored(a.V, a.ld, i, 0, a.W, a.per, vw);

@@ -166,7 +166,9 @@ int cfd_batch_set_mg(cfd_batch* b, int nu_pre, int nu_post, int coarse_sweeps, i
  * once, which only tests the error path). A wait that gives up sets the batch's error
  * flag and the kernel returns (after its copies have landed); the step then fails with
  * CFD_E_CUDA ("a bounded wait inside a kernel timed out") and the batch's fields are
- * invalid: destroy it. The device stays usable. */
+ * invalid: destroy it. The device stays usable. Small batches step by a kernel without such
+ * copies (one launch for several steps); with a limit other than the default they step launch
+ * by launch, with the same bits. */
 int cfd_batch_set_wait_limit(cfd_batch* b, long long polls);
 int cfd_batch_get_mg(cfd_batch* b, int* nu_pre, int* nu_post, int* coarse_sweeps, int* fused);
 int cfd_batch_autotune(cfd_batch* b, int steps, int* out_schedule4, double* out_ms_per_step);
