@@ -7,7 +7,7 @@
 // For them this entry point runs the same solve as cfd_gauss_solve() with its scratch
 // (the second iterate, the reduction partials and a few scalars) in one file-scope
 // device array of fixed size, so the call itself allocates nothing. The solve reads its
-// stop flag on the host after every pair of sweeps, so each call waits for its own work.
+// outcome on the host, so each call waits for its own work.
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -24,7 +24,7 @@ namespace {
 
 // largest grid (n0 * n1 points) the static scratch serves: 2^20 points (1025 x 1023)
 constexpr long long kMaxPoints = CFD_NOALLOC_MAX_POINTS;
-// second iterate + one partial per 256 cells (rounded) + scalars + counter
+// second iterate, scalars, two partial buffers (cfd_seam_scratch_doubles())
 constexpr long long kScratchDoubles = kMaxPoints + (kMaxPoints / 256 + 64) + 16;
 
 // Every GPU that loads this library holds this array (about 8.4 MB) until the process

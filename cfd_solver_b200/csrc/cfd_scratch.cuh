@@ -1,0 +1,18 @@
+// cfd_scratch.cuh -- device scratch of the seams' calls.
+//
+// A seam call needs scratch for its own duration only. cudaMalloc and cudaFree per call cost
+// 0.7 to 3 ms on a busy host (they synchronise the device and take the driver's locks), more
+// than the solve itself; here the scratch comes from a pool of the library, one per device,
+// stream-ordered on the caller's stream, so calls from several threads and streams share it
+// safely. The pool keeps at most kScratchKeep bytes between calls and gives anything above back
+// to the device at the next synchronisation.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace cfd {
+constexpr unsigned long long kScratchKeep = 256ull << 20;
+// scratch of `bytes` bytes on the current device, usable by work on `st`; nullptr: no memory
+void* scratch_take(size_t bytes, cudaStream_t st);
+// gives it back once the work queued on `st` so far is done
+void scratch_give(void* p, cudaStream_t st);
+}  // namespace cfd

@@ -10,18 +10,37 @@
 // column n0-1 duplicates column 0 as in the reference, unknowns i = 0..n0-2;
 // otherwise columns 0 and n0-1 are fixed. 9-point rows: j = 1, n1-2 (and, when not
 // periodic, i = 1, n0-2).
+//
+// The whole solve is one cooperative launch: the bounds, the sweeps and the stop rule, with a
+// counter barrier between them whose polls are bounded. The host reads the outcome once (per
+// kSeamSweeps sweeps). Every CTA sums the partial residuals itself in the same order, so all
+// take the same decision. The pass that finds the bounds also forms the first sweep's Jacobi
+// corrections, which need only the step length 2 / (a + b) from it: the first sweep then adds
+// them without reading the 25 planes again. Bound by the coefficient planes' bytes on large
+// grids (1025^2: 41 us a sweep of 28 planes, 5.7 TB/s; 24 sweeps 2.73 -> 1.05 ms a call) and by
+// the launch, the barriers and the loads' latency on small ones (257^2, 4 sweeps: 772 -> 50 us;
+// before, a cudaMalloc, a launch per sweep, a host wait per pair and a cudaFree).
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <atomic>
 #include <cmath>
+#include <mutex>
 
 #include "../../include/cfd_b200.h"
+#include "cfd_scratch.cuh"
 
 namespace cfd_seam {
 
 constexpr int BS = 256;
+constexpr int MAX_BLOCKS = 2048;         // rows of a partial buffer
+constexpr int kSeamSweeps = 512;         // sweeps of one launch at most
+constexpr unsigned kSeamPolls = 1u << 24;  // polls of the barrier before it gives up (about 10 s)
 
-// scratch layout (doubles): [0..7] scalars, [8..8+nblk) partials, then the second iterate
-enum { SC_MAXAP, SC_MAXOFF, SC_R0, SC_R, SC_W, SC_DONE, SC_CNT, SC_A };
+// scratch layout (doubles): scalars, two partial buffers of three columns, the second iterate
+enum { SC_A, SC_B, SC_R0, SC_W, SC_DONE, SC_SWEEPS, SC_FAIL, SC_CNT, NSC };
+constexpr int SCRATCH_HEAD = 8 + 4096;
+static_assert(NSC <= 8 && 8 + 2 * MAX_BLOCKS <= SCRATCH_HEAD, "scratch layout");
 
 struct Sys {
     int n0, n1, periodic;
@@ -30,142 +49,239 @@ struct Sys {
     double* x1;           // scratch iterate
     const double* q;
     double* sc;           // scalars
-    double* part;         // per-block partials
-    unsigned int* cnt;
+    double* part;         // per-block partials, two buffers of MAX_BLOCKS
+    unsigned int* cnt;    // barrier arrivals, zero at launch
 };
 
 // gauss() argument order: ap, ae, as, an, aw, ase, asw, ane, anw, ass, assee, assww, asse,
 // assw, asee, asww, ann, annee, annww, anne, annw, anee, anww, aee, aww
-__constant__ int kDx[25] = {0, 1, 0, 0, -1, 1, -1, 1, -1, 0, 2, -2, 1, -1, 2, -2, 0, 2, -2, 1, -1, 2, -2, 2, -2};
-__constant__ int kDy[25] = {0, 0, -1, 1, 0, -1, -1, 1, 1, -2, -2, -2, -2, -2, -1, -1, 2, 2, 2, 2, 2, 1, 1, 0, 0};
-
-__device__ __forceinline__ bool cell_of(const Sys& s, int e, int& i, int& j) {
-    const int ilo = s.periodic ? 0 : 1, ihi = s.n0 - 2;
-    const int nx = ihi - ilo + 1, ny = s.n1 - 2;
-    if (e >= nx * ny) return false;
-    i = ilo + e % nx;
-    j = 1 + e / nx;
-    return true;
+__host__ __device__ constexpr int dx_of(int m) {
+    constexpr int d[25] = {0, 1, 0, 0, -1, 1, -1, 1, -1, 0, 2, -2, 1, -1, 2, -2, 0, 2, -2, 1, -1, 2, -2, 2, -2};
+    return d[m];
+}
+__host__ __device__ constexpr int dy_of(int m) {
+    constexpr int d[25] = {0, 0, -1, 1, 0, -1, -1, 1, 1, -2, -2, -2, -2, -2, -1, -1, 2, 2, 2, 2, 2, 1, 1, 0, 0};
+    return d[m];
 }
 
-__device__ __forceinline__ int wrap(const Sys& s, int i) {
-    if (!s.periodic) return i;
-    const int P = s.n0 - 1;
-    return i < 0 ? i + P : (i >= P ? i - P : i);
-}
-
-__device__ __forceinline__ bool near9(const Sys& s, int i, int j) {
-    if (j == 1 || j == s.n1 - 2) return true;
-    return !s.periodic && (i == 1 || i == s.n0 - 2);
-}
-
-__device__ double block_sum(double v, double* sm) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = v;
+// all CTAs have arrived and see one another's stores; false when the polls ran out
+__device__ __forceinline__ bool seam_barrier(const Sys& s, unsigned& target) {
+    target += gridDim.x;
     __syncthreads();
-    double r = 0.0;
-    if (threadIdx.x < 32) {
-        r = threadIdx.x < (blockDim.x >> 5) ? sm[threadIdx.x] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) r += __shfl_down_sync(0xffffffffu, r, o);
-    }
-    __syncthreads();
-    return r;
-}
-
-__device__ double block_max(double v, double* sm) {
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
-    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = v;
-    __syncthreads();
-    double r = 0.0;
-    if (threadIdx.x < 32) {
-        r = threadIdx.x < (blockDim.x >> 5) ? sm[threadIdx.x] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) r = fmax(r, __shfl_down_sync(0xffffffffu, r, o));
-    }
-    __syncthreads();
-    return r;
-}
-
-// spectrum bounds: max ap and max sum|a_nb|/ap over the unknowns (all values >= 0)
-__global__ void __launch_bounds__(BS) k_seam_bounds(Sys s) {
-    __shared__ double sm[32];
-    int i, j;
-    double ap = 0.0, off = 0.0;
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (cell_of(s, e, i, j)) {
-        const long long k = (long long)j * s.n0 + i;
-        ap = fabs(s.c[0][k]);
-        const int nc = near9(s, i, j) ? 9 : 25;
-        for (int m = 1; m < nc; m++) off += fabs(s.c[m][k]);
-        off /= ap;
-    }
-    const double a = block_max(ap, sm), o = block_max(off, sm);
+    bool got = true;
     if (threadIdx.x == 0) {
-        atomicMax((unsigned long long*)&s.sc[SC_MAXAP], __double_as_longlong(a));
-        atomicMax((unsigned long long*)&s.sc[SC_MAXOFF], __double_as_longlong(o));
-    }
-}
-
-// one Chebyshev-Jacobi sweep src -> dst (x_{k+1} overwrites x_{k-1} in dst)
-__global__ void __launch_bounds__(BS) k_seam_sweep(Sys s, int to_scratch, int sweep, double tol) {
-    __shared__ double sm[32];
-    __shared__ int last;
-    if (s.sc[SC_DONE] != 0.0) return;
-    const double* src = to_scratch ? s.x0 : s.x1;
-    double* dst = to_scratch ? s.x1 : s.x0;
-    const double a = 0.9 / s.sc[SC_MAXAP], b = 1.05 * (1.0 + s.sc[SC_MAXOFF]);
-    const double g = 2.0 / (a + b);
-    const double w = sweep == 0 ? 1.0 : s.sc[SC_W];
-    int i, j;
-    double r = 0.0;
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (cell_of(s, e, i, j)) {
-        const int n0 = s.n0;
-        const long long k = (long long)j * n0 + i;
-        const int nc = near9(s, i, j) ? 9 : 25;
-        double sum = 0.0;
-        for (int m = 1; m < nc; m++) {
-            const int ii = wrap(s, i + kDx[m]), jj = j + kDy[m];
-            sum += s.c[m][k] * src[(long long)jj * n0 + ii];
-        }
-        const double ap = s.c[0][k], rhs = s.q[k], xk = src[k];
-        const double xj = (rhs - sum) / ap;
-        double xn = xk + g * (xj - xk);
-        if (sweep > 0) {
-            const double xm = dst[k];
-            xn = w * (xk + g * (xj - xk) - xm) + xm;
-        }
-        dst[k] = xn;
-        if (s.periodic && i == 0) dst[(long long)j * n0 + n0 - 1] = xn;  // seam column
-        r = fabs(rhs - ap * xk - sum);
-    }
-    r = block_sum(r, sm);
-    if (threadIdx.x == 0) {
-        s.part[blockIdx.x] = r;
         __threadfence();
-        last = atomicAdd(s.cnt, 1u) == gridDim.x - 1;
+        atomicAdd(s.cnt, 1u);
+        got = false;
+        for (unsigned n = 0; n < kSeamPolls && !got; n++) {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(s.cnt) : "memory");
+            got = (int)(v - target) >= 0;
+        }
+        __threadfence();
+        if (!got) s.sc[SC_FAIL] = 1.0;
+    }
+    return __syncthreads_and(got);
+}
+
+template <bool MAX>
+__device__ __forceinline__ double block_fold(double v, double* sm) {
+    for (int o = 16; o > 0; o >>= 1) {
+        const double y = __shfl_down_sync(0xffffffffu, v, o);
+        v = MAX ? fmax(v, y) : v + y;
     }
     __syncthreads();
-    if (!last) return;
-    __threadfence();
-    double t = 0.0;
-    for (int m = threadIdx.x; m < (int)gridDim.x; m += blockDim.x) t += __ldcg(s.part + m);
-    t = block_sum(t, sm);
-    if (threadIdx.x == 0) {
-        *s.cnt = 0u;
-        if (sweep == 0) s.sc[SC_R0] = t != 0.0 ? t : 1.0;
-        s.sc[SC_R] = t;
-        const double s2 = ((b + a) / (b - a)) * ((b + a) / (b - a));
-        s.sc[SC_W] = sweep == 0 ? 1.0 / (1.0 - 1.0 / (2.0 * s2)) : 1.0 / (1.0 - s.sc[SC_W] / (4.0 * s2));
-        // pairs end in the caller's array; the stop is decided on the second sweep of a pair
-        if (!to_scratch && (t / s.sc[SC_R0] < tol || !isfinite(t))) s.sc[SC_DONE] = isfinite(t) ? 1.0 : 2.0;
+    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double r = sm[0];
+    for (int w = 1; w < BS / 32; w++) r = MAX ? fmax(r, sm[w]) : r + sm[w];
+    return r;  // in every thread
+}
+// fold of one value per CTA over the grid, the same bits in every CTA
+template <bool MAX>
+__device__ __forceinline__ double grid_fold(const double* part, double* sm) {
+    double v = 0.0;
+    for (int m = threadIdx.x; m < (int)gridDim.x; m += BS) v = MAX ? fmax(v, part[m]) : v + part[m];
+    return block_fold<MAX>(v, sm);
+}
+
+struct Cell {
+    int i, j;
+    int col[5];  // array column of i - 2 .. i + 2, less i (the periodic wrap without a branch)
+    long long k;
+    bool near9;
+    __device__ __forceinline__ Cell(const Sys& s, int e, int ilo, int nx) {
+        j = 1 + e / nx;
+        i = ilo + (e - (j - 1) * nx);
+        k = (long long)j * s.n0 + i;
+        near9 = j == 1 || j == s.n1 - 2 || (!s.periodic && (i == 1 || i == s.n0 - 2));
+        const int P = s.n0 - 1;
+#pragma unroll
+        for (int d = -2; d <= 2; d++) {
+            const int ii = i + d;
+            col[d + 2] = s.periodic ? (ii < 0 ? d + P : ii >= P ? d - P : d) : d;
+        }
     }
+};
+
+// sum of the off-centre couplings of `src` at the cell, in gauss()'s order; with ABS also the
+// sum of the couplings' magnitudes
+template <bool ABS>
+__device__ __forceinline__ double couplings(const Sys& s, const Cell& t, const double* src, double& off) {
+    double a[8], x[8], sum = 0.0;
+#pragma unroll
+    for (int b = 0; b < 3; b++) {  // eight at a time: their loads in flight together
+        if (b > 0 && t.near9) break;
+#pragma unroll
+        for (int m = 0; m < 8; m++) {
+            const int q = 1 + 8 * b + m;
+            a[m] = s.c[q][t.k];
+            x[m] = src[t.k + (long long)dy_of(q) * s.n0 + t.col[dx_of(q) + 2]];
+        }
+#pragma unroll
+        for (int m = 0; m < 8; m++) {
+            sum += a[m] * x[m];
+            if (ABS) off += fabs(a[m]);
+        }
+    }
+    return sum;
+}
+
+__device__ __forceinline__ void put(const Sys& s, double* dst, const Cell& t, double v) {
+    dst[t.k] = v;
+    if (s.periodic && t.i == 0) dst[(long long)t.j * s.n0 + s.n0 - 1] = v;  // seam column
+}
+
+// sweeps [first, first + nsweeps) of the solve (an even number); first == 0 also finds the bounds
+__global__ void __launch_bounds__(BS, 2) k_seam_solve(const __grid_constant__ Sys s, int first, int nsweeps, double tol) {
+    __shared__ double sm[BS / 32];
+    unsigned target = 0;
+    const int ilo = s.periodic ? 0 : 1, nx = s.n0 - 2 - ilo + 1, ncell = nx * (s.n1 - 2);
+    const int stride = gridDim.x * BS, e0 = blockIdx.x * BS + threadIdx.x;
+    double a, b, r0, w;
+    int sweep = first;
+    if (first == 0) {
+        // bounds; the first sweep's corrections xj - x into x1; its residual
+        double ap_most = 0.0, off_most = 0.0, r = 0.0;
+        for (int e = e0; e < ncell; e += stride) {
+            const Cell t(s, e, ilo, nx);
+            const double ap = s.c[0][t.k], rhs = s.q[t.k], xk = s.x0[t.k];
+            double off = 0.0;
+            const double sum = couplings<true>(s, t, s.x0, off);
+            const double xj = (rhs - sum) / ap;
+            s.x1[t.k] = xj - xk;
+            r += fabs(rhs - ap * xk - sum);
+            ap_most = fmax(ap_most, fabs(ap));
+            off_most = fmax(off_most, off / fabs(ap));
+        }
+        // boundary values of the second iterate
+        for (int e = e0; e < s.n0; e += stride) {
+            s.x1[e] = s.x0[e];
+            const long long k = (long long)(s.n1 - 1) * s.n0 + e;
+            s.x1[k] = s.x0[k];
+        }
+        if (!s.periodic)
+            for (int e = e0; e < s.n1; e += stride) {
+                const long long k = (long long)e * s.n0;
+                s.x1[k] = s.x0[k];
+                s.x1[k + s.n0 - 1] = s.x0[k + s.n0 - 1];
+            }
+        double* p = s.part;
+        ap_most = block_fold<true>(ap_most, sm);
+        off_most = block_fold<true>(off_most, sm);
+        r = block_fold<false>(r, sm);
+        const int G = gridDim.x;
+        if (threadIdx.x == 0) {
+            p[blockIdx.x] = ap_most;
+            p[G + blockIdx.x] = off_most;
+            p[2 * G + blockIdx.x] = r;
+        }
+        if (!seam_barrier(s, target)) return;
+        ap_most = grid_fold<true>(p, sm);
+        off_most = grid_fold<true>(p + G, sm);
+        r = grid_fold<false>(p + 2 * G, sm);
+        a = 0.9 / ap_most;
+        b = 1.05 * (1.0 + off_most);
+        r0 = r != 0.0 ? r : 1.0;
+        const double g = 2.0 / (a + b), s2 = ((b + a) / (b - a)) * ((b + a) / (b - a));
+        w = 1.0 / (1.0 - 1.0 / (2.0 * s2));
+        for (int e = e0; e < ncell; e += stride) {
+            const Cell t(s, e, ilo, nx);
+            put(s, s.x1, t, s.x0[t.k] + g * s.x1[t.k]);
+        }
+        if (!seam_barrier(s, target)) return;
+        sweep = 1;
+    } else {
+        a = s.sc[SC_A];
+        b = s.sc[SC_B];
+        r0 = s.sc[SC_R0];
+        w = s.sc[SC_W];
+    }
+    const double g = 2.0 / (a + b), s2 = ((b + a) / (b - a)) * ((b + a) / (b - a));
+    double done = 0.0;
+    for (; sweep < first + nsweeps; sweep++) {
+        // x_{k+1} overwrites x_{k-1}: even sweeps from the caller's array into the scratch
+        const bool to_scratch = (sweep & 1) == 0;
+        const double* src = to_scratch ? s.x0 : s.x1;
+        double* dst = to_scratch ? s.x1 : s.x0;
+        double r = 0.0, unused = 0.0;
+        for (int e = e0; e < ncell; e += stride) {
+            const Cell t(s, e, ilo, nx);
+            const double ap = s.c[0][t.k], rhs = s.q[t.k], xk = src[t.k], xm = dst[t.k];
+            const double sum = couplings<false>(s, t, src, unused);
+            const double xj = (rhs - sum) / ap;
+            put(s, dst, t, w * (xk + g * (xj - xk) - xm) + xm);
+            r += fabs(rhs - ap * xk - sum);
+        }
+        w = 1.0 / (1.0 - w / (4.0 * s2));
+        // pairs end in the caller's array; the stop is decided on the second sweep of a pair
+        double* p = s.part + ((sweep >> 1) & 1) * MAX_BLOCKS;
+        if (!to_scratch) {
+            r = block_fold<false>(r, sm);
+            if (threadIdx.x == 0) p[blockIdx.x] = r;
+        }
+        if (!seam_barrier(s, target)) return;
+        if (to_scratch) continue;
+        const double t = grid_fold<false>(p, sm);
+        if (t / r0 < tol || !isfinite(t)) {
+            done = isfinite(t) ? 1.0 : 2.0;
+            sweep++;
+            break;
+        }
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        s.sc[SC_A] = a;
+        s.sc[SC_B] = b;
+        s.sc[SC_R0] = r0;
+        s.sc[SC_W] = w;
+        s.sc[SC_DONE] = done;
+        s.sc[SC_SWEEPS] = (double)sweep;
+    }
+}
+
+// CTAs that are resident together on the current device (0: the query failed)
+int resident_blocks() {
+    static std::atomic<int> known[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    int n = known[dev].load();
+    if (n == 0) {
+        int sms = 0, per = 0;
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_seam_solve, BS, 0) != cudaSuccess)
+            return 0;
+        n = sms * per;
+        if (n > MAX_BLOCKS / 3) n = MAX_BLOCKS / 3;
+        known[dev].store(n);
+    }
+    return n;
 }
 
 }  // namespace cfd_seam
 
 void cfd_internal_set_error(const char* msg);
 
-// shared driver: `scratch` holds (8 + nblk) doubles, a second n1*n0 iterate, and a counter
+// shared driver on `scratch` (cfd_seam_scratch_doubles() doubles, 16-byte aligned)
 int cfd_seam_solve(int n0, int n1, int periodic, const double* const* coef, double* phi, const double* q,
                    double tol, int maxit, int* sweeps, void* stream, double* scratch) {
     using namespace cfd_seam;
@@ -174,41 +290,50 @@ int cfd_seam_solve(int n0, int n1, int periodic, const double* const* coef, doub
     s.n0 = n0; s.n1 = n1; s.periodic = periodic;
     for (int m = 0; m < 25; m++) s.c[m] = coef[m];
     const int nx = periodic ? n0 - 1 : n0 - 2, ny = n1 - 2;
-    const int ncell = nx * ny;
-    const int nblk = (ncell + BS - 1) / BS;
     s.sc = scratch;
+    s.cnt = reinterpret_cast<unsigned int*>(scratch + SC_CNT);
     s.part = scratch + 8;
     s.x0 = phi;
-    s.x1 = scratch + 8 + ((nblk + 31) / 32) * 32;
-    s.cnt = (unsigned int*)(s.x1 + (size_t)n0 * n1);
+    s.x1 = scratch + SCRATCH_HEAD;
     s.q = q;
-    if (cudaMemsetAsync(scratch, 0, 8 * sizeof(double), st) != cudaSuccess ||
-        cudaMemsetAsync(s.cnt, 0, sizeof(unsigned int), st) != cudaSuccess ||
-        cudaMemcpyAsync(s.x1, phi, sizeof(double) * (size_t)n0 * n1, cudaMemcpyDeviceToDevice, st) != cudaSuccess) {
+    const int most = resident_blocks();
+    if (most <= 0) {
+        cfd_internal_set_error("gauss seam: no usable device");
+        return CFD_E_CUDA;
+    }
+    const int grid = (int)std::min<long long>(most, ((long long)nx * ny + BS - 1) / BS);
+    // sweeps run in pairs (the pair ends in the caller's array), so at most maxit rounded
+    // down to even sweeps are taken; the outcome is read once per launch
+    double sc[8] = {};
+    if (cudaMemsetAsync(scratch, 0, sizeof(sc), st) != cudaSuccess) {
         cfd_internal_set_error("gauss seam: scratch initialisation failed");
         return CFD_E_CUDA;
     }
-    k_seam_bounds<<<nblk, BS, 0, st>>>(s);
     int done = 0;
-    double flag = 0.0;
-    // sweeps run in pairs (the pair ends in the caller's array), so at most maxit rounded
-    // down to even sweeps are taken
-    for (int k = 0; k + 2 <= maxit && !done; k += 2) {
-        k_seam_sweep<<<nblk, BS, 0, st>>>(s, 1, k, tol);
-        k_seam_sweep<<<nblk, BS, 0, st>>>(s, 0, k + 1, tol);
-        if (cudaMemcpyAsync(&flag, s.sc + SC_DONE, sizeof(double), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+    for (int first = 0; first + 2 <= maxit && !done; first += kSeamSweeps) {
+        int nsweeps = std::min(kSeamSweeps, (maxit - first) / 2 * 2);
+        if (first > 0 && cudaMemsetAsync(s.cnt, 0, sizeof(double), st) != cudaSuccess) {
+            cfd_internal_set_error("gauss seam: stream error");
+            return CFD_E_CUDA;
+        }
+        void* args[] = {&s, &first, &nsweeps, &tol};
+        if (cudaLaunchCooperativeKernel((const void*)k_seam_solve, dim3(grid), dim3(BS), args, 0, st) != cudaSuccess) {
+            cfd_internal_set_error("gauss seam: kernel launch failed");
+            return CFD_E_CUDA;
+        }
+        if (cudaMemcpyAsync(sc, scratch, sizeof(sc), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess) {
             cfd_internal_set_error("gauss seam: stream error");
             return CFD_E_CUDA;
         }
-        if (sweeps) *sweeps = k + 2;
-        done = flag != 0.0;
+        if (sc[SC_FAIL] != 0.0) {
+            cfd_internal_set_error("gauss seam: a bounded wait inside the kernel timed out");
+            return CFD_E_CUDA;
+        }
+        if (sweeps) *sweeps = (int)sc[SC_SWEEPS];
+        done = sc[SC_DONE] != 0.0;
     }
-    if (cudaGetLastError() != cudaSuccess) {
-        cfd_internal_set_error("gauss seam: kernel launch failed");
-        return CFD_E_CUDA;
-    }
-    if (flag == 2.0) {
+    if (sc[SC_DONE] == 2.0) {
         cfd_internal_set_error("gauss seam: residual not finite");
         return CFD_E_DIVERGED;
     }
@@ -217,10 +342,50 @@ int cfd_seam_solve(int n0, int n1, int periodic, const double* const* coef, doub
 }
 
 size_t cfd_seam_scratch_doubles(int n0, int n1, int periodic) {
-    const int nx = periodic ? n0 - 1 : n0 - 2, ny = n1 - 2;
-    const int nblk = (nx * ny + cfd_seam::BS - 1) / cfd_seam::BS;
-    return 8 + ((size_t)(nblk + 31) / 32) * 32 + (size_t)n0 * n1 + 1;
+    (void)periodic;
+    return (size_t)cfd_seam::SCRATCH_HEAD + (size_t)n0 * n1;
 }
+
+// ---- the library's scratch pool (cfd_scratch.cuh)
+namespace cfd {
+namespace {
+constexpr int kMaxDevices = 64;
+std::mutex g_pool_mu;
+cudaMemPool_t g_pool[kMaxDevices] = {};
+
+cudaMemPool_t scratch_pool() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    if (!g_pool[dev]) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t p = nullptr;
+        if (cudaMemPoolCreate(&p, &props) != cudaSuccess) return nullptr;
+        unsigned long long keep = kScratchKeep;
+        cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+        g_pool[dev] = p;
+    }
+    return g_pool[dev];
+}
+}  // namespace
+
+void* scratch_take(size_t bytes, cudaStream_t st) {
+    void* p = nullptr;
+    cudaMemPool_t pool = scratch_pool();
+    if (!pool || cudaMallocFromPoolAsync(&p, bytes, pool, st) != cudaSuccess) {
+        cudaGetLastError();  // the failure is reported by the caller
+        return nullptr;
+    }
+    return p;
+}
+
+void scratch_give(void* p, cudaStream_t st) {
+    if (p) cudaFreeAsync(p, st);
+}
+}  // namespace cfd
 
 extern "C" int cfd_gauss_solve(int n0, int n1, int periodic, const double* const* coef, double* phi,
                                const double* q, double tol, int maxit, int* sweeps, void* stream) {
@@ -233,14 +398,14 @@ extern "C" int cfd_gauss_solve(int n0, int n1, int periodic, const double* const
             cfd_internal_set_error("cfd_gauss_solve: null coefficient plane");
             return CFD_E_ARG;
         }
-    double* scratch = nullptr;
-    const size_t nd = cfd_seam_scratch_doubles(n0, n1, periodic);
-    if (cudaMalloc((void**)&scratch, nd * sizeof(double)) != cudaSuccess) {
-        cfd_internal_set_error("cfd_gauss_solve: cudaMalloc of the scratch failed");
+    double* scratch = (double*)cfd::scratch_take(cfd_seam_scratch_doubles(n0, n1, periodic) * sizeof(double),
+                                                 (cudaStream_t)stream);
+    if (!scratch) {
+        cfd_internal_set_error("cfd_gauss_solve: no device memory for the scratch");
         return CFD_E_OOM;
     }
-    int rc = cfd_seam_solve(n0, n1, periodic, coef, phi, q, tol, maxit, sweeps, stream, scratch);
-    cudaStreamSynchronize((cudaStream_t)stream);
-    cudaFree(scratch);
+    const int rc = cfd_seam_solve(n0, n1, periodic, coef, phi, q, tol, maxit, sweeps, stream, scratch);
+    if (rc == CFD_E_CUDA) cudaStreamSynchronize((cudaStream_t)stream);
+    cfd::scratch_give(scratch, (cudaStream_t)stream);
     return rc;
 }

@@ -274,9 +274,10 @@ int cfd_batch_work(cfd_batch* b, unsigned long long* out4);
  * periodic with the seam column n0-1 duplicating column 0 (the reference's O-grid);
  * 0: columns 0 and n0-1 are fixed. Chebyshev-accelerated Jacobi sweeps until the
  * relative L1 residual before a sweep is below tol (gauss()'s rule, PSolver.cpp:2438).
- * Sweeps run in pairs, the stop tested after each pair on the host (the call waits for
- * its work), so at most maxit rounded down to even sweeps are taken.
- * Scratch (a second iterate and reduction partials) is allocated and freed per call.
+ * Sweeps run in pairs, the stop tested after each pair (the call waits for its work), so
+ * at most maxit rounded down to even sweeps are taken.
+ * Scratch (a second iterate and reduction partials) comes from the library's pool, which
+ * keeps at most 256 MB per device between calls.
  * Returns CFD_OK, CFD_E_MAXITER or CFD_E_DIVERGED; *sweeps receives the sweep count. */
 int cfd_gauss_solve(int n0, int n1, int periodic, const double* const* coef, double* phi,
                     const double* q, double tol, int maxit, int* sweeps, void* stream);
