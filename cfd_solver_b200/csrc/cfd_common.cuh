@@ -30,17 +30,19 @@ constexpr int BC_THREADS = 256;
 
 enum Profile { OGRID = 0, CAVITY = 1 };
 
-// FP64 plane slots of a case
+// FP64 plane slots of a case. The stencil and the pressure solve's vectors are consecutive: the
+// sip9p() seam backs only those with memory. The preconditioned directions have no planes of
+// their own: they are read where the V-cycle leaves them.
 enum Plane {
     P_X, P_Y, P_XIX, P_XIY, P_ETX, P_ETY, P_ALPH, P_BETA, P_GAM, P_JAC,  // grid
     P_AP, P_AE, P_AW, P_AN, P_AS, P_ANE, P_ANW, P_ASE, P_ASW,            // pressure stencil
+    P_Q, P_PCOR, P_KR, P_KP, P_KV, P_KS, P_KT,                           // q, pcor, BiCGStab vectors
     P_U, P_V, P_P, P_T0, P_T1, P_UP0, P_UP1, P_VP0, P_VP1,               // state (T, up, vp double-buffered)
     P_US, P_VS,                                                          // u*, v*
     P_RU, P_RV, P_RT, P_RUP, P_RVP,                                      // right-hand sides
     P_BU, P_BV, P_BT, P_BUP, P_BVP,                                      // Jacobi scratch
-    P_Q, P_PCOR, P_VORT, P_SI, P_DIL,                                    // q, pcor, diagnostics
+    P_VORT, P_SI, P_DIL,                                                 // diagnostics
     P_VEC,    // rows 0..3: normals xnix, xniy, xnox, xnoy (one value per column)
-    P_KR, P_KRH, P_KP, P_KV, P_KS, P_KT, P_KPH, P_KSH,                   // BiCGStab vectors
     NPLANES
 };
 

@@ -377,11 +377,9 @@ __global__ void __launch_bounds__(NT, 5) k_spmv(BatchDev b, int mode) {
     for (int h = 0; h < 2; h++) {
         if (!in[h]) continue;
         if (mode == 0) {
-            plane(b, c, P_KPH)[k[h]] = xc[h];
             plane(b, c, P_KV)[k[h]] = y[h];
             red[0] += dv[h] * y[h];
         } else {
-            plane(b, c, P_KSH)[k[h]] = xc[h];
             plane(b, c, P_KT)[k[h]] = y[h];
             red[0] += y[h] * dv[h];
             red[1] += y[h] * y[h];
@@ -415,8 +413,9 @@ __global__ void __launch_bounds__(NT, 5) k_bicg_s(BatchDev b) {
     const int i = t.i0 + (int)(threadIdx.x % TX), j0 = t.j0 + (int)(threadIdx.x / TX);
     const double alpha = b.scal[(long long)t.c * NSCAL + S_ALPHA];
     double* X = plane(b, c, P_PCOR);
-    const double *R = plane(b, c, P_KR), *Vv = plane(b, c, P_KV), *PH = plane(b, c, P_KPH);
+    const double *R = plane(b, c, P_KR), *Vv = plane(b, c, P_KV);
     const LevelDev& L = c.lev[0];
+    const float* PH = mplane(b, L, mg_result_plane(b, c, 0));  // p_hat, as the V-cycle left it
     bool in[2];
     long long k[2];
     double x0[2], r[2], v[2], ph[2];
@@ -428,7 +427,7 @@ __global__ void __launch_bounds__(NT, 5) k_bicg_s(BatchDev b) {
         x0[h] = first ? 0.0 : X[k[h]];
         r[h] = R[k[h]];
         v[h] = Vv[k[h]];
-        ph[h] = PH[k[h]];
+        ph[h] = (double)PH[in[h] ? (long long)j * L.ld + i : (long long)L.ld + c.ilo];
     }
     double red[1] = {0.0};
 #pragma unroll
@@ -465,7 +464,9 @@ __global__ void __launch_bounds__(NT, 5) k_bicg_x(BatchDev b, int maxit) {
     const double alpha = sc0[S_ALPHA], omega = sc0[S_OMEGA];
     const int ld = c.ld;
     double* X = plane(b, c, P_PCOR);
-    const double *SH = plane(b, c, P_KSH), *S = plane(b, c, P_KS), *T = plane(b, c, P_KT), *Q = plane(b, c, P_Q);
+    const LevelDev& L = c.lev[0];
+    const float* SH = mplane(b, L, mg_result_plane(b, c, 0));  // s_hat, as the V-cycle left it
+    const double *S = plane(b, c, P_KS), *T = plane(b, c, P_KT), *Q = plane(b, c, P_Q);
     bool in[2];
     long long k[2];
     double x0[2], sh[2], s[2], tt[2], q[2];
@@ -475,7 +476,7 @@ __global__ void __launch_bounds__(NT, 5) k_bicg_x(BatchDev b, int maxit) {
         in[h] = i >= c.ilo && i <= c.ihi && j <= c.n1 - 2;
         k[h] = in[h] ? (long long)j * ld + i : (long long)ld + c.ilo;
         x0[h] = X[k[h]];
-        sh[h] = SH[k[h]];
+        sh[h] = (double)SH[in[h] ? (long long)j * L.ld + i : (long long)L.ld + c.ilo];
         s[h] = S[k[h]];
         tt[h] = T[k[h]];
         q[h] = Q[k[h]];

@@ -779,6 +779,43 @@ __device__ __forceinline__ void mg_gs_tile(const BatchDev& b, const CaseDev& c, 
 // of more than one unknown per thread used before, each pass paid L2 round trips instead: five
 // steps of a 181 x 91 O-grid (90 x 44 unknowns on its coarsest level) took 5.75 ms, with the
 // stencils in registers 2.68.
+//
+// mg_coarse_small: a level with no more unknowns than threads, one each (less set-up: 30
+// against 38 us per step of the 256-case sweep).
+template <class Grp>
+__device__ __forceinline__ void mg_coarse_small(const BatchDev& b, const CaseDev& c, const LevelDev& L, int sweeps,
+                                                float* xs, const Grp& g) {
+    const int ld = L.ld, per = c.periodic, W = L.W;
+    const int nx = L.ihi - L.ilo + 1, n = nx * (L.n1 - 2);
+    const int ncol = (per && (W & 1)) ? 6 : 4;
+    const int sw = W + 2 * H;
+    for (int e = g.tid; e < L.n1 * sw; e += Grp::N) xs[e] = 0.0f;  // x = 0 (and boundaries)
+    const bool in = g.tid < n;
+    const int i = L.ilo + (in ? g.tid % nx : 0), j = 1 + (in ? g.tid / nx : 0);
+    const long long p = (long long)j * ld + i;
+    float f[9];
+#pragma unroll
+    for (int m = 0; m < 9; m++) f[m] = mplane(b, L, M_AP + m)[p];
+    const float rhs = mplane(b, L, M_B)[p], rd = __frcp_rn(f[0]);
+    const int col = in ? mg_colour(i, j, W, per) : -1;
+    const int m = mirror_col(i, W, per);
+    float* x = xs + j * sw + i + H;
+    g.sync();
+    for (int s = 0; s < sweeps; s++) {
+        for (int cc = 0; cc < ncol; cc++) {
+            if (col == cc) {
+                const float sm = f[1] * x[1] + f[2] * x[-1] + f[3] * x[sw] + f[4] * x[-sw] + f[5] * x[sw + 1] +
+                                 f[6] * x[sw - 1] + f[7] * x[-sw + 1] + f[8] * x[-sw - 1];
+                const float v = mg_div(rhs - sm, f[0], rd);
+                x[0] = v;
+                if (m > -1000000) xs[j * sw + m + H] = v;
+            }
+            g.sync();
+        }
+    }
+    if (in) store_mirrored(mplane(b, L, M_X), ld, i, j, W, per, x[0]);
+}
+
 struct MgColour {
     int fi, fj, nx, n;  // first column and row, points in a row, points
     __device__ __forceinline__ MgColour(const LevelDev& L, int per, int cc) {
@@ -897,6 +934,7 @@ __device__ __forceinline__ void mg_coarse_solve(const BatchDev& b, const CaseDev
     // column parities the most
     const int most = max(MgColour(L, c.periodic, 2).n, MgColour(L, c.periodic, 3).n);
     if (most > KMAX * Grp::N || L.n1 * (L.W + 2 * H) > xs_cap) mg_coarse_global(b, c, L, sweeps, g);
+    else if ((L.ihi - L.ilo + 1) * (L.n1 - 2) <= Grp::N) mg_coarse_small(b, c, L, sweeps, xs, g);
     else if (KMAX == 1 || most <= Grp::N) mg_coarse_regs<1>(b, c, L, sweeps, xs, g);
     else mg_coarse_regs<KMAX>(b, c, L, sweeps, xs, g);
 }
