@@ -612,65 +612,14 @@ __global__ void __launch_bounds__(MGC_THREADS) k_mg_coarse(BatchDev b, int l, in
     mg_coarse_solve<1>(b, c, c.lev[l >= 0 ? l : c.nlev - 1], sweeps, xs, MGC_SMEM, BlockGroup<MGC_THREADS>());
 }
 
-// Galerkin coarse operator A_{l+1} = R A_l P (R full weighting, P bilinear, R = P^T / 4)
-__device__ __forceinline__ bool lev_unknown(const LevelDev& L, int periodic, int i, int j) {
-    if (j < 1 || j > L.n1 - 2) return false;
-    if (periodic) return true;
-    return i >= L.ilo && i <= L.ihi;
-}
-
+// Galerkin coarse operator of level l + 1 (mg_galerkin_point): one thread per coarse point
 __global__ void __launch_bounds__(NT) k_mg_galerkin(BatchDev b, int l, int toff) {
     const Tile t = b.atiles[l + 1][toff + blockIdx.x];
     const CaseDev& c = b.cases[t.c];
-    const LevelDev& F = c.lev[l];
     const LevelDev& C = c.lev[l + 1];
     const int I = t.i0 + (int)(threadIdx.x % TX), J = t.j0 + (int)(threadIdx.x / TX);
     if (I < C.ilo || I > C.ihi || J > C.n1 - 2) return;
-    const int per = c.periodic;
-    const int fl = F.ld;
-    const float* fa[9];
-#pragma unroll
-    for (int m = 0; m < 9; m++) fa[m] = mplane(b, F, M_AP + m);
-    // stencil offsets in M_AP.. order: p, e, w, n, s, ne, nw, se, sw
-    const int ox[9] = {0, 1, -1, 0, 0, 1, -1, 1, -1};
-    const int oy[9] = {0, 0, 0, 1, -1, 1, 1, -1, -1};
-    double acc[9];  // indexed (dy + 1) * 3 + (dx + 1)
-#pragma unroll
-    for (int m = 0; m < 9; m++) acc[m] = 0.0;
-    for (int bj = -1; bj <= 1; bj++) {
-        for (int bi = -1; bi <= 1; bi++) {
-            const int fi = 2 * I + bi, fj = 2 * J + bj;
-            if (!lev_unknown(F, per, fi, fj)) continue;
-            const double wr = 0.25 * (bi == 0 ? 1.0 : 0.5) * (bj == 0 ? 1.0 : 0.5);
-            const long long kf = (long long)fj * fl + fi;
-            for (int m = 0; m < 9; m++) {
-                const int gi = fi + ox[m], gj = fj + oy[m];
-                if (!lev_unknown(F, per, gi, gj)) continue;
-                const double a = wr * (double)fa[m][kf];
-                // coarse parents of fine point (gi, gj)
-                int pi[2], pj[2];
-                double wi[2], wj[2];
-                int ni, nj;
-                if (!(gi & 1)) { pi[0] = gi >> 1; wi[0] = 1.0; ni = 1; }
-                else { pi[0] = (gi - 1) >> 1; pi[1] = (gi + 1) >> 1; wi[0] = wi[1] = 0.5; ni = 2; }
-                if (!(gj & 1)) { pj[0] = gj >> 1; wj[0] = 1.0; nj = 1; }
-                else { pj[0] = (gj - 1) >> 1; pj[1] = (gj + 1) >> 1; wj[0] = wj[1] = 0.5; nj = 2; }
-                for (int x = 0; x < ni; x++) {
-                    for (int y = 0; y < nj; y++) {
-                        if (!lev_unknown(C, per, pi[x], pj[y])) continue;
-                        const int dx = pi[x] - I, dy = pj[y] - J;
-                        acc[(dy + 1) * 3 + (dx + 1)] += a * wi[x] * wj[y];
-                    }
-                }
-            }
-        }
-    }
-    const long long kc = (long long)J * C.ld + I;
-    const int idx[9] = {4, 5, 3, 7, 1, 8, 6, 2, 0};  // p, e, w, n, s, ne, nw, se, sw
-#pragma unroll
-    for (int m = 0; m < 9; m++)
-        store_mirrored(mplane(b, C, M_AP + m), C.ld, I, J, C.W, per, (float)acc[idx[m]]);
-    (void)kc;
+    mg_galerkin_point(b, c, l, I, J);
 }
 
 // ---------------------------------------------------------------------------
@@ -956,110 +905,6 @@ __global__ void __launch_bounds__(256) k_state_pack(BatchDev b, double* stage, c
             for (int i = lane; i < nc; i += 32) store_mirrored(row, 0, i, 0, d.W, d.periodic, srow[i]);
         }
     }
-}
-
-}  // namespace cfd
-
-// ---------------------------------------------------------------------------
-// The sip9p() seam (cfd_sip_solve, PSolver.cpp:2067-2278): a one-case batch whose pressure
-// stencil is the caller's nine stored planes instead of the grid's. The solve is the step's
-// own BiCGStab + multigrid, run on the correction e of A (phi0 + e) = q with e = 0 on the
-// boundary rows (and, without periodic xi, the boundary columns), as sip9p holds them.
-namespace cfd {
-
-// caller's [j][i] arrays -> case 0's padded planes: the stencil on the unknown cells (zero
-// elsewhere, as k_assemble_p leaves it) in FP64 and as multigrid level 0, phi0 into P_SI and
-// q into P_VORT at every stored point; a periodic case's halo columns take the wrap
-__global__ void k_sip_pack(BatchDev b, SipIn in) {
-    const CaseDev& c = b.cases[0];
-    const int W = c.W, per = c.periodic;
-    const int ncols = W + 2 * H;  // padded columns -H .. W + H - 1
-    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (long long)c.n1 * ncols) return;
-    const int j = (int)(e / ncols), col = (int)(e % ncols) - H;
-    int i = col;  // the caller's column
-    if (per) i = col < 0 ? col + W : (col >= W ? col - W : col);
-    else if (col < 0 || col >= c.n0) return;
-    const long long src = (long long)j * in.n0 + i;
-    const long long k = (long long)j * c.ld + col;
-    const bool unknown = j >= 1 && j <= c.n1 - 2 && i >= c.ilo && i <= c.ihi;
-    const LevelDev& L0 = c.lev[0];
-    const long long k0 = (long long)j * L0.ld + col;
-#pragma unroll
-    for (int q = 0; q < 9; q++) {
-        const double v = unknown ? in.a[q][src] : 0.0;
-        plane(b, c, P_AP + q)[k] = v;
-        mplane(b, L0, M_AP + q)[k0] = (float)v;
-    }
-    plane(b, c, P_SI)[k] = in.phi[src];
-    plane(b, c, P_VORT)[k] = in.q[src];
-}
-
-// r0 = q - A phi0 on the unknown cells (phi0's boundary values enter through the stencil),
-// then the pressure solve's start as k_face_q leaves it for a step: r0 is the right-hand
-// side, the shadow residual and the first preconditioner input; the iterate starts at zero
-__global__ void __launch_bounds__(NT) k_sip_init(BatchDev b) {
-    const Tile t = b.jtiles[blockIdx.x];
-    const CaseDev& c = b.cases[t.c];
-    const int tid = threadIdx.x, li = tid % TX, lj = tid / TX, i = t.i0 + li;
-    const int ld = c.ld;
-    const double* X = plane(b, c, P_SI);
-    const double* Q = plane(b, c, P_VORT);
-    const LevelDev& L0 = c.lev[0];
-    double red[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        const int j = t.j0 + lj + h * TY;
-        if (i < c.ilo || i > c.ihi || j > c.n1 - 2) continue;
-        const long long k = (long long)j * ld + i;
-        const double ax = plane(b, c, P_AP)[k] * X[k] + plane(b, c, P_AE)[k] * X[k + 1] +
-                          plane(b, c, P_AW)[k] * X[k - 1] + plane(b, c, P_AN)[k] * X[k + ld] +
-                          plane(b, c, P_AS)[k] * X[k - ld] + plane(b, c, P_ANE)[k] * X[k + ld + 1] +
-                          plane(b, c, P_ANW)[k] * X[k + ld - 1] + plane(b, c, P_ASE)[k] * X[k - ld + 1] +
-                          plane(b, c, P_ASW)[k] * X[k - ld - 1];
-        const double r = Q[k] - ax;
-        plane(b, c, P_Q)[k] = r;
-        plane(b, c, P_KR)[k] = r;
-        mplane(b, L0, M_B)[(long long)j * L0.ld + i] = (float)r;
-        red[0] += fabs(r);
-        red[1] += r * r;
-        red[2] = fmax(red[2], fabs(r));
-    }
-    if (case_reduce<3, 0x4u>(b, t.c, blockIdx.x, c.jt_begin, c.jt_count, red) && tid == 0) {
-        double* sc = b.scal + (long long)t.c * NSCAL;
-        int* is = b.iscal + (long long)t.c * NISCAL;
-        sc[S_QL1] = red[0];
-        sc[S_QL2] = sqrt(red[1]);
-        sc[S_QMAX] = red[2];
-        sc[S_RHO] = red[1];
-        sc[S_ALPHA] = 1.0;
-        sc[S_OMEGA] = 1.0;
-        sc[S_BETA] = 0.0;
-        sc[S_NB1] = red[0];
-        sc[S_RL1] = red[0];
-        is[I_PIT] = 0;
-        is[I_PSTATUS] = 0;
-        if (red[0] == 0.0 || !isfinite(red[0])) {
-            is[I_PDONE] = 1;
-            if (!isfinite(red[0])) is[I_STATUS] |= ST_NAN;
-        } else {
-            is[I_PDONE] = 0;
-            atomicAdd(b.active, 1);
-        }
-    }
-}
-
-// phi = phi0 + e on the unknown cells of the caller's [j][i] array (a periodic case's seam
-// column n0 - 1 repeats column 0); boundary values are left as the caller gave them
-__global__ void k_sip_out(BatchDev b, double* phi, int n0) {
-    const CaseDev& c = b.cases[0];
-    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (long long)c.n1 * n0) return;
-    const int j = (int)(e / n0), i = (int)(e % n0);
-    const int col = (c.periodic && i == n0 - 1) ? 0 : i;
-    if (j < 1 || j > c.n1 - 2 || col < c.ilo || col > c.ihi) return;
-    const long long k = (long long)j * c.ld + col;
-    phi[e] = plane(b, c, P_SI)[k] + plane(b, c, P_PCOR)[k];
 }
 
 }  // namespace cfd

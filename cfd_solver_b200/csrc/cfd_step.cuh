@@ -769,6 +769,63 @@ __device__ __forceinline__ void mg_gs_tile(const BatchDev& b, const CaseDev& c, 
         }
 }
 
+// Galerkin coarse operator A_{l+1} = R A_l P at coarse point (I, J) (R full weighting, P
+// bilinear, R = P^T / 4). Which coarse points a coupling reaches and with what weight depends
+// only on the offsets, so the unrolled sums run over fixed registers; what is tested at run
+// time is whether a point is an unknown.
+__device__ __forceinline__ bool lev_unknown(const LevelDev& L, int periodic, int i, int j) {
+    if (j < 1 || j > L.n1 - 2) return false;
+    if (periodic) return true;
+    return i >= L.ilo && i <= L.ihi;
+}
+__device__ __forceinline__ void mg_galerkin_point(const BatchDev& b, const CaseDev& c, int l, int I, int J) {
+    const LevelDev& F = c.lev[l];
+    const LevelDev& C = c.lev[l + 1];
+    const int per = c.periodic, fl = F.ld;
+    const float* A = mplane(b, F, M_AP);
+    // stencil offsets in M_AP.. order: p, e, w, n, s, ne, nw, se, sw
+    constexpr int ox[9] = {0, 1, -1, 0, 0, 1, -1, 1, -1};
+    constexpr int oy[9] = {0, 0, 0, 1, -1, 1, 1, -1, -1};
+    bool cu[3][3];  // coarse points around (I, J) that are unknowns
+#pragma unroll
+    for (int y = 0; y < 3; y++)
+#pragma unroll
+        for (int x = 0; x < 3; x++) cu[y][x] = lev_unknown(C, per, I + x - 1, J + y - 1);
+    double acc[9];  // indexed (dy + 1) * 3 + (dx + 1)
+#pragma unroll
+    for (int m = 0; m < 9; m++) acc[m] = 0.0;
+#pragma unroll
+    for (int bj = -1; bj <= 1; bj++) {
+#pragma unroll
+        for (int bi = -1; bi <= 1; bi++) {
+            const int fi = 2 * I + bi, fj = 2 * J + bj;
+            if (!lev_unknown(F, per, fi, fj)) continue;
+            const double wr = 0.25 * (bi == 0 ? 1.0 : 0.5) * (bj == 0 ? 1.0 : 0.5);
+            const long long kf = (long long)fj * fl + fi;
+#pragma unroll
+            for (int m = 0; m < 9; m++) {
+                const int sx = bi + ox[m], sy = bj + oy[m];  // fine point 2 (I, J) + (sx, sy)
+                if (!lev_unknown(F, per, 2 * I + sx, 2 * J + sy)) continue;
+                const double a = wr * (double)A[m * F.ps + kf];
+                // its coarse parents: one along an even direction, two along an odd one
+                const int nx = (sx & 1) ? 2 : 1, ny = (sy & 1) ? 2 : 1;
+                const int px = (sx & 1) ? (sx - 1) / 2 : sx / 2, py = (sy & 1) ? (sy - 1) / 2 : sy / 2;
+#pragma unroll
+                for (int x = 0; x < 2; x++)
+#pragma unroll
+                    for (int y = 0; y < 2; y++) {
+                        if (x >= nx || y >= ny || !cu[py + y + 1][px + x + 1]) continue;
+                        acc[(py + y + 1) * 3 + px + x + 1] += a * (nx == 2 ? 0.5 : 1.0) * (ny == 2 ? 0.5 : 1.0);
+                    }
+            }
+        }
+    }
+    constexpr int idx[9] = {4, 5, 3, 7, 1, 8, 6, 2, 0};  // p, e, w, n, s, ne, nw, se, sw
+#pragma unroll
+    for (int m = 0; m < 9; m++)
+        store_mirrored(mplane(b, C, M_AP + m), C.ld, I, J, C.W, per, (float)acc[idx[m]]);
+}
+
 // Coarsest level: `sweeps` multicolour Gauss-Seidel sweeps by one group, x in shared memory
 // (all rows, columns -H .. W+H-1). A thread holds the stencils of up to K points of each of the
 // four parity colours in registers, so that every pass keeps all lanes busy; the last column

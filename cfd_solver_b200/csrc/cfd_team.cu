@@ -525,7 +525,7 @@ __device__ __noinline__ void team_face(int nxt) {
     }
 }
 
-__device__ __noinline__ void team_face_total() {
+__device__ __noinline__ void team_face_total() {  // also the sip seam's start: its `mask` is 0
     TeamState& ts = sh().ts;
     double v[3];
     team_total<3, 0x4u>(part(2), cell_tiles().n, NT, v);
@@ -546,6 +546,14 @@ __device__ __noinline__ void team_face_total() {
         if (!isfinite(v[0])) ts.status |= ST_NAN;
     }
     __syncthreads();
+}
+
+// first level whose pre-smoothing has few regions: from there one CTA runs the V-cycle
+__device__ __forceinline__ int team_tail(const CaseDev& c) {
+    int tail = 0;
+    for (int l = 0; l + 1 < c.nlev; l++)
+        if (Tiling(c.lev[l + 1].ihi, c.lev[l + 1].n1, TY).n > TAIL_TILES) tail = l + 1;
+    return tail;
 }
 
 // ---- one V-cycle from M_B of level 0 into its result plane (form 2 of run_vcycle)
@@ -780,7 +788,7 @@ __device__ __noinline__ void team_bicg_p() {
 __device__ __noinline__ bool team_pressure() {
     TeamState& ts = sh().ts;
     const CaseDev& c = sh().c;
-    for (int it = 0; it < sh().a.maxit_p && !ts.pdone; it++) {
+    for (int it = 0; it < sh().a.p_iters && !ts.pdone; it++) {
         if (!team_vcycle()) return false;
         team_spmv(0);
         TEAM_SYNC();
@@ -1156,11 +1164,7 @@ __device__ __forceinline__ void team_run(const TeamArgs& a) {
     }
     if (tid == 0) {
         s.fb = b.f64 + c.base + H;
-        // first level whose pre-smoothing has few regions: from there one CTA runs the V-cycle
-        int tail = 0;
-        for (int l = 0; l + 1 < c.nlev; l++)
-            if (Tiling(c.lev[l + 1].ihi, c.lev[l + 1].n1, TY).n > TAIL_TILES) tail = l + 1;
-        s.tail = tail;
+        s.tail = team_tail(c);
     }
     __syncthreads();
     int cur = b.cur;
@@ -1201,12 +1205,141 @@ __device__ __forceinline__ void team_run(const TeamArgs& a) {
         for (int k = 0; k < 4; k++) atomicAdd(&b.work[k], ts.work[k]);
     }
 }
+
+// ---- the sip9p() seam (cfd_sip_solve, PSolver.cpp:2067-2278): the step's pressure solve on the
+// caller's stencil, for the correction e of A (phi0 + e) = q with e = 0 on the boundary rows
+// (and, without periodic xi, the boundary columns), as sip9p holds them.
+//
+// One pass over the unknown cells: the caller's stencil into the case's planes and multigrid
+// level 0, r0 = q - A phi0 (phi0's boundary values enter through the stencil) as right-hand
+// side, shadow residual and first preconditioner input, and its sums; the V-cycle's x planes
+// start from zero
+__device__ __noinline__ void sip_start(const SipArgs& p) {
+    const CaseDev& c = sh().c;
+    const Tiling jt = cell_tiles();
+    const NamedGroup<256> g;
+    const LevelDev& L0 = c.lev[0];
+    double* const fb = sh().fb;
+    const int n0 = c.n0, nr = sh().a.nr, W = c.W;
+    for (int l = 0; l < c.nlev; l++) {
+        const LevelDev& L = c.lev[l];
+        for (int q = 0; q < 2; q++) {
+            float* x = mplane(sh().a.b, L, q == 0 ? M_X : M_R) - H;
+            const long long n = (long long)L.n1 * L.ld;
+            for (long long e = (long long)sh().rank * NT5 + threadIdx.x; e < n; e += (long long)nr * NT5) x[e] = 0.0f;
+        }
+    }
+    for (int t = g.id * nr + sh().rank; t < jt.n; t += 2 * nr) {
+        const int i = jt.i0(t) + g.tid % TX, j0 = jt.j0(t, TYJ) + g.tid / TX;
+        double r[3] = {0.0, 0.0, 0.0};
+#pragma unroll 1
+        for (int h = 0; h < 2; h++) {
+            const int j = j0 + h * TY;
+            if (i < c.ilo || i > c.ihi || j > c.n1 - 2) continue;
+            const long long k = (long long)j * c.ld + i, s = (long long)j * n0 + i;
+            // the caller's columns to both sides (column n0 - 1 of a periodic array repeats column 0)
+            const int e = c.periodic && i + 1 == W ? 1 - W : 1, w = c.periodic && i == 0 ? W - 1 : -1;
+            const double* X = p.phi + s;
+            double a[9];
+#pragma unroll
+            for (int q = 0; q < 9; q++) a[q] = p.a[q][s];
+            const double ax = a[0] * X[0] + a[1] * X[e] + a[2] * X[w] + a[3] * X[n0] + a[4] * X[-n0] + a[5] * X[n0 + e] +
+                              a[6] * X[n0 + w] + a[7] * X[-n0 + e] + a[8] * X[-n0 + w];
+            const double res = p.q[s] - ax;
+#pragma unroll
+            for (int q = 0; q < 9; q++) {
+                fb[(P_AP + q) * c.ps + k] = a[q];
+                store_mirrored(mplane(sh().a.b, L0, M_AP + q), L0.ld, i, j, W, c.periodic, (float)a[q]);
+            }
+            fb[P_Q * c.ps + k] = res;
+            fb[P_KR * c.ps + k] = res;
+            mplane(sh().a.b, L0, M_B)[(long long)j * L0.ld + i] = (float)res;
+            r[0] += fabs(res);
+            r[1] += res * res;
+            r[2] = fmax(r[2], fabs(res));
+        }
+        group_reduce<3, 0x4u>(r, sh().red + g.id * 256, g);
+        if (g.tid == 0)
+            for (int q = 0; q < 3; q++) part(2)[(long long)t * PSTRIDE + q] = r[q];
+    }
+}
+
+__device__ __noinline__ void sip_galerkin(int l) {
+    const CaseDev& c = sh().c;
+    const LevelDev& C = c.lev[l + 1];
+    const int nx = C.ihi - C.ilo + 1, n = nx * (C.n1 - 2);
+    for (int e = sh().rank * NT5 + threadIdx.x; e < n; e += sh().a.nr * NT5)
+        mg_galerkin_point(sh().a.b, c, l, C.ilo + e % nx, 1 + e / nx);
+}
+
+// phi = phi0 + e on the unknown cells (the seam column repeats column 0)
+__device__ __noinline__ void sip_out(const SipArgs& p) {
+    const CaseDev& c = sh().c;
+    const int nx = c.ihi - c.ilo + 1, n = nx * (c.n1 - 2);
+    const double* E = sh().fb + P_PCOR * c.ps;
+    if (sh().ts.pit == 0) return;  // no iteration ran: e = 0
+    for (int q = sh().rank * NT5 + threadIdx.x; q < n; q += sh().a.nr * NT5) {
+        const int i = c.ilo + q % nx, j = 1 + q / nx;
+        double* x = p.phi + (long long)j * c.n0 + i;
+        const double v = *x + E[(long long)j * c.ld + i];
+        *x = v;
+        if (c.periodic && i == 0) x[c.n0 - 1] = v;
+    }
+}
+
+__device__ __forceinline__ bool sip_run(const SipArgs& p) {
+    TeamSh& s = sh();
+    const int tid = threadIdx.x;
+    for (int k = tid; k < (int)(sizeof(TeamArgs) / 4); k += NT5)
+        reinterpret_cast<int*>(&s.a)[k] = reinterpret_cast<const int*>(&p.t)[k];
+    for (int k = tid; k < (int)(sizeof(CaseDev) / 4); k += NT5)
+        reinterpret_cast<int*>(&s.c)[k] = reinterpret_cast<const int*>(&p.c)[k];
+    static_assert(sizeof(TeamState) <= kSipStateBytes && sizeof(TeamState) % 4 == 0, "state between launches");
+    for (int k = tid; k < (int)(sizeof(TeamState) / 4); k += NT5)
+        reinterpret_cast<int*>(&s.ts)[k] = p.first ? 0 : reinterpret_cast<const int*>(p.state)[k];
+    if (tid == 0) {
+        s.rank = blockIdx.x;
+        s.bar = p.t.bar;
+        s.target = 0;
+        s.fb = p.t.b.f64 + p.c.base + H;
+        s.tail = team_tail(p.c);
+    }
+    __syncthreads();
+    if (p.first) {
+        sip_start(p);
+        TEAM_SYNC();
+        for (int l = 0; l + 1 < s.c.nlev; l++) {
+            sip_galerkin(l);
+            TEAM_SYNC();
+        }
+        team_face_total();
+    }
+    if (!team_pressure()) return false;
+    const bool over = s.ts.pdone || s.ts.pit >= p.t.maxit_p;
+    if (over) sip_out(p);
+    TEAM_SYNC();
+    if (blockIdx.x == 0) {
+        for (int k = tid; k < (int)(sizeof(TeamState) / 4); k += NT5)
+            reinterpret_cast<int*>(p.state)[k] = reinterpret_cast<const int*>(&s.ts)[k];
+        if (tid == 0) {
+            p.out[0] = over;
+            p.out[1] = s.ts.pit;
+            p.out[2] = s.ts.status;
+            p.out[3] = s.ts.pstatus;
+        }
+    }
+    return true;
+}
 #undef TEAM_SYNC
 
 }  // namespace
 
 __global__ void __launch_bounds__(TEAM_THREADS, 1) k_team_f64(const __grid_constant__ TeamArgs a) { team_run<false>(a); }
 __global__ void __launch_bounds__(TEAM_THREADS, 1) k_team_mx(const __grid_constant__ TeamArgs a) { team_run<true>(a); }
+
+__global__ void __launch_bounds__(TEAM_THREADS, 1) k_team_sip(const __grid_constant__ SipArgs p) { sip_run(p); }
+
+size_t sip_smem() { return (size_t)WORK_OFF + WORK_MIN; }
 
 size_t team_smem(int max_W) {
     const size_t rows = 4 * (size_t)(max_W + 1) * sizeof(double);  // the far field's rows

@@ -291,8 +291,8 @@ int cfd_gauss_solve(int n0, int n1, int periodic, const double* const* coef, dou
  * column n0-1 duplicating column 0. BiCGStab preconditioned by a Galerkin multigrid V-cycle
  * built from the given planes (replacing the SIP iteration, which has no parallel form)
  * until the L1 residual is below tol times the initial one (sip9p's rule,
- * PSolver.cpp:2259). The call allocates a one-case batch for the solve (device memory of
- * about cfd_case_bytes(n0, n1, profile)), waits for `stream` before it starts, and returns
+ * PSolver.cpp:2259). The work runs on `stream`; its scratch (about 190 bytes per point) comes
+ * from the library's pool, which keeps at most 256 MB per device between calls. Returns
  * once phi is written. Returns CFD_OK, CFD_E_MAXITER, CFD_E_BREAKDOWN or CFD_E_DIVERGED;
  * *iters receives the BiCGStab iterations. */
 int cfd_sip_solve(int n0, int n1, int periodic, const double* const* coef9, double* phi,
