@@ -264,41 +264,38 @@ __device__ __forceinline__ void rhs_seed(double* fb, long long ps, int nextm, in
 // FP64 plane of field f's iterate for state parity nxt (u*, v*, T, up, vp)
 __device__ __forceinline__ int sw_iter_plane(int f, int nxt) { return f < 2 ? P_US + f : P_T0 + 2 * (f - 2) + nxt; }
 
-// off-centre sums of the u-type operator for the cell whose window centre row is `r0 + 2`:
-// the 25-point (4th-order) rows and the 9-point near-wall rows
-#define WX(dy, dx) w[r0 + 2 + (dy)][2 + (dx)]
-template <typename ST>
-__device__ __forceinline__ ST sw_sum25(const ST (&w)[8][5], int r0, ST E, ST G, ST B) {
-    const ST ex = ST(-4.0 / 3.0) * (WX(0, 1) + WX(0, -1)) + ST(1.0 / 12.0) * (WX(0, 2) + WX(0, -2));
-    const ST gy = ST(-4.0 / 3.0) * (WX(1, 0) + WX(-1, 0)) + ST(1.0 / 12.0) * (WX(2, 0) + WX(-2, 0));
-    const ST bx = ST(8.0 / 9.0) * (WX(1, 1) + WX(-1, -1) - WX(1, -1) - WX(-1, 1)) +
-                  ST(1.0 / 72.0) * (WX(2, 2) + WX(-2, -2) - WX(2, -2) - WX(-2, 2)) +
-                  ST(1.0 / 9.0) * (WX(2, -1) + WX(-2, 1) + WX(1, -2) + WX(-1, 2) - WX(2, 1) - WX(-2, -1) -
-                                   WX(1, 2) - WX(-1, -2));
+// Off-centre sums of the u-type operator at a cell, x(dy, dx) giving the values around it: the
+// 25-point (4th-order) rows and the 9-point near-wall rows.
+template <typename ST, class X>
+__device__ __forceinline__ ST sw_sum25(const X& x, ST E, ST G, ST B) {
+    const ST ex = ST(-4.0 / 3.0) * (x(0, 1) + x(0, -1)) + ST(1.0 / 12.0) * (x(0, 2) + x(0, -2));
+    const ST gy = ST(-4.0 / 3.0) * (x(1, 0) + x(-1, 0)) + ST(1.0 / 12.0) * (x(2, 0) + x(-2, 0));
+    const ST bx = ST(8.0 / 9.0) * (x(1, 1) + x(-1, -1) - x(1, -1) - x(-1, 1)) +
+                  ST(1.0 / 72.0) * (x(2, 2) + x(-2, -2) - x(2, -2) - x(-2, 2)) +
+                  ST(1.0 / 9.0) * (x(2, -1) + x(-2, 1) + x(1, -2) + x(-1, 2) - x(2, 1) - x(-2, -1) - x(1, 2) - x(-1, -2));
     return E * ex + G * gy + B * bx;
 }
-template <typename ST>
-__device__ __forceinline__ ST sw_sum9(const ST (&w)[8][5], int r0, ST E, ST G, ST B, bool drop_s, bool drop_n) {
-    ST s = -E * (WX(0, 1) + WX(0, -1));
-    const ST n = -G * WX(1, 0) + ST(0.5) * B * (WX(1, 1) - WX(1, -1));
-    const ST so = -G * WX(-1, 0) + ST(0.5) * B * (WX(-1, -1) - WX(-1, 1));
+template <typename ST, class X>
+__device__ __forceinline__ ST sw_sum9(const X& x, ST E, ST G, ST B, bool drop_s, bool drop_n) {
+    ST s = -E * (x(0, 1) + x(0, -1));
+    const ST n = -G * x(1, 0) + ST(0.5) * B * (x(1, 1) - x(1, -1));
+    const ST so = -G * x(-1, 0) + ST(0.5) * B * (x(-1, -1) - x(-1, 1));
     if (!drop_n) s += n;
     if (!drop_s) s += so;
     return s;
 }
-#undef WX
 
-// residual of one cell (row q of the window) for operator E, G, B; `scale` is 1/Pr for T
-template <typename ST>
-__device__ __forceinline__ ST sw_residual(const ST (&w)[8][5], int q, ST E, ST G, ST B, bool nearw, bool drop_s,
-                                          bool drop_n, bool tbug, ST scale, ST rhs) {
+// residual of one cell for operator E, G, B; `scale` is 1/Pr for T
+template <typename ST, class X>
+__device__ __forceinline__ ST sw_residual(const X& x, ST E, ST G, ST B, bool nearw, bool drop_s, bool drop_n, bool tbug,
+                                          ST scale, ST rhs) {
     // off-centre sum: the 25-point form, or the 9-point form on the near-wall cells
-    ST sm = nearw ? sw_sum9<ST>(w, q, E, G, B, drop_s, drop_n) : sw_sum25<ST>(w, q, E, G, B);
-    if (tbug && !nearw) sm -= B * w[q + 4][1];
+    ST sm = nearw ? sw_sum9<ST>(x, E, G, B, drop_s, drop_n) : sw_sum25<ST>(x, E, G, B);
+    if (tbug && !nearw) sm -= B * x(2, -1);
     sm *= scale;
     const ST D = (nearw ? ST(2) : ST(2.5)) * (E + G);
     const ST ap = ST(1) + D * scale;
-    return rhs - ap * w[q + 2][2] - sm;
+    return rhs - ap * x(0, 0) - sm;
 }
 
 // x_{k+1} from the residual (Chebyshev weight wgt on every sweep but the first)

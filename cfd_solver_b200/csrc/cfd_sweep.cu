@@ -4,19 +4,23 @@
 // One CTA sweeps one 32 x 16 tile of one case for all of its still-iterating fields.
 // The fields stream through two shared-memory buffers: each field's x tile with its
 // 2-cell halo, its right-hand side and (after the first sweep) the previous iterate
-// arrive by tensor copies completed on the buffer's mbarrier, and the copies of field
-// k+2 are issued as soon as field k has been read into registers, so they overlap the
-// arithmetic of field k and the wait for field k+1. The first field also brings alpha,
+// arrive by tensor copies completed on the buffer's mbarrier. The barrier that opens field k
+// also tells that field k-1 has been read, so the copies of field k+1 go out then and overlap
+// the arithmetic of field k: one barrier per field. The first field also brings alpha,
 // beta, gamma; every thread turns its own cells' values into the operator (E, G, B and
 // the two inverse diagonals) in place, in a thread-private part of shared memory that
 // needs no barrier and costs no registers.
 //
 // A warp owns four consecutive rows of the tile, a lane one column: the thread reads its
-// eight-row x five-column window once into registers, so its four cells cost ten
-// shared-memory loads each instead of twenty-five. Each cell's off-centre sum (25-point, or
-// 9-point on the near-wall cells) is formed just before its update, and the per-CTA
-// constants and each field's warp residual sums sit in shared memory, so the kernel holds
-// its 128 registers with little spilling. The per-tile L1 residuals go to one partial row
+// eight-row x five-column window once, row by row, so its four cells cost ten shared-memory
+// loads each instead of twenty-five, and finishes each cell (off-centre sum: 25-point, or
+// 9-point on the near-wall cells; right-hand side, previous iterate, update) as its last row
+// comes in. With five live rows instead of eight, and the cells' flags packed in one
+// word, the kernel needs 118 registers where it filled 128 and spilled; k_sweep_f64 went from
+// 987 to 878 us per step of the 256-case twin sweep (bound by the latency of the FP64 chains,
+// then by bytes). Five CTAs per SM need 96 registers and spill (1,079 us), or re-read the
+// outer columns (922). The per-CTA constants and each field's warp residual sums sit in
+// shared memory. The per-tile L1 residuals go to one partial row
 // per tile that k_sweep_fin sums per case in a fixed order after the launch.
 //
 // Three modes share the code:
@@ -200,14 +204,15 @@ __device__ __forceinline__ void sweep_tile(const BatchDev& b, unsigned char* sm,
     }
     const int ld = c.ld, xld = c.xld, W = c.W, per = c.periodic;
     const int i = t.i0 + lane;
-    bool inq[SW_ROWS], nearw[SW_ROWS], drop_s[SW_ROWS], drop_n[SW_ROWS];
+    // the thread's cells, four bits each: in the case, near a wall, no southern / northern coupling
+    unsigned cell = 0;
 #pragma unroll
     for (int q = 0; q < SW_ROWS; q++) {
         const int j = t.j0 + wrp * SW_ROWS + q;
-        inq[q] = i >= c.ilo && i <= c.ihi && j <= c.n1 - 2;
-        nearw[q] = j == 1 || j == c.n1 - 2 || (c.profile == CAVITY && (i == 1 || i == c.n0 - 2));
-        drop_s[q] = c.profile == OGRID && j == 1;
-        drop_n[q] = c.profile == OGRID && j == c.n1 - 2;
+        const bool in = i >= c.ilo && i <= c.ihi && j <= c.n1 - 2;
+        const bool nw = j == 1 || j == c.n1 - 2 || (c.profile == CAVITY && (i == 1 || i == c.n0 - 2));
+        const bool ds = c.profile == OGRID && j == 1, dn = c.profile == OGRID && j == c.n1 - 2;
+        cell |= (in | nw << 1 | ds << 2 | dn << 3) << (4 * q);
     }
     __syncthreads();
 
@@ -236,7 +241,7 @@ __device__ __forceinline__ void sweep_tile(const BatchDev& b, unsigned char* sm,
             for (int q = 0; q < SW_ROWS; q++) {
                 const int o = (wrp * SW_ROWS + q) * TX + lane;
                 const double E = kE * MET[o], B = kB * MET[SW_CELLS + o], G = kG * MET[2 * SW_CELLS + o];
-                const double D = (nearw[q] ? 2.0 : 2.5) * (E + G);
+                const double D = ((cell >> (4 * q) & 2) ? 2.0 : 2.5) * (E + G);
                 OPS[o] = (ST)E;
                 OPS[SW_CELLS + o] = (ST)G;
                 OPS[2 * SW_CELLS + o] = (ST)B;
@@ -245,33 +250,18 @@ __device__ __forceinline__ void sweep_tile(const BatchDev& b, unsigned char* sm,
                 RAP[SW_CELLS + o] = (float)__drcp_rn(1.0 + D * rPr64);
             }
         }
+        // every thread has read field k - 1: its buffer takes field k + 1
+        if (k >= 1 && tid == 0) {
+            const int nx = fm & (fm - 1);
+            if (nx) {
+                const int f2 = __ffs(nx) - 1;
+                sw_issue<MODE>(t, f2, sweep, nxt, maps, sm + (bi ^ 1) * L::BUF, nullptr, &bar[bi ^ 1], (flipm >> f2) & 1);
+            }
+        }
         const bool isT = f == F_T;
         const XT* X = reinterpret_cast<const XT*>(buf + L::X);
         const RT* R = reinterpret_cast<const RT*>(buf + L::RHS);
         const XT* P = reinterpret_cast<const XT*>(buf + L::PREV);
-        // the thread's window: rows wrp*4 - 2 .. wrp*4 + 5, columns lane - 2 .. lane + 2
-        ST w[8][5];
-        ST rhs[SW_ROWS], xm[SW_ROWS];
-#pragma unroll
-        for (int q = 0; q < SW_ROWS; q++) {
-            const int o = (wrp * SW_ROWS + q) * TX + lane;
-            rhs[q] = (ST)R[o];
-            xm[q] = has_prev ? (ST)P[o] : ST(0);
-        }
-#pragma unroll
-        for (int rr = 0; rr < 8; rr++)
-#pragma unroll
-            for (int cl = 0; cl < 5; cl++) w[rr][cl] = (ST)X[(wrp * SW_ROWS + rr) * C::XW + lane + cl + C::XO - 2];
-        __syncthreads();  // the buffer has been read: refill it with the field after next
-        if (tid == 0) {
-            int nx = fm & (fm - 1);
-            nx &= nx - 1;
-            if (nx) {
-                const int f2 = __ffs(nx) - 1;
-                sw_issue<MODE>(t, f2, sweep, nxt, maps, sm + bi * L::BUF, nullptr, &bar[bi], (flipm >> f2) & 1);
-            }
-        }
-
         const ST g = sconst[isT ? 1 : 0], wgt = sconst[isT ? 3 : 2];
         const ST scale = isT ? sconst[4] : ST(1);
         // the reference's T solve passes atnw in the annw slot (PSolver.cpp:1290): the
@@ -292,29 +282,41 @@ __device__ __forceinline__ void sweep_tile(const BatchDev& b, unsigned char* sm,
             dst32 = xplane(b, c, (sweep & 1) == 0 ? X_DB + f : X_DA + f);
             dld = xld;
         }
+        // the thread's window, rows wrp*4 - 2 .. wrp*4 + 5, columns lane - 2 .. lane + 2
+        ST w[SW_ROWS + 4][5];
+        const int row0 = (t.j0 + wrp * SW_ROWS) * dld;
+        const XT* xw = X + (wrp * SW_ROWS) * C::XW + lane + C::XO - 2;
         double racc = 0.0;
 #pragma unroll
-        for (int q = 0; q < SW_ROWS; q++) {
+        for (int rr = 0; rr < SW_ROWS + 4; rr++) {
+#pragma unroll
+            for (int cl = 0; cl < 5; cl++) w[rr][cl] = (ST)xw[rr * C::XW + cl];
+            if (rr < 4) continue;
+            const int q = rr - 4;
             const int o = (wrp * SW_ROWS + q) * TX + lane;
+            const bool nearw = cell >> (4 * q) & 2;
             const ST E = OPS[o], G = OPS[SW_CELLS + o], B = OPS[2 * SW_CELLS + o];
-            const ST res = sw_residual<ST>(w, q, E, G, B, nearw[q], drop_s[q], drop_n[q], tbug, scale, rhs[q]);
+            const auto x = [&](int dy, int dx) { return w[q + 2 + dy][2 + dx]; };
+            const ST res = sw_residual<ST>(x, E, G, B, nearw, cell >> (4 * q) & 4, cell >> (4 * q) & 8, tbug, scale,
+                                           (ST)R[o]);
             const ST rap = (ST)RAP[rapoff + o];
             const ST xk = w[q + 2][2];
-            racc += inq[q] ? fabs((double)res) : 0.0;
-            const long long kk = (long long)(t.j0 + wrp * SW_ROWS + q) * dld;
+            const bool in = cell >> (4 * q) & 1;
+            racc += in ? fabs((double)res) : 0.0;
+            const int kk = row0 + q * dld;
             if (MODE == SW_MX0) {
-                const float d1 = (float)(g * res * rap), rr = (float)res;
-                if (inq[q]) {
+                const float d1 = (float)(g * res * rap), rr32 = (float)res;
+                if (in) {
                     dst32[kk + i] = d1;
-                    res32[kk + i] = rr;
+                    res32[kk + i] = rr32;
                     if (mcol > -1000000) {
                         dst32[kk + mcol] = d1;
-                        res32[kk + mcol] = rr;
+                        res32[kk + mcol] = rr32;
                     }
                 }
             } else {
-                const ST xn = sw_next<ST>(xk, g, res, rap, weighted, wgt, xm[q]);
-                if (inq[q]) {
+                const ST xn = sw_next<ST>(xk, g, res, rap, weighted, wgt, has_prev ? (ST)P[o] : ST(0));
+                if (in) {
                     if (MODE == SW_F64) {
                         dst64[kk + i] = (double)xn;
                         if (mcol > -1000000) dst64[kk + mcol] = (double)xn;
@@ -334,7 +336,7 @@ __device__ __forceinline__ void sweep_tile(const BatchDev& b, unsigned char* sm,
         if (tid == 0) {
             atomicExch(b.error, 1);
             // let the copies still in flight land before the CTA leaves (the long default limit)
-            for (int m = k; m < nf && m < k + 2; m++) mbar_wait_bounded(&bar[m & 1], (m >> 1) & 1);
+            for (int m = k; m < nf && m < max(k + 1, 2); m++) mbar_wait_bounded(&bar[m & 1], (m >> 1) & 1);
         }
         return;
     }

@@ -344,7 +344,8 @@ __device__ __noinline__ void team_sweep(int sweep, int nxt) {
             for (int q = 0; q < SW_ROWS; q++) {
                 const int o = (wrp * SW_ROWS + q) * TX + lane;
                 const ST E = (ST)OPS[o], G = (ST)OPS[TX * TYJ + o], B = (ST)OPS[2 * TX * TYJ + o];
-                const ST res = sw_residual<ST>(w, q, E, G, B, nearw[q], drop_s[q], drop_n[q], tbug, scale, rhs[q]);
+                const auto x = [&](int dy, int dx) { return w[q + 2 + dy][2 + dx]; };
+                const ST res = sw_residual<ST>(x, E, G, B, nearw[q], drop_s[q], drop_n[q], tbug, scale, rhs[q]);
                 const ST rap = (ST)RAP[rapoff + o];
                 const ST xk = w[q + 2][2];
                 racc += inq[q] ? fabs((double)res) : 0.0;
