@@ -601,7 +601,7 @@ __global__ void __launch_bounds__(MG_GS_THREADS, 8) k_mg_gs(BatchDev b, int l, i
 }
 
 // coarsest level: `sweeps` multicolour GS sweeps by one CTA per case (mg_coarse_solve)
-constexpr int MGC_THREADS = 1024, MGC_SMEM = 6144;
+constexpr int MGC_THREADS = 1024, MGC_SMEM = 12000;
 __global__ void __launch_bounds__(MGC_THREADS) k_mg_coarse(BatchDev b, int l, int sweeps) {
     __shared__ float xs[MGC_SMEM];
     // l < 0: one launch for every case, each on its own coarsest level (the case lists of

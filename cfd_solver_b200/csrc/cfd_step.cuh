@@ -949,31 +949,59 @@ __device__ __forceinline__ void mg_coarse_regs(const BatchDev& b, const CaseDev&
     }
 }
 
-// the same sweeps through global memory, for a level whose x does not fit
+// The same sweeps for a level with more points of a colour than the threads hold: the stencils are
+// read in every pass (from L2: a colour's are a quarter of the level's), four points per thread
+// in flight at a time, and only the points of the pass's colour are visited. x is in shared
+// memory where it fits, else in its own plane: `x` is point (0, 0), rows `xs` apart. Four steps of
+// a 36 x 217 cavity (one level of 34 x 215 unknowns) take 14.7 ms with it, 33.0 with a visit of
+// every point per pass and all of x in global memory.
 template <class Grp>
-__device__ __forceinline__ void mg_coarse_global(const BatchDev& b, const CaseDev& c, const LevelDev& L, int sweeps,
-                                                 const Grp& g) {
-    const int ld = L.ld, per = c.periodic, tid = g.tid;
-    const int nx = L.ihi - L.ilo + 1, ny = L.n1 - 2;
-    const int ncol = (per && (L.W & 1)) ? 6 : 4;
-    float* X = mplane(b, L, M_X);
+__device__ __forceinline__ void mg_coarse_stream(const BatchDev& b, const CaseDev& c, const LevelDev& L, int sweeps,
+                                                 float* x, int xs, const Grp& g) {
+    constexpr int U = 4;
+    const int ld = L.ld, per = c.periodic, W = L.W;
+    const int nx = L.ihi - L.ilo + 1, n = nx * (L.n1 - 2);
+    const float* A = mplane(b, L, M_AP);
     const float* Bv = mplane(b, L, M_B);
-    for (int e = tid; e < nx * ny; e += Grp::N) {  // x = 0
-        const int i = L.ilo + e % nx, j = 1 + e / nx;
-        store_mirrored(X, ld, i, j, L.W, per, 0.0f);
-    }
+    for (int e = g.tid; e < n; e += Grp::N) store_mirrored(x, xs, L.ilo + e % nx, 1 + e / nx, W, per, 0.0f);
     g.sync();
+    const bool odd = per && (W & 1);
     for (int s = 0; s < sweeps; s++) {
-        for (int col = 0; col < ncol; col++) {
-            for (int e = tid; e < nx * ny; e += Grp::N) {
-                const int i = L.ilo + e % nx, j = 1 + e / nx;
-                if (mg_colour(i, j, L.W, per) != col) continue;
-                const long long k = (long long)j * ld + i;
-                const float sm = mplane(b, L, M_AE)[k] * X[k + 1] + mplane(b, L, M_AW)[k] * X[k - 1] +
-                                 mplane(b, L, M_AN)[k] * X[k + ld] + mplane(b, L, M_AS)[k] * X[k - ld] +
-                                 mplane(b, L, M_ANE)[k] * X[k + ld + 1] + mplane(b, L, M_ANW)[k] * X[k + ld - 1] +
-                                 mplane(b, L, M_ASE)[k] * X[k - ld + 1] + mplane(b, L, M_ASW)[k] * X[k - ld - 1];
-                store_mirrored(X, ld, i, j, L.W, per, (Bv[k] - sm) / mplane(b, L, M_AP)[k]);
+        for (int cc = 0; cc < (odd ? 6 : 4); cc++) {
+            // colours 4 and 5: the last column's even and odd rows
+            MgColour q(L, per, cc & 3);
+            if (cc >= 4) {
+                q.fi = W - 1;
+                q.fj = 6 - cc;
+                q.nx = 1;
+                q.n = (L.n1 - 2 - q.fj) / 2 + 1;
+            }
+            for (int e0 = g.tid; e0 < q.n; e0 += U * Grp::N) {
+                float f[U][9], rhs[U];
+                int at[U], ii[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int e = e0 + u * Grp::N;
+                    const int r = e < q.n ? e / q.nx : 0, i = e < q.n ? q.fi + 2 * (e - r * q.nx) : q.fi, j = q.fj + 2 * r;
+                    const long long p = (long long)j * ld + i;
+#pragma unroll
+                    for (int m = 0; m < 9; m++) f[u][m] = A[m * L.ps + p];
+                    rhs[u] = Bv[p];
+                    at[u] = j * xs + i;
+                    ii[u] = e < q.n ? i : -1;
+                }
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    if (ii[u] < 0) continue;
+                    float* v = x + at[u];
+                    const float sm = f[u][1] * v[1] + f[u][2] * v[-1] + f[u][3] * v[xs] + f[u][4] * v[-xs] +
+                                     f[u][5] * v[xs + 1] + f[u][6] * v[xs - 1] + f[u][7] * v[-xs + 1] +
+                                     f[u][8] * v[-xs - 1];
+                    const float r = (rhs[u] - sm) / f[u][0];
+                    v[0] = r;
+                    const int m = mirror_col(ii[u], W, per);
+                    if (m > -1000000) v[m - ii[u]] = r;
+                }
             }
             g.sync();
         }
@@ -987,10 +1015,26 @@ __device__ __forceinline__ void mg_coarse_solve(const BatchDev& b, const CaseDev
     // the odd rows' colours have at least as many points as the even rows', and one of the two
     // column parities the most
     const int most = max(MgColour(L, c.periodic, 2).n, MgColour(L, c.periodic, 3).n);
-    if (most > KMAX * Grp::N || L.n1 * (L.W + 2 * H) > xs_cap) mg_coarse_global(b, c, L, sweeps, g);
-    else if ((L.ihi - L.ilo + 1) * (L.n1 - 2) <= Grp::N) mg_coarse_small(b, c, L, sweeps, xs, g);
-    else if (KMAX == 1 || most <= Grp::N) mg_coarse_regs<1>(b, c, L, sweeps, xs, g);
-    else mg_coarse_regs<KMAX>(b, c, L, sweeps, xs, g);
+    const int sw = L.W + 2 * H, nx = L.ihi - L.ilo + 1, n = nx * (L.n1 - 2);
+    const bool fits = L.n1 * sw <= xs_cap;
+    float* X = mplane(b, L, M_X);
+    if (fits && n <= Grp::N) {
+        mg_coarse_small(b, c, L, sweeps, xs, g);
+    } else if (fits && most <= Grp::N) {
+        mg_coarse_regs<1>(b, c, L, sweeps, xs, g);
+    } else if (fits && KMAX > 1 && most <= KMAX * Grp::N) {
+        mg_coarse_regs<KMAX>(b, c, L, sweeps, xs, g);
+    } else if (fits) {
+        for (int e = g.tid; e < L.n1 * sw; e += Grp::N) xs[e] = 0.0f;
+        g.sync();
+        mg_coarse_stream(b, c, L, sweeps, xs + H, sw, g);
+        for (int e = g.tid; e < n; e += Grp::N) {
+            const int i = L.ilo + e % nx, j = 1 + e / nx;
+            store_mirrored(X, L.ld, i, j, L.W, c.periodic, xs[j * sw + i + H]);
+        }
+    } else {
+        mg_coarse_stream(b, c, L, sweeps, X, L.ld, g);
+    }
 }
 
 // ---------------------------------------------------------------------------

@@ -18,7 +18,7 @@
 // comes in. With five live rows instead of eight, and the cells' flags packed in one
 // word, the kernel needs 118 registers where it filled 128 and spilled; k_sweep_f64 went from
 // 987 to 878 us per step of the 256-case twin sweep (bound by the latency of the FP64 chains,
-// then by bytes). Five CTAs per SM need 96 registers and spill (1,079 us), or re-read the
+// then by bytes). Five CTAs per SM need 96 registers: with spills 1,213 us, re-reading the
 // outer columns (922). The per-CTA constants and each field's warp residual sums sit in
 // shared memory. The per-tile L1 residuals go to one partial row
 // per tile that k_sweep_fin sums per case in a fixed order after the launch.

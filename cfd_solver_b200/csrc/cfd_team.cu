@@ -67,7 +67,7 @@ struct TeamSh {
 constexpr int OPS_BYTES = 3 * TX * TYJ * 8 + 2 * TX * TYJ * 4;  // one sweep group's operator
 constexpr int OPS_OFF = (sizeof(TeamSh) + 127) / 128 * 128;
 constexpr int WORK_OFF = OPS_OFF + (NT5 / SW_THREADS) * OPS_BYTES;
-constexpr int COARSE_WORDS = 6144;
+constexpr int COARSE_WORDS = 12000;
 constexpr int WORK_MIN = COARSE_WORDS * 4;
 static_assert((2 * MPR_XP + 2 * MPR_RP) * 4 <= WORK_MIN && 4 * 2 * MG_GS_XP * 4 <= WORK_MIN, "work area");
 

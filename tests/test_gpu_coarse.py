@@ -2,7 +2,7 @@
 
 A grid whose sides do not halve has one level, so the whole preconditioner is the coarsest
 level's sweeps. They run with one, two or four unknowns per thread in registers (1024
-threads), or through global memory above that; every size here is one side or the other of
+threads), or re-read them in every pass above that; every size here is one side or the other of
 an edge. The solve must reach the sparse direct solution (tests/test_gpu_seam.py's bar).
 """
 import numpy as np
@@ -17,10 +17,11 @@ pytestmark = pytest.mark.gpu
     ("ogrid", 46, 24),    # 45 x 22 = 990 unknowns: one per thread (odd width: six colours)
     ("ogrid", 46, 26),    # 45 x 24 = 1080: two
     ("ogrid", 46, 48),    # 45 x 46 = 2070: four
-    ("ogrid", 46, 94),    # 45 x 92 = 4140: global memory
+    ("ogrid", 46, 94),    # 45 x 92 = 4140: stencils re-read in every pass
+    ("ogrid", 132, 130),  # 131 x 128, x of 130 x 137 words: x in its plane as well
     ("cavity", 34, 34),   # 32 x 32 = 1024: one (four colours)
     ("cavity", 66, 66),   # 64 x 64 = 4096: four, x of 66 x 70 words
-    ("cavity", 10, 512),  # 8 x 510 = 4080 unknowns, x of 512 x 14 words: global memory
+    ("cavity", 10, 512),  # 8 x 510 = 4080 unknowns, x of 512 x 14 words: two, four or re-read
 ])
 def test_single_level_solve_matches_direct_solve(kind, n0, n1):
     from oracle import oracle
