@@ -58,12 +58,12 @@ constexpr int NFLAGS = 10;  // device flag words of a batch
 enum KernelId {
     K_ASSEMBLE_P, K_RHS, K_SWEEP, K_UPBC, K_FACE_Q, K_BICG_P, K_SPMV, K_BICG_S, K_BICG_X,
     K_MG_SMOOTH, K_MG_RR, K_MG_POST, K_MG_COARSE, K_MG_GALERKIN,
-    K_CORRECT, K_BC, K_DIAG, K_SI, K_MOM_UPDATE, K_SWEEP_FIN, K_MG_PRR, K_MOM_FIX, NKERNEL
+    K_CORRECT, K_BC, K_DIAG, K_SI, K_MOM_UPDATE, K_SWEEP_FIN, K_MG_PRR, K_MOM_FIX, K_FIN, NKERNEL
 };
 const char* kKernelNames[NKERNEL] = {
     "k_assemble_p", "k_rhs", "k_sweep", "k_upbc", "k_face_q", "k_bicg_p", "k_spmv", "k_bicg_s",
     "k_bicg_x", "k_mg_presmooth", "k_mg_rr", "k_mg_postsmooth", "k_mg_coarse",
-    "k_mg_galerkin", "k_correct", "k_bc", "k_diag", "k_si", "k_mom_update", "k_sweep_fin", "k_mg_prr", "k_mom_fix"};
+    "k_mg_galerkin", "k_correct", "k_bc", "k_diag", "k_si", "k_mom_update", "k_sweep_fin", "k_mg_prr", "k_mom_fix", "k_fin"};
 
 struct LevelGeom {
     int W, n1, ld, ilo, ihi;
@@ -166,7 +166,6 @@ struct cfd_batch {
     double* scal = nullptr;
     int* iscal = nullptr;
     double* partial = nullptr;
-    unsigned int* counter = nullptr;
     // device flags: [0] cases still in the pressure solve, [1] (case, field) pairs still in
     // the momentum solves, [2] / [3] this step's momentum-pair / pressure-iteration counts,
     // [4] kernel wait timeout, [5] / [6] cumulative pair / iteration counts (graph steps),
@@ -712,6 +711,11 @@ void enq_mom_mx_next(cfd_batch* b, BatchDev& bd) {
 int mom_loop_cap(const cfd_batch* b) {
     return b->precision == CFD_PRECISION_MIXED ? std::max(1, b->maxit_mom - 1) : std::max(1, b->maxit_mom / 2);
 }
+// the totals of the tile kernel just launched
+void enq_fin(cfd_batch* b, BatchDev& bd, FinKernel what) {
+    Prof pr(b, K_FIN);
+    k_fin<<<b->n, NT, 0, b->st>>>(bd, what, b->maxit_p);
+}
 void enq_mid(cfd_batch* b, BatchDev& bd) {
     if (b->precision == CFD_PRECISION_MIXED) {
         Prof pr(b, K_MOM_UPDATE);
@@ -724,8 +728,11 @@ void enq_mid(cfd_batch* b, BatchDev& bd) {
         Prof pr(b, K_UPBC);
         k_upbc<<<b->n, BC_THREADS, 0, b->st>>>(bd);
     }
-    Prof pr(b, K_FACE_Q);
-    k_face_q<<<bd.njtiles, NT, kFaceQSmem, b->st>>>(bd);
+    {
+        Prof pr(b, K_FACE_Q);
+        k_face_q<<<bd.njtiles, NT, kFaceQSmem, b->st>>>(bd);
+    }
+    enq_fin(b, bd, FIN_FACE_Q);
 }
 // one BiCGStab iteration in two halves: up to the half-step exit (k_bicg_s), and the rest,
 // which the step graph skips when every case stopped at the half step. The next iteration's
@@ -736,13 +743,17 @@ void enq_p_first(cfd_batch* b, BatchDev& bd) {
     const int nf = bd.njtiles;  // the BiCGStab kernels run on the 32 x 16 tiles
     run_vcycle(b);
     { Prof pr(b, K_SPMV); k_spmv<<<nf, NT, 0, b->st>>>(bd, 0); }
+    enq_fin(b, bd, FIN_SPMV0);
     { Prof pr(b, K_BICG_S); k_bicg_s<<<nf, NT, 0, b->st>>>(bd); }
+    enq_fin(b, bd, FIN_BICG_S);
 }
 void enq_p_second(cfd_batch* b, BatchDev& bd) {
     const int nf = bd.njtiles;
     run_vcycle(b);
     { Prof pr(b, K_SPMV); k_spmv<<<nf, NT, 0, b->st>>>(bd, 1); }
-    { Prof pr(b, K_BICG_X); k_bicg_x<<<nf, NT, 0, b->st>>>(bd, b->maxit_p); }
+    enq_fin(b, bd, FIN_SPMV1);
+    { Prof pr(b, K_BICG_X); k_bicg_x<<<nf, NT, 0, b->st>>>(bd); }
+    enq_fin(b, bd, FIN_BICG_X);
     { Prof pr(b, K_BICG_P); k_bicg_p<<<nf, NT, 0, b->st>>>(bd); }
 }
 void enq_p_iter(cfd_batch* b, BatchDev& bd) {
@@ -753,6 +764,7 @@ void enq_end(cfd_batch* b, BatchDev& bd) {
     { Prof pr(b, K_CORRECT); k_correct<<<bd.njtiles, NT, 0, b->st>>>(bd); }
     { Prof pr(b, K_BC); k_bc<<<b->n, BC_THREADS, 2 * (b->max_W + 1) * sizeof(double), b->st>>>(bd); }
     { Prof pr(b, K_DIAG); k_diag<<<bd.njtiles, NT, 0, b->st>>>(bd); }
+    enq_fin(b, bd, FIN_STEP);
 }
 
 // one step with host-side loop control (per-kernel profiling works on this path)
@@ -1509,7 +1521,6 @@ int cfd_batch_create(int ncases, const cfd_grid* grids, const cfd_params* params
     ALLOC(b->dc, sizeof(CaseDev) * ncases);
     ALLOC(b->scal, sizeof(double) * NSCAL * ncases);
     ALLOC(b->iscal, sizeof(int) * NISCAL * ncases);
-    ALLOC(b->counter, sizeof(unsigned) * ncases);
     ALLOC(b->flags, sizeof(int) * NFLAGS);
     ALLOC(b->work, sizeof(unsigned long long) * 4);
     ALLOC(b->dtmaps, (size_t)TMAP_STRIDE * ncases);
@@ -1520,7 +1531,6 @@ int cfd_batch_create(int ncases, const cfd_grid* grids, const cfd_params* params
     cudaMemsetAsync(b->f32, 0, (size_t)b->n32 * sizeof(float), b->st);
     cudaMemsetAsync(b->scal, 0, sizeof(double) * NSCAL * ncases, b->st);
     cudaMemsetAsync(b->iscal, 0, sizeof(int) * NISCAL * ncases, b->st);
-    cudaMemsetAsync(b->counter, 0, sizeof(unsigned) * ncases, b->st);
     cudaMemsetAsync(b->work, 0, sizeof(unsigned long long) * 4, b->st);
     cudaMemsetAsync(b->flags, 0, sizeof(int) * NFLAGS, b->st);
     CK(cudaStreamSynchronize(b->st));
@@ -1533,7 +1543,7 @@ int cfd_batch_create(int ncases, const cfd_grid* grids, const cfd_params* params
 
     BatchDev& bd = b->bd;
     bd.cases = b->dc; bd.ncases = ncases; bd.f64 = b->f64; bd.f32 = b->f32;
-    bd.scal = b->scal; bd.iscal = b->iscal; bd.counter = b->counter;
+    bd.scal = b->scal; bd.iscal = b->iscal;
     bd.active = b->flags; bd.mactive = b->flags + 1;
     bd.work = b->work;
     bd.tmaps = b->dtmaps;
@@ -1663,7 +1673,6 @@ int cfd_pool_create(size_t hbm_budget, int max_cases, int precision, cfd_batch**
     ALLOC(b->dc, sizeof(CaseDev) * max_cases);
     ALLOC(b->scal, sizeof(double) * NSCAL * max_cases);
     ALLOC(b->iscal, sizeof(int) * NISCAL * max_cases);
-    ALLOC(b->counter, sizeof(unsigned) * max_cases);
     ALLOC(b->flags, sizeof(int) * NFLAGS);
     ALLOC(b->work, sizeof(unsigned long long) * 4);
     ALLOC(b->dtmaps, (size_t)TMAP_STRIDE * max_cases);
@@ -1675,7 +1684,6 @@ int cfd_pool_create(size_t hbm_budget, int max_cases, int precision, cfd_batch**
     for (int c = 0; c < max_cases; c++) is[(size_t)c * NISCAL + I_PDONE] = 1;
     if (cudaMemsetAsync(b->scal, 0, sizeof(double) * NSCAL * max_cases, b->st) != cudaSuccess ||
         cudaMemcpyAsync(b->iscal, is.data(), sizeof(int) * is.size(), cudaMemcpyHostToDevice, b->st) != cudaSuccess ||
-        cudaMemsetAsync(b->counter, 0, sizeof(unsigned) * max_cases, b->st) != cudaSuccess ||
         cudaMemsetAsync(b->work, 0, sizeof(unsigned long long) * 4, b->st) != cudaSuccess ||
         cudaMemsetAsync(b->flags, 0, sizeof(int) * NFLAGS, b->st) != cudaSuccess ||
         cudaStreamSynchronize(b->st) != cudaSuccess)
@@ -1683,7 +1691,7 @@ int cfd_pool_create(size_t hbm_budget, int max_cases, int precision, cfd_batch**
     if (int rc = set_kernel_attributes(b)) return cleanup(rc);
     BatchDev& bd = b->bd;
     bd.cases = b->dc; bd.ncases = max_cases; bd.f64 = b->f64; bd.f32 = b->f32;
-    bd.scal = b->scal; bd.iscal = b->iscal; bd.counter = b->counter;
+    bd.scal = b->scal; bd.iscal = b->iscal;
     bd.active = b->flags; bd.mactive = b->flags + 1;
     bd.work = b->work;
     bd.tmaps = b->dtmaps;
@@ -1830,7 +1838,7 @@ int cfd_batch_destroy(cfd_batch* b) {
     if ((void*)b->f32 != (void*)b->f64) cudaFree(b->f32);
     cudaFree(b->f64); cudaFree(b->dc); cudaFree(b->scal); cudaFree(b->iscal);
     cudaFree(b->stage); cudaFree(b->stage_off);
-    cudaFree(b->partial); cudaFree(b->counter); cudaFree(b->flags); cudaFree(b->work); cudaFree(b->tword); cudaFree(b->dtiles); cudaFree(b->dcc); cudaFree(b->dtmaps);
+    cudaFree(b->partial); cudaFree(b->flags); cudaFree(b->work); cudaFree(b->tword); cudaFree(b->dtiles); cudaFree(b->dcc); cudaFree(b->dtmaps);
     cudaFree(b->team_ids); cudaFree(b->team_bar);
     if (b->h_flags) cudaFreeHost(b->h_flags);
     if (b->st) cudaStreamDestroy(b->st);

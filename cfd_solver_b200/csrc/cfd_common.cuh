@@ -158,8 +158,7 @@ struct BatchDev {
     float* f32;
     double* scal;          // ncases * NSCAL
     int* iscal;            // ncases * NISCAL
-    double* partial;       // reduction partials: ntiles_max * 8
-    unsigned int* counter; // per case, last-block detection
+    double* partial;       // reduction partials: rows of 8 per tile
     int* active;           // global count of cases still iterating (pressure)
     int* mactive;          // global count of (case, field) pairs still iterating (momentum)
     int* error;            // set when a bounded wait in a kernel gives up

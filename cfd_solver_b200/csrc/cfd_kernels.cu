@@ -275,31 +275,7 @@ __global__ void __launch_bounds__(NT, 4) k_face_q(BatchDev b) {
         red[1] += q * q;
         red[2] = fmax(red[2], fabs(q));
     }
-    if (case_reduce<3, 0x4u>(b, t.c, blockIdx.x, c.jt_begin, c.jt_count, red) && tid == 0) {
-        double* sc = b.scal + (long long)t.c * NSCAL;
-        int* is = b.iscal + (long long)t.c * NISCAL;
-        sc[S_QL1] = red[0];
-        sc[S_QL2] = sqrt(red[1]);
-        if (is[I_NSTEP] == 0) sc[S_QL2_0] = sqrt(red[1]);
-        sc[S_QMAX] = red[2];
-        sc[S_RHO] = red[1];
-        sc[S_ALPHA] = 1.0;
-        sc[S_OMEGA] = 1.0;
-        sc[S_BETA] = 0.0;
-        sc[S_NB1] = red[0];
-        sc[S_RL1] = red[0];
-        is[I_PIT] = 0;
-        // this step's solver status starts with the momentum / energy solves: a field still
-        // iterating when their loop ended stopped at the sweep cap
-        is[I_PSTATUS] = (is[I_MWORD] & ((1 << NFIELD) - 1)) ? ST_MAXITER : 0;
-        if (red[0] == 0.0 || !isfinite(red[0])) {
-            is[I_PDONE] = 1;
-            if (!isfinite(red[0])) is[I_STATUS] |= ST_NAN;
-        } else {
-            is[I_PDONE] = 0;
-            atomicAdd(b.active, 1);
-        }
-    }
+    tile_partial<3, 0x4u>(b, blockIdx.x, 0, red);
 }
 
 // ---------------------------------------------------------------------------
@@ -385,20 +361,11 @@ __global__ void __launch_bounds__(NT, 5) k_spmv(BatchDev b, int mode) {
             red[1] += y[h] * y[h];
         }
     }
-    if (case_reduce<2, 0u>(b, t.c, blockIdx.x, c.jt_begin, c.jt_count, red) && threadIdx.x == 0) {
-        double* sc = b.scal + (long long)t.c * NSCAL;
-        int* is = b.iscal + (long long)t.c * NISCAL;
-        if (mode == 0) {
-            if (red[0] == 0.0 || !isfinite(red[0])) {
-                is[I_PSTATUS] |= ST_BREAKDOWN;
-                is[I_PDONE] = 1;
-                atomicSub(b.active, 1);
-            } else {
-                sc[S_ALPHA] = sc[S_RHO] / red[0];
-            }
-        } else {
-            sc[S_OMEGA] = red[1] > 0.0 ? red[0] / red[1] : 0.0;
-        }
+    if (mode == 0) {
+        const double one[1] = {red[0]};
+        tile_partial<1, 0u>(b, blockIdx.x, 0, one);
+    } else {
+        tile_partial<2, 0u>(b, blockIdx.x, 0, red);
     }
 }
 
@@ -441,27 +408,16 @@ __global__ void __launch_bounds__(NT, 5) k_bicg_s(BatchDev b) {
         mplane(b, L, M_B)[(long long)j * L.ld + i] = (float)s;
         red[0] += fabs(s);
     }
-    if (case_reduce<1, 0u>(b, t.c, blockIdx.x, c.jt_begin, c.jt_count, red) && threadIdx.x == 0) {
-        double* sc = b.scal + (long long)t.c * NSCAL;
-        int* is = b.iscal + (long long)t.c * NISCAL;
-        const bool conv = red[0] <= c.tol_p * sc[S_NB1] || red[0] <= c.atol_p;
-        if (conv || !isfinite(red[0])) {
-            is[I_PIT] += 1;
-            sc[S_RL1] = red[0];
-            if (!isfinite(red[0])) is[I_STATUS] |= ST_NAN;
-            is[I_PDONE] = 1;
-            atomicSub(b.active, 1);
-        }
-    }
+    tile_partial<1, 0u>(b, blockIdx.x, 0, red);
 }
 
-__global__ void __launch_bounds__(NT, 5) k_bicg_x(BatchDev b, int maxit) {
+__global__ void __launch_bounds__(NT, 5) k_bicg_x(BatchDev b) {
     const Tile t = b.jtiles[blockIdx.x];
     if (b.iscal[(long long)t.c * NISCAL + I_PDONE]) return;
     const CaseDev& c = b.cases[t.c];
     const int i = t.i0 + (int)(threadIdx.x % TX), j0 = t.j0 + (int)(threadIdx.x / TX);
     const double* sc0 = b.scal + (long long)t.c * NSCAL;
-    const double alpha = sc0[S_ALPHA], omega = sc0[S_OMEGA];
+    const double omega = sc0[S_OMEGA];
     const int ld = c.ld;
     double* X = plane(b, c, P_PCOR);
     const LevelDev& L = c.lev[0];
@@ -493,25 +449,7 @@ __global__ void __launch_bounds__(NT, 5) k_bicg_x(BatchDev b, int maxit) {
         red[0] += q[h] * r;
         red[1] += fabs(r);
     }
-    if (case_reduce<2, 0u>(b, t.c, blockIdx.x, c.jt_begin, c.jt_count, red) && threadIdx.x == 0) {
-        double* sc = b.scal + (long long)t.c * NSCAL;
-        int* is = b.iscal + (long long)t.c * NISCAL;
-        const int it = ++is[I_PIT];
-        const double rho_new = red[0];
-        sc[S_RL1] = red[1];
-        const bool conv = red[1] <= c.tol_p * sc[S_NB1] || red[1] <= c.atol_p;
-        bool stop = conv;
-        if (!isfinite(red[1])) { is[I_STATUS] |= ST_NAN; stop = true; }
-        else if (!conv && (omega == 0.0 || rho_new == 0.0)) { is[I_PSTATUS] |= ST_BREAKDOWN; stop = true; }
-        else if (!conv && it >= maxit) { is[I_PSTATUS] |= ST_MAXITER; stop = true; }
-        if (!stop) {
-            sc[S_BETA] = (rho_new / sc[S_RHO]) * (alpha / omega);
-            sc[S_RHO] = rho_new;
-        } else {
-            is[I_PDONE] = 1;
-            atomicSub(b.active, 1);
-        }
-    }
+    tile_partial<2, 0u>(b, blockIdx.x, 0, red);
 }
 
 // ---------------------------------------------------------------------------
@@ -601,7 +539,7 @@ __global__ void __launch_bounds__(MG_GS_THREADS, 8) k_mg_gs(BatchDev b, int l, i
 }
 
 // coarsest level: `sweeps` multicolour GS sweeps by one CTA per case (mg_coarse_solve)
-constexpr int MGC_THREADS = 1024, MGC_SMEM = 12000;
+constexpr int MGC_THREADS = 1024, MGC_SMEM = 12000;  // x of the level: 46.9 KB
 __global__ void __launch_bounds__(MGC_THREADS) k_mg_coarse(BatchDev b, int l, int sweeps) {
     __shared__ float xs[MGC_SMEM];
     // l < 0: one launch for every case, each on its own coarsest level (the case lists of
@@ -685,8 +623,7 @@ __global__ void __launch_bounds__(NT, 4) k_correct(BatchDev b) {
         // record the boundary pcor (output only)
         correct_bnd(PC, ld, W, per, cav, n0, n1, i, j, pc, far);
     }
-    if (case_reduce<1, 0u>(b, t.c, blockIdx.x, c.jt_begin, c.jt_count, red) && threadIdx.x == 0)
-        b.scal[(long long)t.c * NSCAL + S_DUL1] = red[0];
+    tile_partial<1, 0u>(b, blockIdx.x, 3, red);  // column 3: k_diag has 0 .. 2, one k_fin sums all
 }
 
 // ---------------------------------------------------------------------------
@@ -799,17 +736,117 @@ __global__ void __launch_bounds__(NT, 3) k_diag(BatchDev b) {
         red[1] += dT;
         red[2] = fmax(red[2], dT);
     }
-    if (case_reduce<3, 0x5u>(b, t.c, blockIdx.x, c.jt_begin, c.jt_count, red) && threadIdx.x == 0) {
-        double* sc = b.scal + (long long)t.c * NSCAL;
-        int* is = b.iscal + (long long)t.c * NISCAL;
+    tile_partial<3, 0x5u>(b, blockIdx.x, 0, red);
+}
+
+// The case's totals of the tile kernel just launched and what follows from them: one CTA per
+// case. `maxit` is the pressure solve's cap.
+template <int WHAT>
+__device__ __forceinline__ void fin_case(const BatchDev& b, int cid, int maxit) {
+    const CaseDev& c = b.cases[cid];
+    int* is = b.iscal + (long long)cid * NISCAL;
+    double* sc = b.scal + (long long)cid * NSCAL;
+    if (WHAT == FIN_FACE_Q || WHAT == FIN_STEP) {
+        if (!is[I_ACTIVE]) return;
+    } else if (is[I_PDONE]) {
+        return;
+    }
+    const int tb = c.jt_begin, tn = c.jt_count;
+    if constexpr (WHAT == FIN_FACE_Q) {
+        double red[3];
+        case_total<3, 0x4u>(b, tb, tn, red);
+        if (threadIdx.x != 0) return;
+        sc[S_QL1] = red[0];
+        sc[S_QL2] = sqrt(red[1]);
+        if (is[I_NSTEP] == 0) sc[S_QL2_0] = sqrt(red[1]);
+        sc[S_QMAX] = red[2];
+        sc[S_RHO] = red[1];
+        sc[S_ALPHA] = 1.0;
+        sc[S_OMEGA] = 1.0;
+        sc[S_BETA] = 0.0;
+        sc[S_NB1] = red[0];
+        sc[S_RL1] = red[0];
+        is[I_PIT] = 0;
+        // this step's solver status starts with the momentum / energy solves: a field still
+        // iterating when their loop ended stopped at the sweep cap
+        is[I_PSTATUS] = (is[I_MWORD] & ((1 << NFIELD) - 1)) ? ST_MAXITER : 0;
+        if (red[0] == 0.0 || !isfinite(red[0])) {
+            is[I_PDONE] = 1;
+            if (!isfinite(red[0])) is[I_STATUS] |= ST_NAN;
+        } else {
+            is[I_PDONE] = 0;
+            atomicAdd(b.active, 1);
+        }
+    } else if constexpr (WHAT == FIN_SPMV0) {
+        double red[1];
+        case_total<1, 0u>(b, tb, tn, red);
+        if (threadIdx.x != 0) return;
+        if (red[0] == 0.0 || !isfinite(red[0])) {
+            is[I_PSTATUS] |= ST_BREAKDOWN;
+            is[I_PDONE] = 1;
+            atomicSub(b.active, 1);
+        } else {
+            sc[S_ALPHA] = sc[S_RHO] / red[0];
+        }
+    } else if constexpr (WHAT == FIN_SPMV1) {
+        double red[2];
+        case_total<2, 0u>(b, tb, tn, red);
+        if (threadIdx.x == 0) sc[S_OMEGA] = red[1] > 0.0 ? red[0] / red[1] : 0.0;
+    } else if constexpr (WHAT == FIN_BICG_S) {
+        double red[1];
+        case_total<1, 0u>(b, tb, tn, red);
+        if (threadIdx.x != 0) return;
+        const bool conv = red[0] <= c.tol_p * sc[S_NB1] || red[0] <= c.atol_p;
+        if (conv || !isfinite(red[0])) {
+            is[I_PIT] += 1;
+            sc[S_RL1] = red[0];
+            if (!isfinite(red[0])) is[I_STATUS] |= ST_NAN;
+            is[I_PDONE] = 1;
+            atomicSub(b.active, 1);
+        }
+    } else if constexpr (WHAT == FIN_BICG_X) {
+        double red[2];
+        case_total<2, 0u>(b, tb, tn, red);
+        if (threadIdx.x != 0) return;
+        const double alpha = sc[S_ALPHA], omega = sc[S_OMEGA];
+        const int it = ++is[I_PIT];
+        const double rho_new = red[0];
+        sc[S_RL1] = red[1];
+        const bool conv = red[1] <= c.tol_p * sc[S_NB1] || red[1] <= c.atol_p;
+        bool stop = conv;
+        if (!isfinite(red[1])) { is[I_STATUS] |= ST_NAN; stop = true; }
+        else if (!conv && (omega == 0.0 || rho_new == 0.0)) { is[I_PSTATUS] |= ST_BREAKDOWN; stop = true; }
+        else if (!conv && it >= maxit) { is[I_PSTATUS] |= ST_MAXITER; stop = true; }
+        if (!stop) {
+            sc[S_BETA] = (rho_new / sc[S_RHO]) * (alpha / omega);
+            sc[S_RHO] = rho_new;
+        } else {
+            is[I_PDONE] = 1;
+            atomicSub(b.active, 1);
+        }
+    } else {  // the step's residuals: k_diag's columns 0 .. 2, k_correct's 3
+        double red[4];
+        case_total<4, 0x5u>(b, tb, tn, red);
+        if (threadIdx.x != 0) return;
         sc[S_DMAX] = fmax(red[0], 0.0);
         sc[S_DTL1] = red[1];
         sc[S_DTMAX] = red[2];
+        sc[S_DUL1] = red[3];
         // steady residual: mean (|du| + |dv| + |dT|) / dt over the unknown cells
         const double ncell = (double)(c.ihi - c.ilo + 1) * (c.n1 - 2);
-        sc[S_SR] = (sc[S_DUL1] + red[1]) / (c.dt * ncell);
+        sc[S_SR] = (red[3] + red[1]) / (c.dt * ncell);
         if (is[I_NSTEP] == 0) sc[S_SR0] = sc[S_SR];
         is[I_NSTEP] += 1;
+    }
+}
+__global__ void __launch_bounds__(NT) k_fin(BatchDev b, FinKernel what, int maxit) {
+    switch (what) {
+        case FIN_FACE_Q: fin_case<FIN_FACE_Q>(b, blockIdx.x, maxit); break;
+        case FIN_SPMV0: fin_case<FIN_SPMV0>(b, blockIdx.x, maxit); break;
+        case FIN_SPMV1: fin_case<FIN_SPMV1>(b, blockIdx.x, maxit); break;
+        case FIN_BICG_S: fin_case<FIN_BICG_S>(b, blockIdx.x, maxit); break;
+        case FIN_BICG_X: fin_case<FIN_BICG_X>(b, blockIdx.x, maxit); break;
+        case FIN_STEP: fin_case<FIN_STEP>(b, blockIdx.x, maxit); break;
     }
 }
 

@@ -12,7 +12,9 @@ __global__ void k_face_q(BatchDev b);
 __global__ void k_bicg_p(BatchDev b);
 __global__ void k_spmv(BatchDev b, int mode);
 __global__ void k_bicg_s(BatchDev b);
-__global__ void k_bicg_x(BatchDev b, int maxit);
+__global__ void k_bicg_x(BatchDev b);
+enum FinKernel { FIN_FACE_Q, FIN_SPMV0, FIN_SPMV1, FIN_BICG_S, FIN_BICG_X, FIN_STEP };
+__global__ void k_fin(BatchDev b, FinKernel what, int maxit);
 __global__ void k_mg_gs(BatchDev b, int l, int mode, int src, int dst, int inner);
 constexpr int MG_GS_THREADS = 128;  // k_mg_gs: one thread per 2 x 2 block of a 32 x 16 tile
 __global__ void k_mg_rr(BatchDev b, int l, int src);

@@ -153,7 +153,7 @@ __device__ __forceinline__ void group_reduce(double (&v)[NV], double* smem, cons
 }
 
 // The case's totals from its tiles' partial rows (row t at part + t * PSTRIDE), in thread 0: the
-// sum case_reduce() and k_sweep_fin form with `nthr` threads. The threads above add nothing
+// sum k_fin and k_sweep_fin form with `nthr` threads. The threads above add nothing
 // (adding their zeros changes no bit); up to 32 rows one warp holds every term, and the
 // block's second stage would only add zeros to its sum.
 template <int NV, unsigned MAXMASK>
