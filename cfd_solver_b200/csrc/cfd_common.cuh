@@ -182,6 +182,15 @@ struct BatchDev {
     int mg_res;            // multigrid plane (M_X or M_R) holding a non-coarsest level's V-cycle result
 };
 
+// First statement of every kernel of the step graph. Its launch may begin while the kernel before
+// it drains (a programmatic edge): the CTAs are scheduled as slots come free and wait here
+// until that kernel has completed and its writes are visible. Every CTA of every such kernel
+// waits, so a completed kernel implies that all before it have completed.
+__device__ __forceinline__ void after_previous() {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // ------------------------------------------------------------------------
 __device__ __forceinline__ double* plane(const BatchDev& b, const CaseDev& c, int k) {
     return b.f64 + c.base + (long long)k * c.ps + H;

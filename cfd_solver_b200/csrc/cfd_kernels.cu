@@ -101,6 +101,7 @@ const size_t kRhsSmem = RHS_SMEM;
 // registers left the SM idle between a CTA's copies and its arithmetic (431 vs 373 us per
 // step on the 256-case twin sweep).
 __global__ void __launch_bounds__(NT, 3) k_rhs(BatchDev b) {
+    after_previous();
     extern __shared__ __align__(128) unsigned char rraw[];
     __shared__ __align__(8) uint64_t bar;
     double* sm = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(rraw) + 127) & ~uintptr_t(127));
@@ -189,6 +190,7 @@ __global__ void __launch_bounds__(NT, 3) k_rhs(BatchDev b) {
 // ---------------------------------------------------------------------------
 // up/vp far-field condition (PSolver.cpp:1356-1382), one CTA per O-grid case
 __global__ void __launch_bounds__(BC_THREADS) k_upbc(BatchDev b) {
+    after_previous();
     const CaseDev& c = b.cases[blockIdx.x];
     if (c.profile != OGRID || !b.iscal[(long long)blockIdx.x * NISCAL + I_ACTIVE]) return;
     const int ld = c.ld, j = c.n1 - 1, nxt = b.cur ^ 1;
@@ -222,6 +224,7 @@ constexpr size_t FQ_SMEM = (size_t)FQ_HALO * JTW * JTH * sizeof(double) + 128;
 const size_t kFaceQSmem = FQ_SMEM;
 
 __global__ void __launch_bounds__(NT, 4) k_face_q(BatchDev b) {
+    after_previous();
     extern __shared__ __align__(128) unsigned char fraw[];
     __shared__ __align__(8) uint64_t bar;
     double* sm = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(fraw) + 127) & ~uintptr_t(127));
@@ -283,6 +286,7 @@ __global__ void __launch_bounds__(NT, 4) k_face_q(BatchDev b) {
 // The BiCGStab kernels run on the 32 x 16 tiles, two cells per thread (rows lj and
 // lj + 8), every load of both cells issued before the arithmetic.
 __global__ void __launch_bounds__(NT, 3) k_bicg_p(BatchDev b) {
+    after_previous();
     const Tile t = b.jtiles[blockIdx.x];
     if (b.iscal[(long long)t.c * NISCAL + I_PDONE]) return;
     // p_{k+1} = r_k + beta (p_k - omega v_k), launched at the end of iteration k (after
@@ -325,6 +329,7 @@ __global__ void __launch_bounds__(NT, 3) k_bicg_p(BatchDev b) {
 // y = A * x with x = (double) MG level-0 result; mode 0: p_hat, v, (r_hat, v) -> alpha
 //                                               mode 1: s_hat, t, (t, s), (t, t) -> omega
 __global__ void __launch_bounds__(NT, 5) k_spmv(BatchDev b, int mode) {
+    after_previous();
     const Tile t = b.jtiles[blockIdx.x];
     if (b.iscal[(long long)t.c * NISCAL + I_PDONE]) return;
     const CaseDev& c = b.cases[t.c];
@@ -373,6 +378,7 @@ __global__ void __launch_bounds__(NT, 5) k_spmv(BatchDev b, int mode) {
 // the solve ends here (the standard early exit: x + alpha p_hat is the iterate whose
 // residual is s) and the second preconditioner application of the iteration is skipped
 __global__ void __launch_bounds__(NT, 5) k_bicg_s(BatchDev b) {
+    after_previous();
     const Tile t = b.jtiles[blockIdx.x];
     if (b.iscal[(long long)t.c * NISCAL + I_PDONE]) return;
     const bool first = b.iscal[(long long)t.c * NISCAL + I_PIT] == 0;
@@ -412,6 +418,7 @@ __global__ void __launch_bounds__(NT, 5) k_bicg_s(BatchDev b) {
 }
 
 __global__ void __launch_bounds__(NT, 5) k_bicg_x(BatchDev b) {
+    after_previous();
     const Tile t = b.jtiles[blockIdx.x];
     if (b.iscal[(long long)t.c * NISCAL + I_PDONE]) return;
     const CaseDev& c = b.cases[t.c];
@@ -469,6 +476,7 @@ __global__ void __launch_bounds__(NT, 5) k_bicg_x(BatchDev b) {
 // in shared memory, then full-weighting restriction into b_{l+1} (tiles of level l + 1;
 // levels start from x = 0 on their own). Fine points that are not unknowns contribute 0.
 __global__ void __launch_bounds__(NT) k_mg_rr(BatchDev b, int l, int src) {
+    after_previous();
     constexpr int RW = 2 * TX + 1, RH = 2 * TY + 1;  // fine residual region
     constexpr int XW = RW + 2, XH = RH + 2;          // fine x region (one-cell halo)
     __shared__ float xs[XH * XW];
@@ -521,6 +529,7 @@ __global__ void __launch_bounds__(NT) k_mg_rr(BatchDev b, int l, int src) {
 // pre-smoothing folded into the residual + restriction pass (mg_prr_tile): one CTA per
 // 32 x 8 tile of level l + 1
 __global__ void __launch_bounds__(MG_PRR_THREADS, 3) k_mg_prr(BatchDev b, int l, int dst, int inner) {
+    after_previous();
     __shared__ float xs[2 * MPR_XP];
     __shared__ float rs[2 * MPR_RP];
     const Tile t = b.atiles[l + 1][blockIdx.x];
@@ -531,6 +540,7 @@ __global__ void __launch_bounds__(MG_PRR_THREADS, 3) k_mg_prr(BatchDev b, int l,
 
 // multicolour Gauss-Seidel sweeps of level l on a 32 x 16 tile (mg_gs_tile)
 __global__ void __launch_bounds__(MG_GS_THREADS, 8) k_mg_gs(BatchDev b, int l, int mode, int src, int dst, int inner) {
+    after_previous();
     __shared__ float xs[2 * MG_GS_XP];
     const Tile t = b.mtiles[l][blockIdx.x];
     if (b.iscal[(long long)t.c * NISCAL + I_PDONE]) return;
@@ -541,6 +551,7 @@ __global__ void __launch_bounds__(MG_GS_THREADS, 8) k_mg_gs(BatchDev b, int l, i
 // coarsest level: `sweeps` multicolour GS sweeps by one CTA per case (mg_coarse_solve)
 constexpr int MGC_THREADS = 1024, MGC_SMEM = 12000;  // x of the level: 46.9 KB
 __global__ void __launch_bounds__(MGC_THREADS) k_mg_coarse(BatchDev b, int l, int sweeps) {
+    after_previous();
     __shared__ float xs[MGC_SMEM];
     // l < 0: one launch for every case, each on its own coarsest level (the case lists of
     // all levels are stored back to back from ccases[0])
@@ -564,6 +575,7 @@ __global__ void __launch_bounds__(NT) k_mg_galerkin(BatchDev b, int l, int toff)
 // pcor boundary conditions + velocity / pressure correction (PSolver.cpp:1471-1542);
 // also the momentum part of the steady residual, sum |u^{n+1} - u^n| + |v^{n+1} - v^n|
 __global__ void __launch_bounds__(NT, 4) k_correct(BatchDev b) {
+    after_previous();
     // a 32 x 16 tile, two cells per thread (rows lj and lj + 8): every load of both cells
     // is issued before any arithmetic
     const Tile t = b.jtiles[blockIdx.x];
@@ -630,6 +642,7 @@ __global__ void __launch_bounds__(NT, 4) k_correct(BatchDev b) {
 // boundary update, boundary pressure and wall integrals: one CTA per case
 // (O-grid: PSolver.cpp:1549-1783 and 1855-1983; cavity: this project's walls)
 __global__ void __launch_bounds__(BC_THREADS, 2) k_bc(BatchDev b) {
+    after_previous();
     const int cid = blockIdx.x;
     const CaseDev& c = b.cases[cid];
     if (!b.iscal[(long long)cid * NISCAL + I_ACTIVE]) return;
@@ -694,6 +707,7 @@ __global__ void __launch_bounds__(BC_THREADS, 2) k_bc(BatchDev b) {
 // ---------------------------------------------------------------------------
 // dilatation, interior vorticity, dmax and the energy residual (PSolver.cpp:1807-1853)
 __global__ void __launch_bounds__(NT, 3) k_diag(BatchDev b) {
+    after_previous();
     // a 32 x 16 tile, two cells per thread; all loads of both cells first
     const Tile t = b.jtiles[blockIdx.x];
     const CaseDev& c = b.cases[t.c];
@@ -840,6 +854,7 @@ __device__ __forceinline__ void fin_case(const BatchDev& b, int cid, int maxit) 
     }
 }
 __global__ void __launch_bounds__(NT) k_fin(BatchDev b, FinKernel what, int maxit) {
+    after_previous();
     switch (what) {
         case FIN_FACE_Q: fin_case<FIN_FACE_Q>(b, blockIdx.x, maxit); break;
         case FIN_SPMV0: fin_case<FIN_SPMV0>(b, blockIdx.x, maxit); break;

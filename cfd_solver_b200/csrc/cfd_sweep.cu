@@ -166,8 +166,8 @@ __device__ __forceinline__ void sweep_tile(const BatchDev& b, unsigned char* sm,
     // (FP64 form), and the sweeps done (the same for every still-active field of the case)
     const int word = b.tword[blockIdx.x];
     const int mask = word & ((1 << NFIELD) - 1);
-    if (mask == 0) return;  // uniform over the case's CTAs
     const int sweep = word >> (2 * NFIELD);
+    if (mask == 0) return;  // uniform over the case's CTAs
     const int flipm = MODE == SW_F64 ? (word >> NFIELD) & ((1 << NFIELD) - 1) : 0;
     const int tid = threadIdx.x, lane = tid & 31, wrp = tid >> 5;
     const int nxt = b.cur ^ 1;
@@ -354,6 +354,7 @@ __device__ __forceinline__ void sweep_tile(const BatchDev& b, unsigned char* sm,
 }  // namespace
 
 __global__ void __launch_bounds__(SW_THREADS, 4) k_sweep_f64(BatchDev b) {
+    after_previous();
     extern __shared__ __align__(128) unsigned char swraw[];
     __shared__ __align__(8) uint64_t bar[2];
     unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(swraw) + 127) & ~uintptr_t(127));
@@ -363,6 +364,7 @@ __global__ void __launch_bounds__(SW_THREADS, 4) k_sweep_f64(BatchDev b) {
 // precision form, the step's first sweep (every still-iterating field of every case starts
 // at sweep 0 together): the FP64 residual r = rhs - A x0 and the first FP32 correction
 __global__ void __launch_bounds__(SW_THREADS, 4) k_sweep_mx0(BatchDev b) {
+    after_previous();
     extern __shared__ __align__(128) unsigned char swraw[];
     __shared__ __align__(8) uint64_t bar[2];
     unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(swraw) + 127) & ~uintptr_t(127));
@@ -373,6 +375,7 @@ __global__ void __launch_bounds__(SW_THREADS, 4) k_sweep_mx0(BatchDev b) {
 // sweep it needs 80 registers and no spills, so six CTAs (37 KB of shared memory each)
 // share an SM instead of four
 __global__ void __launch_bounds__(SW_THREADS, 6) k_sweep_mx1(BatchDev b) {
+    after_previous();
     extern __shared__ __align__(128) unsigned char swraw[];
     __shared__ __align__(8) uint64_t bar[2];
     unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(swraw) + 127) & ~uintptr_t(127));
@@ -460,6 +463,7 @@ __device__ __forceinline__ int fin_case(const BatchDev& b, int cid, int* is, int
 // tile of the case the sweep kernel's new word (the stores spread over the CTA's threads:
 // a 1025 x 1025 case has 2,048 tiles)
 __global__ void __launch_bounds__(SWF_THREADS) k_sweep_fin(BatchDev b) {
+    after_previous();
     __shared__ double red[NFIELD * 32];
     __shared__ int s_word;
     const int cid = blockIdx.x;
@@ -495,6 +499,7 @@ size_t sweep_smem_mx1() { return (size_t)SwLayout<SW_MX>::TOTAL + 128; }
 // the other parity than predicted): copy it into the iterate plane. 32 x 16 tiles, two
 // cells per thread; the CTAs of a case with no such solve leave at once.
 __global__ void __launch_bounds__(NT) k_mom_fix(BatchDev b) {
+    after_previous();
     const Tile t = b.jtiles[blockIdx.x];
     const int* is = b.iscal + (long long)t.c * NISCAL;
     int odd = 0;  // solves whose result is in the scratch plane: stopped there, or ran to the
@@ -518,6 +523,7 @@ __global__ void __launch_bounds__(NT) k_mom_fix(BatchDev b) {
 }
 
 __global__ void __launch_bounds__(NT) k_mom_update(BatchDev b) {
+    after_previous();
     const Tile t = b.ftiles[blockIdx.x];
     const CaseDev& c = b.cases[t.c];
     if (!b.iscal[(long long)t.c * NISCAL + I_ACTIVE]) return;  // uniform over the case
