@@ -699,38 +699,38 @@ void enq_begin(cfd_batch* b, BatchDev& bd) {
     Prof pr(b, K_RHS);
     go(b, k_rhs, bd.njtiles, NT, kRhsSmem, bd);
 }
-// FP64 form: sweeps in pairs (the iterates ping-pong between two planes)
-void enq_mom_pair(cfd_batch* b, BatchDev& bd) {
-    for (int s = 0; s < 2; s++) {
-        {
-            Prof pr(b, K_SWEEP);
-            go(b, k_sweep_f64, b->sw_grid, SW_THREADS, b->sw_smem, bd);
-        }
-        Prof pr(b, K_SWEEP_FIN);
-        go(b, k_sweep_fin, b->n, b->swf_threads, 0, bd);
-    }
-}
-// precision form: the step's first sweep (FP64 residual, k_sweep_mx0), then one FP32
-// sweep (k_sweep_mx1) per loop iteration
-void enq_mom_mx_first(cfd_batch* b, BatchDev& bd) {
+// one sweep of the momentum / energy solves and its bookkeeping
+void enq_sweep(cfd_batch* b, BatchDev& bd, void (*kernel)(BatchDev), size_t smem) {
     {
         Prof pr(b, K_SWEEP);
-        go(b, k_sweep_mx0, b->sw_grid, SW_THREADS, b->sw_smem, bd);
+        go(b, kernel, b->sw_grid, SW_THREADS, smem, bd);
     }
     Prof pr(b, K_SWEEP_FIN);
     go(b, k_sweep_fin, b->n, b->swf_threads, 0, bd);
 }
-void enq_mom_mx_next(cfd_batch* b, BatchDev& bd) {
-    {
-        Prof pr(b, K_SWEEP);
-        go(b, k_sweep_mx1, b->sw_grid, SW_THREADS, b->sw_smem1, bd);
-    }
-    Prof pr(b, K_SWEEP_FIN);
-    go(b, k_sweep_fin, b->n, b->swf_threads, 0, bd);
+// the precision form's first sweep (FP64 residual); its later ones are FP32
+void enq_mom_first(cfd_batch* b, BatchDev& bd) {
+    if (b->precision == CFD_PRECISION_MIXED) enq_sweep(b, bd, k_sweep_mx0, b->sw_smem);
 }
-// loop iterations that bound the momentum / energy solves at maxit_mom sweeps
+// The sweeps of one loop body. An iteration of a graph loop costs 6.3 us beside its kernels (the
+// condition kernel and the loop node); a sweep that finds every case done costs 3 us and 2 ns
+// per tile. FP64 solves start at an iterate that takes 3-4 sweeps on the O-grids and 12 on the
+// cavities: bodies of 2 / 4 give 1403 / 1399 us per step of 100 O-grids, 2386 / 2357 of 100 cavities.
+// In the precision form the first sweep is outside the loop and the O-grids need 2 more: bodies of
+// 1 / 2 / 4 give 1407 / 1406 / 1416 and 2250 / 2211 / 2200.
+int mom_body(const cfd_batch* b) { return b->precision == CFD_PRECISION_MIXED ? 2 : 4; }
+void enq_mom_next(cfd_batch* b, BatchDev& bd) {
+    const bool mixed = b->precision == CFD_PRECISION_MIXED;
+    for (int s = mom_body(b); s > 0; s--)
+        enq_sweep(b, bd, mixed ? k_sweep_mx1 : k_sweep_f64, mixed ? b->sw_smem1 : b->sw_smem);
+}
+// sweeps of a step at most (FP64 form: an even number), and the loop iterations that hold them
+int mom_cap(const cfd_batch* b) {
+    return b->precision == CFD_PRECISION_MIXED ? std::max(2, b->maxit_mom) : 2 * std::max(1, b->maxit_mom / 2);
+}
 int mom_loop_cap(const cfd_batch* b) {
-    return b->precision == CFD_PRECISION_MIXED ? std::max(1, b->maxit_mom - 1) : std::max(1, b->maxit_mom / 2);
+    const int n = mom_cap(b) - (b->precision == CFD_PRECISION_MIXED);
+    return (n + mom_body(b) - 1) / mom_body(b);
 }
 // the totals of the tile kernel just launched
 void enq_fin(cfd_batch* b, BatchDev& bd, FinKernel what) {
@@ -793,21 +793,15 @@ int one_step_direct(cfd_batch* b) {
     BatchDev& bd = b->bd;
     bd.cur = b->cur;
     enq_begin(b, bd);
-    // momentum / energy solves: sweeps (in pairs in the FP64 form) until every (case, field)
-    // stopped; the counter is read every second loop iteration (a finished case's CTAs
-    // leave at once)
-    const bool mixed = b->precision == CFD_PRECISION_MIXED;
-    if (mixed) enq_mom_mx_first(b, bd);
-    const int npairs = mom_loop_cap(b);
-    for (int pair = 0; pair < npairs; pair++) {
-        if (mixed) enq_mom_mx_next(b, bd);
-        else enq_mom_pair(b, bd);
-        if (pair % 2 == 1 || pair == npairs - 1) {
-            int m = 0;
-            int rc = read_flag(b, 1, &m);
-            if (rc) return rc;
-            if (m <= 0) break;
-        }
+    // momentum / energy solves: sweeps until every (case, field) stopped; the counter is read
+    // after every loop body (a finished case's CTAs leave at once)
+    enq_mom_first(b, bd);
+    for (int it = mom_loop_cap(b); it > 0; it--) {
+        enq_mom_next(b, bd);
+        int m = 0;
+        int rc = read_flag(b, 1, &m);
+        if (rc) return rc;
+        if (m <= 0) break;
     }
     enq_mid(b, bd);
     // pressure correction: the first iteration is launched without a check (a case whose
@@ -918,16 +912,12 @@ int build_step_graph(cfd_batch* b, int cur) {
         prev = n;
         return CFD_OK;
     };
-    const bool mixed = b->precision == CFD_PRECISION_MIXED;
     int rc = child([&] {
         enq_begin(b, bd);
-        if (mixed) enq_mom_mx_first(b, bd);
+        enq_mom_first(b, bd);
     });
     const long long la = b->launches;
-    if (!rc) rc = loop([&] {
-        if (mixed) enq_mom_mx_next(b, bd);
-        else enq_mom_pair(b, bd);
-    }, b->flags + 1, b->flags + 2, mom_loop_cap(b), b->flags + 5);
+    if (!rc) rc = loop([&] { enq_mom_next(b, bd); }, b->flags + 1, b->flags + 2, mom_loop_cap(b), b->flags + 5);
     const long long lm = b->launches;
     if (!rc) rc = child([&] { enq_mid(b, bd); });
     const long long lp0 = b->launches;
@@ -979,7 +969,7 @@ int team_steps(cfd_batch* b, int nsteps) {
     a.nr = b->team_nr;
     a.cluster = b->team_cluster;
     a.nsteps = nsteps;
-    a.sweep_cap = b->precision == CFD_PRECISION_MIXED ? 1 + mom_loop_cap(b) : 2 * mom_loop_cap(b);
+    a.sweep_cap = b->bd.mom_cap;
     a.maxit_p = a.p_iters = b->maxit_p;
     a.fin_threads = b->swf_threads;
     a.nu_pre = b->mg_pre;
@@ -1347,6 +1337,7 @@ int build_tables(cfd_batch* b, const std::vector<int>& ids) {
         bd.ccases[l] = b->dcc + pos_cc[l]; bd.nccases[l] = (int)cc[l].size();
     }
     if (int rc = plan_team(b, ids)) return rc;
+    bd.mom_cap = mom_cap(b);
     b->ntable_cases = (int)ids.size();
     b->sw_grid = (int)jtiles.size();  // one CTA per 32 x 16 tile
     b->swf_threads = jt_max >= 1024 ? SWF_THREADS : 128;

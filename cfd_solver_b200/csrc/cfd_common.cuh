@@ -161,6 +161,7 @@ struct BatchDev {
     double* partial;       // reduction partials: rows of 8 per tile
     int* active;           // global count of cases still iterating (pressure)
     int* mactive;          // global count of (case, field) pairs still iterating (momentum)
+    int mom_cap;           // momentum / energy sweeps of a step at most
     int* error;            // set when a bounded wait in a kernel gives up
     unsigned wait_polls;   // polls of a kernel's bounded mbarrier waits before they give up
     int mixed;             // 1: the precision form (momentum iterates are FP32 corrections)

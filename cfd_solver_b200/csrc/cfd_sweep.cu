@@ -167,7 +167,7 @@ __device__ __forceinline__ void sweep_tile(const BatchDev& b, unsigned char* sm,
     const int word = b.tword[blockIdx.x];
     const int mask = word & ((1 << NFIELD) - 1);
     const int sweep = word >> (2 * NFIELD);
-    if (mask == 0) return;  // uniform over the case's CTAs
+    if (mask == 0 || sweep >= b.mom_cap) return;  // uniform over the case's CTAs
     const int flipm = MODE == SW_F64 ? (word >> NFIELD) & ((1 << NFIELD) - 1) : 0;
     const int tid = threadIdx.x, lane = tid & 31, wrp = tid >> 5;
     const int nxt = b.cur ^ 1;
@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(SWF_THREADS) k_sweep_fin(BatchDev b) {
     const CaseDev& c = b.cases[cid];
     int* is = b.iscal + (long long)cid * NISCAL;
     const int word = is[I_MWORD];
-    if (!(word & ((1 << NFIELD) - 1))) return;
+    if (!(word & ((1 << NFIELD) - 1)) || (word >> (2 * NFIELD)) >= b.mom_cap) return;
     const int tid = threadIdx.x;
     FinIn in;
     if (tid == 0) fin_load(b, c, cid, in);
