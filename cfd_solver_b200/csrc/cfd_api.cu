@@ -2078,10 +2078,13 @@ static int state_copy(cfd_batch* b, void* host, size_t bytes, bool to_host) {
     // per-case offsets into the image (a slot pool's cases change with admissions)
     std::vector<long long> off(b->n);
     long long o = 0;
+    int max_n1 = 1;
     for (int c = 0; c < b->n; c++) {
         off[c] = o;
         o += state_doubles(b->hc[c]);
+        max_n1 = std::max(max_n1, b->hc[c].n1);
     }
+    const dim3 pack(b->n * 7, (max_n1 + STATE_ROWS - 1) / STATE_ROWS);
     if (need > b->stage_bytes) {
         CK(cudaStreamSynchronize(b->st));
         cudaFree(b->stage);
@@ -2094,12 +2097,12 @@ static int state_copy(cfd_batch* b, void* host, size_t bytes, bool to_host) {
     CK(cudaMemcpyAsync(b->stage_off, off.data(), sizeof(long long) * b->n, cudaMemcpyHostToDevice, b->st));
     b->bd.cur = b->cur;
     if (to_host) {
-        k_state_pack<<<b->n * 7, 256, 0, b->st>>>(b->bd, b->stage, b->stage_off, 1);
+        k_state_pack<<<pack, 256, 0, b->st>>>(b->bd, b->stage, b->stage_off, 1);
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(host, b->stage, need, cudaMemcpyDeviceToHost, b->st));
     } else {
         CK(cudaMemcpyAsync(b->stage, host, need, cudaMemcpyHostToDevice, b->st));
-        k_state_pack<<<b->n * 7, 256, 0, b->st>>>(b->bd, b->stage, b->stage_off, 0);
+        k_state_pack<<<pack, 256, 0, b->st>>>(b->bd, b->stage, b->stage_off, 0);
         CK(cudaGetLastError());
     }
     CK(cudaStreamSynchronize(b->st));
