@@ -1195,19 +1195,22 @@ int grow(T*& ptr, size_t& cap, size_t need) {
 // The teams of all cases run at the same time (one CTA per SM), so a team gets 1 / n of the chip:
 // as a cluster, the largest power of two up to 16 that n clusters of leave room for, or as a
 // share of a cooperative grid. A step costs a team about 80 us (FP64 form) plus 14 us per
-// 32 x 16 tile and CTA of the largest case, the step graph 160 us plus 0.25 us per tile of the
-// batch, with less to gain the more of the chip the work fills. Measured, us per step, graph
-// against team:
-//   O-grids, 1 case:   65^2 169 / 90, 129^2 166 / 105, 257^2 197 / 121, 513^2 300 / 241 (3.5
-//                      tiles per CTA), 1025^2 672 / 698 (13.8)
-//   n cases:           16 x 33^2 169 / 82, 128 x 33^2 201 / 123, 64 x 65^2 252 / 188, 128 x 65^2
-//                      355 / 318 (8), 16 x 193^2 373 / 331 (8), 64 x 129^2 506 / 550 (16),
-//                      4 x 513^2 598 / 612 (13.8); a second wave of teams loses (256 x 65^2 558 / 630)
-//   cavities, mixed:   65^2 273 / 129, 257^2 319 / 203, 16 x 129^2 478 / 358, 64 x 129^2 901 / 1151 (16)
-// so teams run when they all fit at once and have at most 8 tiles per CTA. A cluster's barrier
-// is quicker than a counter's, but its size is a power of two: with more than two tiles per CTA
-// the larger share of a grid pays (16 x 129^2: clusters of 4 266, grid shares of 9 192).
-constexpr int kTeamTilesPerCta = 8;
+// 32 x 16 tile and CTA of the largest case; the step graph starts higher and gains as the work
+// fills the chip, and a large team's barriers cost more. Measured, us per step, graph / team
+// (tiles per CTA of teams of so many CTAs):
+//   O-grids, FP64:     65^2 169 / 90, 129^2 166 / 105, 257^2 197 / 121, 513^2 269 / 256 (4 of 148),
+//                      577^2 341 / 346 (5 of 148), 737^2 387 / 421 (8 of 148), 2 x 385^2 267 / 249 (4 of 74),
+//                      2 x 417^2 299 / 304 (5 of 74), 16 x 161^2 288 / 273 (6 of 9), 16 x 193^2 329 / 342
+//                      (8 of 9), 36 x 129^2 310 / 302 (8 of 4), 148 x 65^2 368 / 327 (8 of 1),
+//                      64 x 129^2 506 / 550 (16 of 2); a second wave of teams: 256 x 65^2 558 / 630
+//   cavities, FP64:    577^2 925 / 960 (5 of 148), 8 x 225^2 588 / 591 (6 of 18), 8 x 257^2 660 / 700 (8 of 18),
+//                      24 x 129^2 458 / 427 (6 of 6), 36 x 129^2 531 / 525 (8 of 4)
+//   cavities, mixed:   65^2 273 / 129, 513^2 692 / 558 (4 of 148), 2 x 417^2 639 / 678 (5 of 74),
+//                      16 x 161^2 468 / 468 (6 of 9), 36 x 129^2 524 / 495 (8 of 4), 64 x 129^2 901 / 1151 (16 of 2)
+// so teams run when they all fit at once and have at most team_tiles() tiles per CTA. A cluster's
+// barrier is quicker than a counter's, but its size is a power of two: with more than two tiles
+// per CTA the larger share of a grid pays (16 x 129^2: clusters of 4 266, grid shares of 9 192).
+int team_tiles(int nr) { return nr > 32 ? 4 : nr > 4 ? 6 : 8; }
 int plan_team(cfd_batch* b, const std::vector<int>& ids) {
     b->team_nr = 0;
     const int n = (int)ids.size();
@@ -1218,7 +1221,7 @@ int plan_team(cfd_batch* b, const std::vector<int>& ids) {
     const int most = tiles(order[0]);
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->dev));
-    if (n > sms || most > kTeamTilesPerCta * (sms / n)) return CFD_OK;
+    if (n > sms || most > team_tiles(sms / n) * (sms / n)) return CFD_OK;
     const size_t smem = team_smem(b->max_W);
     const void* k = b->precision == CFD_PRECISION_MIXED ? (const void*)k_team_mx : (const void*)k_team_f64;
     if (smem != b->team_smem_bytes) {
@@ -1253,7 +1256,7 @@ int plan_team(cfd_batch* b, const std::vector<int>& ids) {
     const int nr_g = sms / n;
     const bool cluster = nr_c > 0 && (most <= 2 * nr_c || 2 * nr_g < 3 * nr_c);
     const int nr = cluster ? nr_c : nr_g;
-    if (most > kTeamTilesPerCta * nr) return CFD_OK;
+    if (most > team_tiles(nr) * nr) return CFD_OK;
     if (int rc = grow(b->team_ids, b->cap_team_ids, order.size())) return rc;
     if (int rc = grow(b->team_bar, b->cap_team_bar, order.size())) return rc;
     CK(cudaMemcpyAsync(b->team_ids, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice, b->st));

@@ -64,7 +64,7 @@ def _case(kind, n0, n1, mixed=False, dt=None, **kw):
     ("ogrid", 129, 131), ("cavity", 131, 129),  # 33 and 40 tiles: a block sums the totals
     ("ogrid", 46, 46),    # odd width, one level: six colours
     ("ogrid", 181, 91),   # coarsest level 90 x 44: two points of a colour per thread
-    ("ogrid", 131, 130),  # coarsest level 65 x 128 by one CTA: x does not fit, global memory
+    ("ogrid", 131, 130),  # coarsest level 65 x 128 by one CTA: stencils re-read in every pass
     ("cavity", 257, 193),  # a share of the grid: 96 tiles
 ])
 def test_single_case_equals_host_driven(kind, n0, n1, mixed):
@@ -76,7 +76,9 @@ def test_single_case_equals_host_driven(kind, n0, n1, mixed):
     (17, "ogrid", 33, 25, True), (40, "ogrid", 33, 33, True), (148, "ogrid", 17, 17, True),
     (149, "ogrid", 17, 17, False),            # more cases than SMs: the step graph
     (5, "cavity", 129, 97, True), (16, "ogrid", 129, 129, True), (30, "cavity", 129, 129, True),
-    (38, "cavity", 129, 129, False),          # more than 8 tiles per CTA
+    (38, "cavity", 129, 129, False),          # more than 8 tiles per CTA of teams of up to 4
+    (2, "cavity", 385, 385, True), (2, "ogrid", 417, 417, False),     # 4 / 5 per CTA of teams of 74
+    (10, "ogrid", 193, 193, True), (16, "ogrid", 193, 193, False),   # 6 / 8 per CTA of teams of 14 / 9
 ])
 def test_batches_around_the_rule(n, kind, n0, n1, team):
     made = [_case(kind, n0, n1, Re=100.0 + 7 * k) for k in range(n)]
