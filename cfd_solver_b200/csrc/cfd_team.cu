@@ -20,8 +20,10 @@
 //
 // Memory order: a phase's plain stores are read by other CTAs only after the next barrier
 // (release by every CTA, acquire by every CTA); no phase reads what another CTA writes in
-// the same phase. Partial sums alternate between regions, so that a region is not written
-// again before every CTA has read it.
+// the same phase. Partial sums have four regions, and a region is not written again before every
+// CTA has read it: 0 / 1 alternate between sweeps and between the halves of a pressure iteration
+// (a barrier lies between a region's readers and its next writer), 2 is the continuity
+// source's alone, 3 the correction's and the diagnostics'.
 #include "cfd_bulk.cuh"
 #include "cfd_common.cuh"
 #include "cfd_reduce.cuh"
@@ -897,7 +899,9 @@ __device__ __noinline__ void team_correct() {
             correct_bnd(PC, ld, W, per, cav, n0, n1, i, j, pc, far);
         }
         group_reduce<1, 0u>(r, sh().red + g.id * 256, g);
-        if (g.tid == 0) part(2)[(long long)t * PSTRIDE] = r[0];
+        // column 3 of the step's region (team_diag has 0 .. 2): a solve with nothing to do passes no
+        // barrier between team_face_total's reads of part(2) and this store
+        if (g.tid == 0) part(3)[(long long)t * PSTRIDE + 3] = r[0];
     }
 }
 
@@ -1035,18 +1039,16 @@ __device__ __noinline__ void team_diag(int cur, int r0, int r1, int r2, int r3, 
 __device__ __noinline__ void team_step_total() {
     TeamState& ts = sh().ts;
     const CaseDev& c = sh().c;
-    const int n = cell_tiles().n;
-    double v[1], w[3];
-    team_total<1, 0u>(part(2), n, NT, v);
-    team_total<3, 0x5u>(part(3), n, NT, w);
+    double v[4];
+    team_total<4, 0x5u>(part(3), cell_tiles().n, NT, v);
     if (threadIdx.x == 0) {
-        ts.dul1 = v[0];
-        ts.dmax = fmax(w[0], 0.0);
-        ts.dtl1 = w[1];
-        ts.dtmax = w[2];
+        ts.dmax = fmax(v[0], 0.0);
+        ts.dtl1 = v[1];
+        ts.dtmax = v[2];
+        ts.dul1 = v[3];
         // steady residual: mean (|du| + |dv| + |dT|) / dt over the unknown cells
         const double ncell = (double)(c.ihi - c.ilo + 1) * (c.n1 - 2);
-        ts.sr = (v[0] + w[1]) / (c.dt * ncell);
+        ts.sr = (v[3] + v[1]) / (c.dt * ncell);
         if (ts.nstep == 0) ts.sr0 = ts.sr;
     }
 }
