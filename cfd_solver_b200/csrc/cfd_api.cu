@@ -22,6 +22,7 @@
 #include "cfd_kernels.cuh"
 #include "cfd_reduce.cuh"
 #include "cfd_scratch.cuh"
+#include "cfd_share.cuh"
 #include "cfd_sweep.cuh"
 #include "cfd_team.cuh"
 
@@ -52,7 +53,12 @@ namespace {
 
 long long rup(long long x, long long a) { return (x + a - 1) / a * a; }
 
-constexpr int kTeamSteps = 32;  // steps of one team launch at most
+constexpr int kTeamSteps = 32;      // steps of one team launch at most
+// of a launch whose teams hold more than half of the chip, alone and beside other calls, which may
+// have to wait for it (a 65 x 65 case stepped beside twelve: 95th percentile 2,656 us behind launches
+// of 32 steps, 1,100 behind 16, 259 behind 2)
+constexpr int kTeamStepsMost = 16, kTeamStepsShared = 2;
+constexpr int kCrowdSteps = 64;     // steps for which a route chosen for other calls in flight is kept
 constexpr int NFLAGS = 10;  // device flag words of a batch
 
 enum KernelId {
@@ -173,7 +179,7 @@ struct cfd_batch {
     // whose second half ran (graph steps)
     int* flags = nullptr;
     bool use_graph = true;
-    cudaGraphExec_t gexec[2] = {nullptr, nullptr};
+    cudaGraphExec_t gexec[2][2] = {};  // by state parity; [1]: with chained launches
     int launches_per_pair = 2, launches_per_iter = 0, launches_per_half = 0, launches_fixed = 0;
     int flags_total0[3] = {0, 0, 0};
     int* tword = nullptr;                // per tile: the case's momentum-loop word
@@ -218,6 +224,10 @@ struct cfd_batch {
     unsigned* team_bar = nullptr;
     size_t cap_team_ids = 0, cap_team_bar = 0;
     size_t team_smem_bytes = 0;
+    int sms = 0;                      // of the device
+    cudaEvent_t team_ev[2] = {};      // ends of the last two team launches of a long call
+    // steps_done up to which the step graph runs, and runs without chained launches (cfd_batch_step)
+    long long crowded_until = 0, company_until = 0;
     int team_clusters[5] = {};  // clusters of 1, 2, 4, 8, 16 CTAs resident at once (for team_smem_bytes)
     // profiling
     bool prof = false;
@@ -631,7 +641,9 @@ int mg_res_plane(int nu_pre, int nu_post, int fused) {
 
 // Launch a kernel of the step. In a graph segment, a kernel that follows another one may begin
 // while that one drains (after_previous): a 64-case state's step 746 -> 729 us, 64 mixed cavities
-// 1255 -> 1233, one 1025 x 1025 case 949 -> 942, the 256-case sweep 2492 -> 2486.
+// 1255 -> 1233, one 1025 x 1025 case 949 -> 942, the 256-case sweep 2492 -> 2486. The CTAs that wait
+// hold slots, so beside other calls it loses, and the step runs unchained (cfd_batch_step): two
+// batches of 149 33 x 33 O-grids stepped at once 297 / 267 us, four 577 x 577 ones 757 / 638.
 template <class... P, class... A>
 void go(cfd_batch* b, void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem, A... args) {
     cudaLaunchAttribute at = {};
@@ -822,7 +834,7 @@ int one_step_direct(cfd_batch* b) {
 
 // Build the step graph for state parity `cur`: child graphs for the straight segments and
 // two while-loops whose condition kernels read the device counters of still-iterating work.
-int build_step_graph(cfd_batch* b, int cur) {
+int build_step_graph(cfd_batch* b, int cur, bool chained) {
     const bool prof = b->prof;
     b->prof = false;
     const long long l0 = b->launches;
@@ -832,7 +844,7 @@ int build_step_graph(cfd_batch* b, int cur) {
     CK(cudaGraphCreate(&g, 0));
     cudaGraphNode_t prev = nullptr;
     auto segment = [&](auto&& enqueue) {
-        b->chain = cfd_batch::CHAIN_FIRST;
+        b->chain = chained ? cfd_batch::CHAIN_FIRST : cfd_batch::CHAIN_OFF;
         enqueue();
         b->chain = cfd_batch::CHAIN_OFF;
     };
@@ -931,7 +943,7 @@ int build_step_graph(cfd_batch* b, int cur) {
         b->launches_per_iter = (int)(lh1 - lh0) + 2;
         b->launches_per_half = (int)(lh2 - lh1);
         b->launches_fixed = (int)((la - l0) + (lp0 - lm) + (b->launches - lp1));
-        if (cudaGraphInstantiate(&b->gexec[cur], g, 0) != cudaSuccess) rc = fail(CFD_E_CUDA, "graph instantiation failed");
+        if (cudaGraphInstantiate(&b->gexec[chained][cur], g, 0) != cudaSuccess) rc = fail(CFD_E_CUDA, "graph instantiation failed");
     }
     cudaGraphDestroy(g);
     b->launches = l0;
@@ -939,15 +951,17 @@ int build_step_graph(cfd_batch* b, int cur) {
     return rc;
 }
 
-int one_step(cfd_batch* b) {
+// `chained`: the graph whose launches may begin while the one before drains (go)
+int one_step(cfd_batch* b, bool chained) {
     int rc;
     if (b->ntable_cases == 0) return CFD_OK;  // an empty slot pool: nothing to step
     if (b->use_graph && !b->prof) {
-        if (!b->gexec[b->cur]) {
-            rc = build_step_graph(b, b->cur);
+        cudaGraphExec_t& exec = b->gexec[chained][b->cur];
+        if (!exec) {
+            rc = build_step_graph(b, b->cur, chained);
             if (rc) return rc;
         }
-        CK(cudaGraphLaunch(b->gexec[b->cur], b->st));
+        CK(cudaGraphLaunch(exec, b->st));
         b->launches += b->launches_fixed;  // the loops' share is added from the device counters
     } else {
         rc = one_step_direct(b);
@@ -1000,13 +1014,38 @@ int team_steps(cfd_batch* b, int nsteps) {
     return CFD_OK;
 }
 
+// Does a step take the graph because the team launches in flight on the device ask for too much?
+//
+// Team launches that ask for more SMs together than there are take turns, while graph steps of
+// several batches overlap. k batches stepped by k threads, us for a step of all of them, team /
+// (unchained) graph, one step per call, by the SMs that their teams ask for together (148 on the chip):
+//   128 .. 192: 12 x (1 x 65^2) 152 / 328, 3 x (4 x 129^2) 201 / 245, 4 x (3 x 129^2) 196 / 252
+//   256:        8 x (2 x 65^2) 186 / 220, 4 x (4 x 65^2) 184 / 203, 4 x (4 x 129^2) 289 / 267
+//   296:        2 x 193^2 249 / 217, 2 x 257^2 275 / 229, 2 x 257^2 cavities 572 / 454, 2 x 385^2 419 / 309
+//   384, 512:   8 x (3 x 129^2) 420 / 300, 8 x (4 x 65^2) 377 / 232, 8 x (4 x 129^2) 581 / 322
+//   592:        4 x 193^2 506 / 250, 4 x 257^2 579 / 293, 4 x 385^2 837 / 371
+// so the line is at 7/4 of the chip, for a batch whose teams ask for more than a quarter of it (others
+// find room beside one another: 12 x (2 x 65^2) 279 / 326, 12 x (2 x 129^2) 417 / 416). A team that
+// holds more than half of the chip makes smaller calls wait for a whole launch, so beside those it
+// gives way as soon as not all fit (a 65 x 65 case stepped beside a 513 x 513 one: median 8,357 us behind
+// its launches, 140 beside its graph steps, which take 273 us instead of 265). Graph steps queued
+// deep on several streams hold one another up (8 x (4 x 65^2): 512 us with 32 steps queued, 232 with
+// one), so a step that takes the graph for this reason is waited for. Either route gives the same bits.
+bool crowded(const cfd_batch* b, const ChipShare& own) {
+    const int all = own.all_sms(), others = own.all_calls() - 1;
+    if (others < 1 || 4 * own.sms() <= b->sms) return false;
+    const bool beside_small = 2 * own.sms() > b->sms && all > b->sms && 2 * (all - own.sms()) <= b->sms * others;
+    return 4 * all > 7 * b->sms || beside_small;
+}
+
 // adds the loop launches of graph steps (from the cumulative device counters) to the count
 void drop_graphs(cfd_batch* b) {
-    for (int k = 0; k < 2; k++)
-        if (b->gexec[k]) {
-            cudaGraphExecDestroy(b->gexec[k]);
-            b->gexec[k] = nullptr;
-        }
+    for (auto& form : b->gexec)
+        for (auto& exec : form)
+            if (exec) {
+                cudaGraphExecDestroy(exec);
+                exec = nullptr;
+            }
 }
 
 int account_graph_launches(cfd_batch* b) {
@@ -1219,8 +1258,8 @@ int plan_team(cfd_batch* b, const std::vector<int>& ids) {
     auto tiles = [&](int c) { return b->hc[c].jt_count; };
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return tiles(x) > tiles(y); });
     const int most = tiles(order[0]);
-    int sms = 0;
-    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->dev));
+    if (b->sms == 0) CK(cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, b->dev));
+    const int sms = b->sms;
     if (n > sms || most > team_tiles(sms / n) * (sms / n)) return CFD_OK;
     const size_t smem = team_smem(b->max_W);
     const void* k = b->precision == CFD_PRECISION_MIXED ? (const void*)k_team_mx : (const void*)k_team_f64;
@@ -1813,10 +1852,30 @@ int cfd_batch_step(cfd_batch* b, int nsteps) {
     if (!b || nsteps < 0) return fail(CFD_E_ARG, "bad arguments");
     // the team kernel has form 2 of the V-cycle only, and no copy waits for a limit to bound
     const bool team = b->team_nr > 0 && b->use_graph && !b->prof && b->mg_fused == 2 && b->bd.wait_polls == kWaitPolls;
-    for (int s = 0; team && s < nsteps; s += kTeamSteps)
-        if (int rc = team_steps(b, std::min(kTeamSteps, nsteps - s))) return rc;
-    for (int s = 0; !team && s < nsteps; s++) {
-        int rc = one_step(b);
+    const int share = team ? b->team_nr * b->ntable_cases : 0;
+    const ChipShare own(b->dev, share);
+    for (int s = 0, k = 0, rc = CFD_OK; s < nsteps;) {
+        // a long call queues a team launch behind the running one, not a third: what else is in flight
+        // is looked at again before each
+        if (k >= 2) CK(cudaEventSynchronize(b->team_ev[k & 1]));
+        if (own.company()) b->company_until = b->steps_done + kCrowdSteps;
+        if (team && crowded(b, own)) b->crowded_until = b->steps_done + kCrowdSteps;
+        const bool company = b->steps_done < b->company_until;
+        if (team && b->steps_done >= b->crowded_until) {
+            const int most = 2 * share <= b->sms ? kTeamSteps : company ? kTeamStepsShared : kTeamStepsMost;
+            const int n = std::min(most, nsteps - s);
+            rc = team_steps(b, n);
+            s += n;
+            cudaEvent_t& ev = b->team_ev[k++ & 1];
+            if (!rc && s < nsteps) {
+                if (!ev) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+                CK(cudaEventRecord(ev, b->st));
+            }
+        } else {
+            rc = one_step(b, !company);
+            if (!rc && team) CK(cudaStreamSynchronize(b->st));
+            s++;
+        }
         if (rc) return rc;
     }
     CK(cudaStreamSynchronize(b->st));
@@ -1860,6 +1919,8 @@ int cfd_batch_destroy(cfd_batch* b) {
     cudaFree(b->stage); cudaFree(b->stage_off);
     cudaFree(b->partial); cudaFree(b->flags); cudaFree(b->work); cudaFree(b->tword); cudaFree(b->dtiles); cudaFree(b->dcc); cudaFree(b->dtmaps);
     cudaFree(b->team_ids); cudaFree(b->team_bar);
+    for (auto e : b->team_ev)
+        if (e) cudaEventDestroy(e);
     if (b->h_flags) cudaFreeHost(b->h_flags);
     if (b->st) cudaStreamDestroy(b->st);
     delete b;
@@ -2300,6 +2361,7 @@ int cfd_sip_solve(int n0, int n1, int periodic, const double* const* coef9, doub
     p.state = m + o_state;
     p.t.bar = bar;
     p.t.nr = std::min(sms, std::max(16, d.jt_count));  // a CTA per tile, the chip at most
+    const ChipShare share(dev, p.t.nr);  // a step beside this call may give way
     p.t.nu_pre = 1;
     p.t.nu_post = 3;
     p.t.coarse_sweeps = 12;

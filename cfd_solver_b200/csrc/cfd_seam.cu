@@ -29,6 +29,7 @@
 
 #include "../../include/cfd_b200.h"
 #include "cfd_scratch.cuh"
+#include "cfd_share.cuh"
 
 namespace cfd_seam {
 
@@ -259,22 +260,24 @@ __global__ void __launch_bounds__(BS, 2) k_seam_solve(const __grid_constant__ Sy
     }
 }
 
-// CTAs that are resident together on the current device (0: the query failed)
-int resident_blocks() {
+// CTAs that are resident together on the current device, and its SMs (0: the query failed)
+struct Resident {
+    int dev, all, sms;
+};
+Resident resident_blocks() {
     static std::atomic<int> known[64];
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-    int n = known[dev].load();
-    if (n == 0) {
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return {0, 0, 0};
+    int v = known[dev].load();
+    if (v == 0) {
         int sms = 0, per = 0;
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_seam_solve, BS, 0) != cudaSuccess)
-            return 0;
-        n = sms * per;
-        if (n > MAX_BLOCKS / 3) n = MAX_BLOCKS / 3;
-        known[dev].store(n);
+            return {0, 0, 0};
+        v = sms << 16 | std::min(sms * per, MAX_BLOCKS / 3);
+        known[dev].store(v);
     }
-    return n;
+    return {dev, v & 0xffff, v >> 16};
 }
 
 }  // namespace cfd_seam
@@ -296,12 +299,13 @@ int cfd_seam_solve(int n0, int n1, int periodic, const double* const* coef, doub
     s.x0 = phi;
     s.x1 = scratch + SCRATCH_HEAD;
     s.q = q;
-    const int most = resident_blocks();
-    if (most <= 0) {
+    const Resident most = resident_blocks();
+    if (most.all <= 0) {
         cfd_internal_set_error("gauss seam: no usable device");
         return CFD_E_CUDA;
     }
-    const int grid = (int)std::min<long long>(most, ((long long)nx * ny + BS - 1) / BS);
+    const int grid = (int)std::min<long long>(most.all, ((long long)nx * ny + BS - 1) / BS);
+    const cfd::ChipShare share(most.dev, std::min(grid, most.sms));  // a step beside this call may give way
     // sweeps run in pairs (the pair ends in the caller's array), so at most maxit rounded
     // down to even sweeps are taken; the outcome is read once per launch
     double sc[8] = {};

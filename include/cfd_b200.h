@@ -140,6 +140,9 @@ int cfd_case_destroy(cfd_case* c);
 /* ---- batch: many cases of uneven size and parameters in one set of launches ---- */
 int cfd_batch_create(int ncases, const cfd_grid* grids, const cfd_params* params,
                      cfd_batch** out);
+/* `nsteps` outer steps of every active case; returns when they are done. Several threads may step
+ * a batch each at the same time: a step chooses its launches by what else of the library is in
+ * flight on the device, with the same bits either way. */
 int cfd_batch_step(cfd_batch* b, int nsteps);
 int cfd_batch_stats(cfd_batch* b, int case_index, cfd_step_stats* out);
 /* named plane of one case ("u", "v", "T", "p", "up", "vp", "us", "vs", "pcor", "q",
