@@ -5,7 +5,8 @@
 // than the solve itself; here the scratch comes from a pool of the library, one per device,
 // stream-ordered on the caller's stream, so calls from several threads and streams share it
 // safely. The pool keeps at most kScratchKeep bytes between calls and gives anything above back
-// to the device at the next synchronisation.
+// to the device at the next synchronisation. A pool dies with its context (cudaDeviceReset), so
+// it is kept with the context's id.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -15,4 +16,6 @@ constexpr unsigned long long kScratchKeep = 256ull << 20;
 void* scratch_take(size_t bytes, cudaStream_t st);
 // gives it back once the work queued on `st` so far is done
 void scratch_give(void* p, cudaStream_t st);
+// id of the calling thread's context, never used again by another one; 0: none, or the query failed
+unsigned long long context_id();
 }  // namespace cfd

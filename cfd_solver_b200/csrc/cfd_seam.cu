@@ -20,6 +20,7 @@
 // grids (1025^2: 41 us a sweep of 28 planes, 5.7 TB/s; 24 sweeps 2.73 -> 1.05 ms a call) and by
 // the launch, the barriers and the loads' latency on small ones (257^2, 4 sweeps: 772 -> 50 us;
 // before, a cudaMalloc, a launch per sweep, a host wait per pair and a cudaFree).
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -354,14 +355,20 @@ size_t cfd_seam_scratch_doubles(int n0, int n1, int periodic) {
 namespace cfd {
 namespace {
 constexpr int kMaxDevices = 64;
+struct DevicePool {
+    cudaMemPool_t pool;
+    unsigned long long context;
+};
 std::mutex g_pool_mu;
-cudaMemPool_t g_pool[kMaxDevices] = {};
+DevicePool g_pool[kMaxDevices] = {};
 
 cudaMemPool_t scratch_pool() {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
+    const unsigned long long id = context_id();
     std::lock_guard<std::mutex> lock(g_pool_mu);
-    if (!g_pool[dev]) {
+    DevicePool& d = g_pool[dev];
+    if (!d.pool || d.context != id) {  // the pool of a context that is gone went with it
         cudaMemPoolProps props = {};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
@@ -370,11 +377,27 @@ cudaMemPool_t scratch_pool() {
         if (cudaMemPoolCreate(&p, &props) != cudaSuccess) return nullptr;
         unsigned long long keep = kScratchKeep;
         cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
-        g_pool[dev] = p;
+        d = {p, id};
     }
-    return g_pool[dev];
+    return d.pool;
 }
 }  // namespace
+
+unsigned long long context_id() {
+    using GetId = CUresult (*)(CUcontext, unsigned long long*);
+    static const GetId get = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return reinterpret_cast<GetId>(f);
+    }();
+    unsigned long long id = 0;
+    // cudaFree(nullptr) makes the device's context current where the thread has none yet
+    if (cudaFree(nullptr) != cudaSuccess || !get || get(nullptr, &id) != CUDA_SUCCESS) return 0;
+    return id;
+}
 
 void* scratch_take(size_t bytes, cudaStream_t st) {
     void* p = nullptr;
