@@ -14,6 +14,7 @@
 #include <string>
 
 #include "../../include/cfd_b200.h"
+#include "cfd_scratch.cuh"
 
 int cfd_seam_solve(int n0, int n1, int periodic, const double* const* coef, double* phi, const double* q,
                    double tol, int maxit, int* sweeps, void* stream, double* scratch);
@@ -32,7 +33,11 @@ constexpr long long kScratchDoubles = kMaxPoints + (kMaxPoints / 256 + 64) + 16;
 __device__ __align__(256) double g_gauss_scratch[kScratchDoubles];
 
 constexpr int kMaxDevices = 64;
-double* g_scratch_ptr[kMaxDevices] = {};
+struct ScratchAddress {
+    double* p;
+    unsigned long long context;  // the array moves with the context that loads the library
+};
+ScratchAddress g_scratch_ptr[kMaxDevices] = {};
 std::mutex g_scratch_mu;
 
 }  // namespace
@@ -63,19 +68,20 @@ extern "C" int cfd_gauss_solve_noalloc(int n0, int n1, int periodic, const doubl
     }
     double* scratch = nullptr;
     {
-        // set-up, once per device and with that device current: the device address of the
+        // set-up, once per device context and with that device current: the device address of the
         // array (in host code its name is only a host-side stand-in)
+        const unsigned long long context = cfd::context_id();
         std::lock_guard<std::mutex> lock(g_scratch_mu);
-        if (!g_scratch_ptr[dev]) {
+        if (!g_scratch_ptr[dev].p || g_scratch_ptr[dev].context != context) {
             double* p = nullptr;
             cudaError_t e = cudaGetSymbolAddress((void**)&p, g_gauss_scratch);
             if (e != cudaSuccess || !p) {
                 cfd_internal_set_error((std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e)).c_str());
                 return CFD_E_CUDA;
             }
-            g_scratch_ptr[dev] = p;
+            g_scratch_ptr[dev] = {p, context};
         }
-        scratch = g_scratch_ptr[dev];
+        scratch = g_scratch_ptr[dev].p;
     }
     // cfd_seam_solve clears the scalars and the counter it relies on before its first sweep
     const int rc = cfd_seam_solve(n0, n1, periodic, coef, phi, q, tol, maxit, sweeps, stream, scratch);

@@ -1,7 +1,8 @@
 """The seams after the host program has reset the device.
 
 cudaDeviceReset() ends the process's own context and with it whatever the library kept in it (the
-scratch pool); the next call starts again from nothing. Each case runs in a process of its own.
+scratch pool, the address of the static scratch); the next call starts again from nothing. Each
+case runs in a process of its own.
 """
 import subprocess
 import sys
@@ -46,7 +47,7 @@ print("same")
 """
 
 
-@pytest.mark.parametrize("seam", ["gauss", "sip"])
+@pytest.mark.parametrize("seam", ["gauss", "sip", "noalloc"])
 def test_seam_after_a_device_reset(seam):
     r = subprocess.run([sys.executable, "-c", PROGRAM, seam], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "same" in r.stdout, r.stdout + r.stderr
