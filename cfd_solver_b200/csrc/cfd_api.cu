@@ -13,6 +13,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <limits>
 #include <string>
 #include <vector>
 
@@ -607,7 +608,8 @@ void case_scalars_to_dev(CaseDev& d, double dxi0, double dxi1, double ar, const 
     d.rPr = 1.0 / d.Pr;
     d.rd0 = 1.0 / d.d0; d.rd1 = 1.0 / d.d1; d.hd0 = 0.5 / d.d0; d.hd1 = 0.5 / d.d1; d.rdt = 1.0 / d.dt;
     d.circ_de = p.fix_circ_de ? 1.0 / (d.n0 - 1) : 1.0 / (d.n0 - 2);
-    auto by = [](double x) { return DivBy{x, 1.0 / x}; };
+    // (a reciprocal that overflows: the largest number, so that 0 / x stays 0)
+    auto by = [](double x) { return DivBy{x, std::min(1.0 / x, std::numeric_limits<double>::max())}; };
     d.v0 = by(d.d0); d.v1 = by(d.d1); d.v00 = by(d.d0 * d.d0); d.v11 = by(d.d1 * d.d1);
     d.v01 = by(2.0 * d.d0 * d.d1); d.v1x2 = by(2.0 * d.d1); d.vdt = by(d.dt); d.vRe = by(d.Re);
     d.vRePr = by(d.Re * d.Pr); d.v01Re = by(2.0 * d.d0 * d.d1 * d.Re);

@@ -108,15 +108,18 @@ struct LevelDev {
 // Computation of elementary functions on the IBM RISC System/6000 processor, IBM J. Res. Dev.
 // 34, 1990: a quotient within an ulp and a correctly rounded reciprocal give the rounded
 // quotient) are five dependent operations and no branch, where a full FP64 division is some 300
-// cycles that nothing overlaps. Quotients near the ends of the exponent range are not exact.
+// cycles that nothing overlaps. The first quotient stands where it is zero (the corrections would
+// lose its sign, and an infinite divisor, an inviscid case's Re, has the reciprocal 0) or not
+// finite (n is, or the quotient overflows). Subnormal quotients may be a unit in the last place off.
 struct DivBy {
     double d, y;
 };
 #ifdef __CUDACC__
 __device__ __forceinline__ double div_by(double n, const DivBy& D) {
-    double q = n * D.y;
+    const double q0 = n * D.y;
+    double q = fma(fma(-D.d, q0, n), D.y, q0);
     q = fma(fma(-D.d, q, n), D.y, q);
-    return fma(fma(-D.d, q, n), D.y, q);
+    return fabs(q0) > 0.0 && fabs(q0) <= 1.7976931348623157e308 ? q : q0;
 }
 #endif
 
