@@ -212,7 +212,7 @@ struct cfd_batch {
     int mg_pre = 1, mg_post = 3;  // multigrid sweeps before / after the coarse correction
     int mg_fused = 2;             // 1: a smoothing phase's sweeps in one launch; 2: and the
                                   // pre-smoothing inside the residual + restriction launch
-    int swf_threads = 128;  // k_sweep_fin CTA size: 512 when a case has >= 1024 tiles
+    int swf_threads = 128;  // k_sweep_fin CTA size: the most that a case of the batch sums with
     int max_W = 0;
     int cur = 0;
     long long steps_done = 0;
@@ -987,7 +987,6 @@ int team_steps(cfd_batch* b, int nsteps) {
     a.nsteps = nsteps;
     a.sweep_cap = b->bd.mom_cap;
     a.maxit_p = a.p_iters = b->maxit_p;
-    a.fin_threads = b->swf_threads;
     a.nu_pre = b->mg_pre;
     a.nu_post = b->mg_post;
     a.coarse_sweeps = b->coarse_sweeps;
@@ -1384,7 +1383,7 @@ int build_tables(cfd_batch* b, const std::vector<int>& ids) {
     bd.mom_cap = mom_cap(b);
     b->ntable_cases = (int)ids.size();
     b->sw_grid = (int)jtiles.size();  // one CTA per 32 x 16 tile
-    b->swf_threads = jt_max >= 1024 ? SWF_THREADS : 128;
+    b->swf_threads = sweep_sum_threads(jt_max);
     const size_t bc_smem = 2 * (size_t)(b->max_W + 1) * sizeof(double);
     if (bc_smem > 48 * 1024)
         CK(cudaFuncSetAttribute(k_bc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bc_smem));

@@ -475,8 +475,8 @@ __global__ void __launch_bounds__(SWF_THREADS) k_sweep_fin(BatchDev b) {
     FinIn in;
     if (tid == 0) fin_load(b, c, cid, in);
     double v[NFIELD] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    const int np = c.jt_count;  // one row per tile
-    for (int e = tid; e < np; e += blockDim.x) {
+    const int np = c.jt_count, nt = sweep_sum_threads(np);  // one row per tile
+    for (int e = tid < nt ? tid : np; e < np; e += nt) {
         const double* src = b.partial + ((long long)c.jt_begin + e) * PSTRIDE;
 #pragma unroll
         for (int f = 0; f < NFIELD; f++) v[f] += src[f];

@@ -397,7 +397,8 @@ __device__ __noinline__ void team_mom_rule(int sweep) {
     TeamState& ts = sh().ts;
     const CaseDev& c = sh().c;
     double v[NFIELD];
-    team_total<NFIELD, 0u>(part(sweep & 1), cell_tiles().n, sh().a.fin_threads, v);
+    const int n = cell_tiles().n;
+    team_total<NFIELD, 0u>(part(sweep & 1), n, sweep_sum_threads(n), v);
     if (threadIdx.x < 32) {
         const int lane = threadIdx.x, mask = ts.mask, flip = ts.flip;
         double x = 0.0;

@@ -17,7 +17,6 @@ struct TeamArgs {
     int sweep_cap;        // sweeps of one momentum / energy solve
     int maxit_p;          // iteration cap of the pressure solve
     int p_iters;          // iterations of it in this launch
-    int fin_threads;      // threads that sum a sweep's partial residuals (as k_sweep_fin)
     int nu_pre, nu_post, coarse_sweeps;
 };
 
