@@ -975,8 +975,8 @@ int one_step(cfd_batch* b, bool chained) {
     return CFD_OK;
 }
 
-// `nsteps` steps of every case by the team kernel
-int team_steps(cfd_batch* b, int nsteps) {
+// `nsteps` steps of every case by the team kernel, whose grid-form barriers wait `polls` polls at most
+int team_steps(cfd_batch* b, int nsteps, unsigned polls = TEAM_POLLS) {
     TeamArgs a{};
     a.b = b->bd;
     a.b.cur = b->cur;
@@ -990,6 +990,7 @@ int team_steps(cfd_batch* b, int nsteps) {
     a.nu_pre = b->mg_pre;
     a.nu_post = b->mg_post;
     a.coarse_sweeps = b->coarse_sweeps;
+    a.polls = polls;
     if (!a.cluster) CK(cudaMemsetAsync(b->team_bar, 0, sizeof(unsigned) * b->ntable_cases, b->st));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(a.nr * b->ntable_cases));
@@ -1883,6 +1884,15 @@ int cfd_batch_step(cfd_batch* b, int nsteps) {
     return account_graph_launches(b);
 }
 
+// The team kernel's launches with a barrier limit of the caller's (tests: a wait that runs out)
+int cfd_internal_team_steps(cfd_batch* b, int launches, unsigned polls) {
+    if (!b || b->team_nr == 0 || b->team_cluster) return fail(CFD_E_ARG, "the batch has no grid-form teams");
+    for (int k = 0; k < launches; k++)
+        if (int rc = team_steps(b, 1, polls)) return rc;
+    CK(cudaStreamSynchronize(b->st));
+    return account_graph_launches(b);
+}
+
 int cfd_batch_stats(cfd_batch* b, int case_index, cfd_step_stats* out) {
     if (!b || !out || case_index < 0 || case_index >= b->n) return fail(CFD_E_ARG, "bad arguments");
     int rc = fetch_scalars(b);
@@ -2309,8 +2319,8 @@ int cfd_batch_set_state(cfd_batch* b, const void* host, size_t bytes) {
 // a call built a one-case batch, with a host-side grid and every plane of a step, and released
 // it. Measured per call: 257 x 257 cavity, 3 iterations 6.7 -> 0.42 ms; 1025 x 1025, 104 -> 1.10
 // ms; bound by the phases' latency (two V-cycles an iteration), on large grids by their bytes.
-int cfd_sip_solve(int n0, int n1, int periodic, const double* const* coef9, double* phi, const double* q,
-                  double tol, int maxit, int* iters, void* stream) {
+int cfd_internal_sip_solve(int n0, int n1, int periodic, const double* const* coef9, double* phi,
+                           const double* q, double tol, int maxit, int* iters, void* stream, unsigned polls) {
     if (iters) *iters = 0;
     if (n0 < 8 || n1 < (periodic ? 6 : 7) || !coef9 || !phi || !q || maxit < 1 || !(tol >= 0.0))
         return fail(CFD_E_ARG, "cfd_sip_solve: bad arguments");
@@ -2367,6 +2377,7 @@ int cfd_sip_solve(int n0, int n1, int periodic, const double* const* coef9, doub
     p.t.nu_post = 3;
     p.t.coarse_sweeps = 12;
     p.t.maxit_p = maxit;
+    p.t.polls = polls;
     // sip9p's argument order (ap, ae, as, an, aw, ase, asw, ane, anw) -> P_AP .. P_ASW
     const int order[9] = {0, 1, 4, 3, 2, 7, 8, 5, 6};
     for (int k = 0; k < 9; k++) p.a[k] = coef9[order[k]];
@@ -2395,6 +2406,10 @@ int cfd_sip_solve(int n0, int n1, int periodic, const double* const* coef9, doub
     if (status & ST_BREAKDOWN) return finish(fail(CFD_E_BREAKDOWN, "cfd_sip_solve: Krylov breakdown"));
     if (status & ST_MAXITER) return finish(fail(CFD_E_MAXITER, "cfd_sip_solve: maxit reached"));
     return finish(CFD_OK);
+}
+int cfd_sip_solve(int n0, int n1, int periodic, const double* const* coef9, double* phi, const double* q,
+                  double tol, int maxit, int* iters, void* stream) {
+    return cfd_internal_sip_solve(n0, n1, periodic, coef9, phi, q, tol, maxit, iters, stream, TEAM_POLLS);
 }
 
 // ---- single case

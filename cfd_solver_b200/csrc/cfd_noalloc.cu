@@ -17,7 +17,7 @@
 #include "cfd_scratch.cuh"
 
 int cfd_seam_solve(int n0, int n1, int periodic, const double* const* coef, double* phi, const double* q,
-                   double tol, int maxit, int* sweeps, void* stream, double* scratch);
+                   double tol, int maxit, int* sweeps, void* stream, double* scratch, unsigned polls);
 size_t cfd_seam_scratch_doubles(int n0, int n1, int periodic);
 void cfd_internal_set_error(const char* msg);
 
@@ -84,7 +84,7 @@ extern "C" int cfd_gauss_solve_noalloc(int n0, int n1, int periodic, const doubl
         scratch = g_scratch_ptr[dev].p;
     }
     // cfd_seam_solve clears the scalars and the counter it relies on before its first sweep
-    const int rc = cfd_seam_solve(n0, n1, periodic, coef, phi, q, tol, maxit, sweeps, stream, scratch);
+    const int rc = cfd_seam_solve(n0, n1, periodic, coef, phi, q, tol, maxit, sweeps, stream, scratch, cfd::kSeamPolls);
     // an error return can leave sweeps of this call queued on the stream; they must finish
     // before the caller's next call reuses the shared array
     if (rc == CFD_E_CUDA) cudaStreamSynchronize((cudaStream_t)stream);

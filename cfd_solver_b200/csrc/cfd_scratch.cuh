@@ -12,6 +12,7 @@
 
 namespace cfd {
 constexpr unsigned long long kScratchKeep = 256ull << 20;
+constexpr unsigned kSeamPolls = 1u << 24;  // polls of the gauss solve's barrier before it gives up (about 10 s)
 // scratch of `bytes` bytes on the current device, usable by work on `st`; nullptr: no memory
 void* scratch_take(size_t bytes, cudaStream_t st);
 // gives it back once the work queued on `st` so far is done

@@ -37,7 +37,6 @@ namespace cfd_seam {
 constexpr int BS = 256;
 constexpr int MAX_BLOCKS = 2048;         // rows of a partial buffer
 constexpr int kSeamSweeps = 512;         // sweeps of one launch at most
-constexpr unsigned kSeamPolls = 1u << 24;  // polls of the barrier before it gives up (about 10 s)
 
 // scratch layout (doubles): scalars, two partial buffers of three columns, the second iterate
 enum { SC_A, SC_B, SC_R0, SC_W, SC_DONE, SC_SWEEPS, SC_FAIL, SC_CNT, NSC };
@@ -53,6 +52,7 @@ struct Sys {
     double* sc;           // scalars
     double* part;         // per-block partials, two buffers of MAX_BLOCKS
     unsigned int* cnt;    // barrier arrivals, zero at launch
+    unsigned polls;       // of a barrier before it gives up
 };
 
 // gauss() argument order: ap, ae, as, an, aw, ase, asw, ane, anw, ass, assee, assww, asse,
@@ -75,7 +75,7 @@ __device__ __forceinline__ bool seam_barrier(const Sys& s, unsigned& target) {
         __threadfence();
         atomicAdd(s.cnt, 1u);
         got = false;
-        for (unsigned n = 0; n < kSeamPolls && !got; n++) {
+        for (unsigned n = 0; n < s.polls && !got; n++) {
             unsigned v;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(s.cnt) : "memory");
             got = (int)(v - target) >= 0;
@@ -287,7 +287,7 @@ void cfd_internal_set_error(const char* msg);
 
 // shared driver on `scratch` (cfd_seam_scratch_doubles() doubles, 16-byte aligned)
 int cfd_seam_solve(int n0, int n1, int periodic, const double* const* coef, double* phi, const double* q,
-                   double tol, int maxit, int* sweeps, void* stream, double* scratch) {
+                   double tol, int maxit, int* sweeps, void* stream, double* scratch, unsigned polls) {
     using namespace cfd_seam;
     cudaStream_t st = (cudaStream_t)stream;
     Sys s;
@@ -300,6 +300,7 @@ int cfd_seam_solve(int n0, int n1, int periodic, const double* const* coef, doub
     s.x0 = phi;
     s.x1 = scratch + SCRATCH_HEAD;
     s.q = q;
+    s.polls = polls;
     const Resident most = resident_blocks();
     if (most.all <= 0) {
         cfd_internal_set_error("gauss seam: no usable device");
@@ -414,8 +415,9 @@ void scratch_give(void* p, cudaStream_t st) {
 }
 }  // namespace cfd
 
-extern "C" int cfd_gauss_solve(int n0, int n1, int periodic, const double* const* coef, double* phi,
-                               const double* q, double tol, int maxit, int* sweeps, void* stream) {
+extern "C" int cfd_internal_gauss_solve(int n0, int n1, int periodic, const double* const* coef, double* phi,
+                                        const double* q, double tol, int maxit, int* sweeps, void* stream,
+                                        unsigned polls) {
     if (n0 < 8 || n1 < 6 || !coef || !phi || !q || maxit < 2) {
         cfd_internal_set_error("cfd_gauss_solve: bad arguments");
         return CFD_E_ARG;
@@ -431,8 +433,13 @@ extern "C" int cfd_gauss_solve(int n0, int n1, int periodic, const double* const
         cfd_internal_set_error("cfd_gauss_solve: no device memory for the scratch");
         return CFD_E_OOM;
     }
-    const int rc = cfd_seam_solve(n0, n1, periodic, coef, phi, q, tol, maxit, sweeps, stream, scratch);
+    const int rc = cfd_seam_solve(n0, n1, periodic, coef, phi, q, tol, maxit, sweeps, stream, scratch, polls);
     if (rc == CFD_E_CUDA) cudaStreamSynchronize((cudaStream_t)stream);
     cfd::scratch_give(scratch, (cudaStream_t)stream);
     return rc;
+}
+
+extern "C" int cfd_gauss_solve(int n0, int n1, int periodic, const double* const* coef, double* phi,
+                               const double* q, double tol, int maxit, int* sweeps, void* stream) {
+    return cfd_internal_gauss_solve(n0, n1, periodic, coef, phi, q, tol, maxit, sweeps, stream, cfd::kSeamPolls);
 }

@@ -37,7 +37,6 @@ namespace {
 
 constexpr int NT5 = TEAM_THREADS;
 constexpr int TAIL_TILES = 1;  // levels of at most this many regions run in one CTA
-constexpr unsigned kTeamPolls = 1u << 24;  // polls of a counter barrier before it gives up (about 10 s)
 
 // the case's solver state, one copy per CTA, the same in all of them
 struct TeamState {
@@ -104,11 +103,11 @@ __device__ __noinline__ bool team_barrier() {
     bool got = true;
     if (threadIdx.x == 0) {
         unsigned* bar = sh().bar;
-        const unsigned target = sh().target += sh().a.nr;
+        const unsigned target = sh().target += sh().a.nr, limit = sh().a.polls;
         __threadfence();
         atomicAdd(bar, 1u);
         got = false;
-        for (unsigned n = 0; n < kTeamPolls && !got; n++) {
+        for (unsigned n = 0; n < limit && !got; n++) {
             unsigned v;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
             got = (int)(v - target) >= 0;
@@ -1121,6 +1120,8 @@ __device__ __forceinline__ void team_run(const TeamArgs& a) {
     const int cid = a.ids[team];
     int* is = b.iscal + (long long)cid * NISCAL;
     double* sc = b.scal + (long long)cid * NSCAL;
+    // a launch queued behind one whose barrier gave up leaves the batch as it is
+    if (!a.cluster && *b.error) return;
     if (!is[I_ACTIVE]) {  // an empty slot takes no part in the step (uniform over the team)
         if (rank == 0 && tid == 0) {
             int word = 0;

@@ -5,7 +5,7 @@
 namespace cfd {
 
 constexpr int TEAM_THREADS = 512;
-constexpr int TEAM_MAX_CLUSTER = 16;
+constexpr unsigned TEAM_POLLS = 1u << 24;  // polls of a grid-form barrier before it gives up (about 10 s)
 
 struct TeamArgs {
     BatchDev b;           // b.cur: state parity before the first step
@@ -18,6 +18,7 @@ struct TeamArgs {
     int maxit_p;          // iteration cap of the pressure solve
     int p_iters;          // iterations of it in this launch
     int nu_pre, nu_post, coarse_sweeps;
+    unsigned polls;       // limit of the grid form's barrier waits
 };
 
 // The sip9p() seam: one pressure-correction solve by one team (a cooperative grid). The caller's
