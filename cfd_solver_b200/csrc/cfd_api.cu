@@ -60,6 +60,7 @@ constexpr int kTeamSteps = 32;      // steps of one team launch at most
 // of 32 steps, 1,100 behind 16, 259 behind 2)
 constexpr int kTeamStepsMost = 16, kTeamStepsShared = 2;
 constexpr int kCrowdSteps = 64;     // steps for which a route chosen for other calls in flight is kept
+constexpr int kGraphPays = 100;     // steps after which a second form of the step graph has paid for itself
 constexpr int NFLAGS = 10;  // device flag words of a batch
 
 enum KernelId {
@@ -180,7 +181,8 @@ struct cfd_batch {
     // whose second half ran (graph steps)
     int* flags = nullptr;
     bool use_graph = true;
-    cudaGraphExec_t gexec[2][2] = {};  // by state parity; [1]: with chained launches
+    cudaGraphExec_t gexec[2][2] = {};  // [chained launches][state parity]
+    int graph_wanted[2] = {};          // steps that wanted each form since the graphs were dropped
     int launches_per_pair = 2, launches_per_iter = 0, launches_per_half = 0, launches_fixed = 0;
     int flags_total0[3] = {0, 0, 0};
     int* tword = nullptr;                // per tile: the case's momentum-loop word
@@ -953,11 +955,17 @@ int build_step_graph(cfd_batch* b, int cur, bool chained) {
     return rc;
 }
 
-// `chained`: the graph whose launches may begin while the one before drains (go)
+// `chained`: the graph whose launches may begin while the one before drains (go). Building a
+// graph takes 1 to 3 ms, what its other form gains 10 to 60 us a step: while only the other is there,
+// that one runs until this one has been wanted for kGraphPays steps (eight steps each of four
+// batches of 64 cases with their transfers, built on first want: 8.0e8 cell-updates/s instead of 9.3e8).
 int one_step(cfd_batch* b, bool chained) {
     int rc;
     if (b->ntable_cases == 0) return CFD_OK;  // an empty slot pool: nothing to step
     if (b->use_graph && !b->prof) {
+        int& wanted = b->graph_wanted[chained];
+        wanted = std::min(wanted + 1, kGraphPays);
+        if (wanted < kGraphPays && !b->gexec[chained][b->cur] && b->gexec[!chained][b->cur]) chained = !chained;
         cudaGraphExec_t& exec = b->gexec[chained][b->cur];
         if (!exec) {
             rc = build_step_graph(b, b->cur, chained);
@@ -1042,6 +1050,7 @@ bool crowded(const cfd_batch* b, const ChipShare& own) {
 
 // adds the loop launches of graph steps (from the cumulative device counters) to the count
 void drop_graphs(cfd_batch* b) {
+    b->graph_wanted[0] = b->graph_wanted[1] = 0;
     for (auto& form : b->gexec)
         for (auto& exec : form)
             if (exec) {
@@ -2317,7 +2326,7 @@ int cfd_batch_set_state(cfd_batch* b, const void* host, size_t bytes) {
 // (k_team_sip), with the reference's relative L1 stop rule. Its scratch (the stencil, the Krylov
 // vectors, the FP32 hierarchy: about 190 bytes per point) comes from the library's pool. Before,
 // a call built a one-case batch, with a host-side grid and every plane of a step, and released
-// it. Measured per call: 257 x 257 cavity, 3 iterations 6.7 -> 0.42 ms; 1025 x 1025, 104 -> 1.10
+// it. Measured per call: 257 x 257 cavity, 3 iterations 7 to 18 ms (by the host's load) -> 0.44; 1025 x 1025, 104 -> 1.10
 // ms; bound by the phases' latency (two V-cycles an iteration), on large grids by their bytes.
 int cfd_internal_sip_solve(int n0, int n1, int periodic, const double* const* coef9, double* phi,
                            const double* q, double tol, int maxit, int* iters, void* stream, unsigned polls) {
