@@ -1198,37 +1198,39 @@ __device__ __forceinline__ Edge edge_at(const BcCase& a, long long k) {
     return Edge{a.U[k], a.U[k + 1], a.U[k - 1], a.V[k], a.V[k + 1], a.V[k - 1]};
 }
 
-// One component of the boundary momentum balance dp/dx_m = lap(f) / Re - conv(f) - accel +
-// (buoyancy) at a boundary point: f at the point (f0), its neighbours along the boundary (fe,
-// fw) and the two rows inside (f1, f2), the cross difference bd, the convection cy across
-// the boundary
+// One component of the boundary momentum balance lap(f) / Re - conv(f) at a boundary point: f at
+// the point (f0), its neighbours along the boundary (fe, fw) and the two rows inside (f1, f2), the
+// cross difference bd, the convection cy across the boundary. The callers subtract the
+// acceleration of the boundary and add the buoyancy.
 __device__ __forceinline__ double bc_force(const CaseDev& c, double f0, double fe, double fw, double f1, double f2,
-                                           double bd, double al, double ga, double be, double uxi, double cy,
-                                           double alc, double Ri, double T) {
+                                           double bd, double al, double ga, double be, double uxi, double cy) {
     const double aa = div_by(al * (fe + fw - 2 * f0), c.v00);
     const double gg = div_by(ga * (f0 + f2 - 2 * f1), c.v11);
     const double bb = div_by(be * bd, c.v01);
     const double d2u = aa + gg - 2 * bb;
     double cv = div_by(uxi * 0.5 * (fe - fw), c.v0);
     cv = cv + cy;
-    return div_by(1.0 * d2u, c.vRe) - cv - alc + Ri * T;
+    return div_by(1.0 * d2u, c.vRe) - cv;
 }
 
-// O-grid: wall pressure of column i (PSolver.cpp:1668-1725); swall = sin(2 pi F t)
+// O-grid: wall pressure of column i (PSolver.cpp:1668-1725); swall = sin(2 pi F t). A moving wall
+// makes the roundings of its velocity's products and of its acceleration show, so they are written
+// out: which product melts into a sum would otherwise change with the code around it.
 __device__ __forceinline__ double bc_wall_p(const BcCase& a, int i, const Edge& g, double swall) {
     const int ld = a.ld;
     const double *U = a.U, *V = a.V;
     const double d1 = a.d1;
     const long long k = i, k1 = k + ld, k2 = k + 2LL * ld;
     const double al = a.ALPH[k], ga = a.GAM[k], be = a.BETA[k], x = a.XIX[k], y = a.XIY[k], J = a.JAC[k];
-    const double uxi = x * g.u + y * g.v;
-    const double uet = a.ETX[k] * g.u + a.ETY[k] * g.v;
+    const double uxi = __fma_rn(x, g.u, __dmul_rn(y, g.v));
+    const double uet = __fma_rn(a.ETX[k], g.u, __dmul_rn(a.ETY[k], g.v));
     const double u1 = U[k1], u2 = U[k2], ub = U[k1 + 1] + g.uw - U[k1 - 1] - g.ue;
     const double v1 = V[k1], v2 = V[k2], vb = V[k1 + 1] + g.vw - V[k1 - 1] - g.ve;
-    const double alu = a.c.accn_amp * swall * a.Yc[k], alv = -a.c.accn_amp * swall * a.X[k];
-    const double T = a.Tn[k], p1 = a.P[k1];
-    const double fu = bc_force(a.c, g.u, g.ue, g.uw, u1, u2, ub, al, ga, be, uxi, div_by(uet * (u1 - g.u), a.c.v1), alu, 0.0, T);
-    const double fv = bc_force(a.c, g.v, g.ve, g.vw, v1, v2, vb, al, ga, be, uxi, div_by(uet * (v1 - g.v), a.c.v1), alv, a.Ri, T);
+    const double acc = __dmul_rn(a.c.accn_amp, swall), T = a.Tn[k], p1 = a.P[k1];
+    const double tu = bc_force(a.c, g.u, g.ue, g.uw, u1, u2, ub, al, ga, be, uxi, div_by(uet * (u1 - g.u), a.c.v1));
+    const double tv = bc_force(a.c, g.v, g.ve, g.vw, v1, v2, vb, al, ga, be, uxi, div_by(uet * (v1 - g.v), a.c.v1));
+    const double fu = __dsub_rn(tu, __dmul_rn(acc, a.Yc[k]));
+    const double fv = __fma_rn(a.Ri, T, __fma_rn(acc, a.X[k], tv));
     const double pw = p1 - (fu * (-y * J) + fv * (x * J)) * d1;
     store_mirrored(a.P, ld, i, 0, a.W, a.per, pw);
     return pw;
@@ -1251,8 +1253,9 @@ __device__ __forceinline__ void bc_far_p(const BcCase& a, int i, const Edge& g, 
         const double ub = g.ue + U[k1 - 1] - U[k1 + 1] - g.uw, vb = g.ve + V[k1 - 1] - V[k1 + 1] - g.vw;
         const double alu = div_by(g.u - s_old[i], a.c.vdt), alv = div_by(g.v - s_old[W + 1 + i], a.c.vdt);
         const double nu = uet * (3.0 * g.u - 4 * u1 + u2), nv = uet * (3.0 * g.v - 4 * v1 + v2);
-        const double fu = bc_force(a.c, g.u, g.ue, g.uw, u1, u2, ub, al, ga, be, uxi, div_by(nu, a.c.v1x2), alu, 0.0, T);
-        const double fv = bc_force(a.c, g.v, g.ve, g.vw, v1, v2, vb, al, ga, be, uxi, div_by(nv, a.c.v1x2), alv, a.Ri, T);
+        const double fu = bc_force(a.c, g.u, g.ue, g.uw, u1, u2, ub, al, ga, be, uxi, div_by(nu, a.c.v1x2)) - alu;
+        const double tv = bc_force(a.c, g.v, g.ve, g.vw, v1, v2, vb, al, ga, be, uxi, div_by(nv, a.c.v1x2)) - alv;
+        const double fv = __fma_rn(a.Ri, T, tv);
         pf = a.P[k1] + (fu * (-y * J) + fv * (x * J)) * d1;
     } else {
         const double e0 = ex * g.u + ey * g.v;
