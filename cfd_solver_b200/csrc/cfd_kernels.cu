@@ -96,7 +96,7 @@ constexpr int RHS_HALO = 6, RHS_INT = 7;
 constexpr size_t RHS_SMEM = (size_t)(RHS_HALO * JTW * JTH + RHS_INT * TX * TYJ) * sizeof(double) + 128;
 const size_t kRhsSmem = RHS_SMEM;
 
-// Three CTAs per SM (80 registers, 36 bytes of spills; the 63 KB staged per CTA fits three
+// Three CTAs per SM (80 registers, 40 bytes of spills; the 63 KB staged per CTA fits three
 // times): while one CTA computes, two others' copies are in flight. Two CTAs per SM at 122
 // registers left the SM idle between a CTA's copies and its arithmetic (431 vs 373 us per
 // step on the 256-case twin sweep).

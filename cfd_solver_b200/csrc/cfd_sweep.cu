@@ -16,7 +16,7 @@
 // loads each instead of twenty-five, and finishes each cell (off-centre sum: 25-point, or
 // 9-point on the near-wall cells; right-hand side, previous iterate, update) as its last row
 // comes in. With five live rows instead of eight, and the cells' flags packed in one
-// word, the kernel needs 118 registers where it filled 128 and spilled; k_sweep_f64 went from
+// word, the kernel needs 116 registers where it filled 128 and spilled; k_sweep_f64 went from
 // 987 to 878 us per step of the 256-case twin sweep (bound by the latency of the FP64 chains,
 // then by bytes). Five CTAs per SM need 96 registers: with spills 1,213 us, re-reading the
 // outer columns (922). The per-CTA constants and each field's warp residual sums sit in

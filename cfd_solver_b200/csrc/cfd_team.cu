@@ -10,7 +10,7 @@
 // crosses CTAs; a case stops its sweeps and pressure iterations on its own, whatever the
 // other cases of the batch need.
 //
-// A team is a thread-block cluster of up to 16 CTAs (hardware barrier, any number of
+// A team is a thread-block cluster of up to 16 CTAs (hardware barrier, without a limit; any number of
 // teams in waves), or, for one larger case, a share of a cooperative grid with a counter
 // barrier whose polls are bounded. One CTA has 512 threads: four groups of 128 for the
 // sweeps and the post-smoother, two groups of 256 for the cell kernels, the whole CTA for

@@ -253,7 +253,10 @@ typedef struct cfd_serve_stats {
 int cfd_serve(const cfd_serve_config* cfg, const cfd_request* reqs, int nreq, cfd_result* results,
               cfd_serve_stats* stats);
 
-/* ---- timing: per-kernel CUDA-event durations accumulated on the batch's stream ---- */
+/* ---- timing: per-kernel CUDA-event durations accumulated on the batch's stream ----
+ * While profiling is on, every step runs launch by launch from the host. A batch that otherwise
+ * steps by the team kernel (one launch for several steps) is then timed on a path it does not
+ * take, with the same bits; its own time is that of cfd_batch_step() with profiling off. */
 int cfd_batch_profile(cfd_batch* b, int enable);
 /* fills up to cap entries; returns the number of kernel names known */
 int cfd_batch_kernel_times(cfd_batch* b, const char** names, double* total_ms, long long* launches,
